@@ -42,51 +42,146 @@ constexpr int kPartialCluster = 8;  // CTAs whose partials are summed through DS
 
 __device__ __forceinline__ int64_t ceil_div_dev(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// G = sum_parts gpart + mu-terms; d-vectors folded in (see stpm_reduce doc).
-__global__ void stpm_reduce_kernel(StpmReduceArgs a) {
-  const int k = a.k;
+// Sum of v over the first 32 nw threads of the CTA, in a fixed order; red
+// holds 8 doubles.  Every thread gets the sum.  (FP64 runs at 2 operations
+// per clock and SM: warps without a value stay out.)
+__device__ __forceinline__ double cta_sum(double v, int nw, double* red) {
+  const int warp = threadIdx.x >> 5;
+  if (warp < nw) {
+#pragma unroll
+    for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  }
+  __syncthreads();  // red may still be read from the previous sum
+  if ((threadIdx.x & 31) == 0 && warp < nw) red[warp] = v;
+  __syncthreads();
+  double s = red[0];
+#pragma unroll 1
+  for (int w = 1; w < nw; ++w) s += red[w];
+  return s;
+}
+
+// G = sum_parts gpart + mu-terms; d-vectors folded in.  One CTA per column i,
+// a thread per entry: bound by two dependent L2 round trips (Phi and mu before
+// the wait, the partials after it), so the column's mean terms are warp
+// reductions and a thread's partials are loaded 8 at a time.  A power
+// iteration's normalisation runs here too (a.lambda): the column is complete
+// in its CTA, and a kernel of its own took 214 us per iteration at k = 33 (a
+// thread per column walking the matrix).  The two scalars over all columns
+// (the loss, the iterate's change) are summed in a fixed order by the CTA that
+// finishes last.
+__global__ void __launch_bounds__(256) stpm_reduce_kernel(StpmReduceArgs a) {
+  const int k = a.k, i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t kk = (int64_t)k * k;
-  extern __shared__ double mred[];  // m1, m2, m3, dsum(3k)
-  double* m = mred;
-  double* ds = mred + 3 * k;
-  for (int e = threadIdx.x; e < 3 * k; e += blockDim.x) {
-    const int which = e / k, i = e % k;
-    const float* mu = which == 0 ? a.mu1 : which == 1 ? a.mu2 : a.mu3;
+  __shared__ double m[3], ds[3], red[8], inv_norm;
+  __shared__ bool last;
+  if (tid < 3) m[tid] = 0.0;
+  __syncthreads();
+  if (warp < 3) {
+    const float* mu = warp == 0 ? a.mu1 : warp == 1 ? a.mu2 : a.mu3;
     double s = 0.0;
     if (mu)
-      for (int j = 0; j < k; ++j) s += (double)a.phi[(int64_t)i * k + j] * (double)mu[j];
-    m[e] = s;
-    double d = 0.0;
-    for (int p = 0; p < a.nparts; ++p) d += (double)a.gpart[(int64_t)p * a.part_stride + kk + e];
-    ds[e] = d;
+#pragma unroll 1
+      for (int j = lane; j < k; j += 32) s += (double)a.phi[(int64_t)i * k + j] * (double)mu[j];
+#pragma unroll
+    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane == 0) m[warp] = s;
+  }
+  // the contraction may let this kernel start early (it writes only gpart,
+  // and starts only when Phi is final); everything below reads gpart
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  double gsum = 0.0;
+  if (a.mode != kModeLoss && tid < k) {
+    const float* gp = a.gpart + (int64_t)i * k + tid;
+    int p = 0;
+#pragma unroll 1
+    for (; p + 8 <= a.nparts; p += 8) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = __ldcg(gp + (int64_t)(p + u) * a.part_stride);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) gsum += (double)v[u];
+    }
+#pragma unroll 1
+    for (; p < a.nparts; ++p) gsum += (double)__ldcg(gp + (int64_t)p * a.part_stride);
+  }
+  if (warp >= 5) {  // the d-sums of the column
+    const int q = warp - 5;
+    double s = 0.0;
+#pragma unroll 1
+    for (int p = lane; p < a.nparts; p += 32)
+      s += (double)__ldcg(a.gpart + (int64_t)p * a.part_stride + kk + q * k + i);
+#pragma unroll
+    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane == 0) ds[q] = s;
   }
   __syncthreads();
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < kk;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int j = (int)(e % k), i = (int)(e / k);
-    double s = 0.0;
-    if (a.mode != kModeLoss)
-      for (int p = 0; p < a.nparts; ++p) s += (double)a.gpart[(int64_t)p * a.part_stride + e];
-    s *= a.scale;
+  float g = 0.f;
+  if (tid < k) {
+    double s = gsum * a.scale;
     if (a.mode == kModePlain) {
       // mu_out * (c1 m1 m2 + c2 sum Z1 Z2)
-      const double d = a.c1 * m[i] * m[k + i] + a.c2 * ds[i];
-      s += (double)a.mu_out[j] * d;
+      s += (double)a.mu_out[tid] * (a.c1 * m[0] * m[1] + a.c2 * ds[0]);
     } else if (a.mode == kModeAdjoint) {
-      const double dm1 = a.c2 * ds[i] / a.count + a.c1 * m[k + i] * m[2 * k + i];
-      const double dm2 = a.c2 * ds[k + i] / a.count + a.c1 * m[i] * m[2 * k + i];
-      const double dm3 = a.c2 * ds[2 * k + i] / a.count + a.c1 * m[i] * m[k + i];
-      s += (double)a.mu1[j] * dm1 + (double)a.mu2[j] * dm2 + (double)a.mu3[j] * dm3;
+      const double dm1 = a.c2 * ds[0] * a.inv_count + a.c1 * m[1] * m[2];
+      const double dm2 = a.c2 * ds[1] * a.inv_count + a.c1 * m[0] * m[2];
+      const double dm3 = a.c2 * ds[2] * a.inv_count + a.c1 * m[0] * m[1];
+      s += (double)a.mu1[tid] * dm1 + (double)a.mu2[tid] * dm2 + (double)a.mu3[tid] * dm3;
     }
-    a.G[e] = (float)s;
+    g = (float)s;
+    a.G[(int64_t)i * k + tid] = g;
   }
-  if (a.mode == kModeLoss && blockIdx.x == 0 && threadIdx.x == 0) {
+  double term = 0.0;
+  if (a.lambda) {
+    // Phi_new = G (already includes the shift terms), lambda = ||col||^3,
+    // column normalisation, the column's share of ||Phi_new - Phi_old||^2
+    const int nw = (k + 31) / 32;
+    const double s = cta_sum((double)g * (double)g, nw, red);
+    if (tid == 0) {
+      const double nrm = sqrt(s);
+      inv_norm = 1.0 / nrm;  // one division per column
+      a.lambda[i] = s * nrm;
+    }
+    __syncthreads();
+    double e = 0.0;
+    if (tid < k) {
+      float* x = a.phi_out + (int64_t)i * k + tid;
+      const double v = (double)g * inv_norm, d = v - (double)*x;
+      e = d * d;
+      *x = (float)v;
+    }
+    term = cta_sum(e, nw, red);
+  } else if (a.mode == kModeLoss) {
+    term = a.c1 * m[0] * m[1] * m[2];
+  } else {
+    return;  // no scalar over the columns
+  }
+  if (tid == 0) {
+    a.parts[i] = term;
+    __threadfence();
+    last = atomicAdd(a.done, 1u) + 1u == gridDim.x;
+  }
+  __syncthreads();
+  if (!last) return;
+  if (tid == 0) *a.done = 0u;
+  double v = tid < k ? __ldcg(a.parts + tid) : 0.0;
+  if (a.mode == kModeLoss) {
+    // one loss slot per contraction column block
     double t = 0.0;
-    for (int p = 0; p < a.nparts; ++p)  // one loss slot per contraction column block
-      for (int sl = 0; sl < 4; ++sl) t += (double)a.gpart[(int64_t)p * a.part_stride + kk + 3 * k + sl];
-    double that = t / a.count;
-    for (int i = 0; i < k; ++i) that += a.c1 * m[i] * m[k + i] * m[2 * k + i];
-    a.loss_out[0] = that;  // sum_i That(phi_i, phi_i, phi_i)
+#pragma unroll 1
+    for (int e = tid; e < 4 * a.nparts; e += 256)
+      t += (double)__ldcg(a.gpart + (int64_t)(e >> 2) * a.part_stride + kk + 3 * k + (e & 3));
+    v += t * a.inv_count;
+  }
+  v = cta_sum(v, 8, red);
+  if (tid == 0) {
+    if (a.mode == kModeLoss) {
+      a.loss_out[0] = v;  // sum_i That(phi_i, phi_i, phi_i)
+    } else {
+      v = sqrt(v);
+      a.err_out[0] = v;
+      if (a.trace_out) a.trace_out[0] = v;
+    }
   }
 }
 
@@ -2310,36 +2405,6 @@ __global__ void __launch_bounds__(Contract<KP, MODE, BF>::NT) stpm_contract_batc
   contract_body<KP, MODE, BF>(a, a.nblocks);
 }
 
-// batch power: Phi_new = G (already includes the shift terms), lambda = ||col||^3,
-// column normalisation, error = ||Phi_new - Phi_old||_F
-__global__ void __launch_bounds__(1024) batch_update_kernel(int k, float* __restrict__ phi,
-                                                            const float* __restrict__ G,
-                                                            double* __restrict__ lambda,
-                                                            double* __restrict__ err_out) {
-  __shared__ double nrm[256];
-  __shared__ double errsum;
-  const int tid = threadIdx.x;
-  if (tid == 0) errsum = 0.0;
-  for (int i = tid; i < k; i += blockDim.x) {
-    double s = 0.0;
-    for (int j = 0; j < k; ++j) s += (double)G[(int64_t)i * k + j] * G[(int64_t)i * k + j];
-    nrm[i] = sqrt(s);
-    lambda[i] = s * sqrt(s);
-  }
-  __syncthreads();
-  double e = 0.0;
-  for (int idx = tid; idx < k * k; idx += blockDim.x) {
-    const int i = idx / k;
-    const double v = (double)G[idx] / nrm[i];
-    const double d = v - (double)phi[idx];
-    e += d * d;
-    phi[idx] = (float)v;
-  }
-  atomicAdd(&errsum, e);
-  __syncthreads();
-  if (tid == 0) err_out[0] = sqrt(errsum);
-}
-
 // lambda_i = phi_i . G_i (tensor value); sign fix so lambda_i > 0
 __global__ void tensor_value_kernel(int k, float* __restrict__ phi, const float* __restrict__ G,
                                     double* __restrict__ lambda, double* __restrict__ phi64) {
@@ -2602,10 +2667,23 @@ cudaError_t stpm_partial(int mode, const StpmPartialArgs& a, int grid, bool bf16
               : launch_partial_p<false>(mode, KP, a, grid, s);
 }
 
+// The power iteration of k = 33, 10,000 nodes (151 iterations): 261 us per
+// iteration with a thread per column summing the mean terms and normalising,
+// 22 us here; the reduction behind the lambda pass (38 partials) 49 us -> 8 us
+// at k = 100 and 245 us -> 115 us at k = 200, nearly all of that the wait for
+// the contraction it overlaps.
 cudaError_t stpm_reduce(const StpmReduceArgs& a, cudaStream_t s) {
-  const int64_t kk = (int64_t)a.k * a.k;
-  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(2 * kNumSMs, ceil_div(kk, 256)));
-  stpm_reduce_kernel<<<grid, 256, sizeof(double) * 6 * a.k, s>>>(a);
+  if (a.k > 256 || (!a.done && (a.lambda || a.mode == kModeLoss))) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)a.k, 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // follows the contraction
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MMSB_CUDA_TRY(cudaLaunchKernelEx(&cfg, stpm_reduce_kernel, a));
   ++g_launch_count;
   return cudaGetLastError();
 }
@@ -2660,13 +2738,6 @@ cudaError_t stpm_update_batched(int KP, const StpmUpdateArgs* args, int graphs, 
     case 128: return launch_step_batched_k<128>(args, graphs, s);
     default: return cudaErrorInvalidValue;
   }
-}
-
-cudaError_t stpm_batch_update(int k, float* phi, const float* G, double* lambda, double* err,
-                              cudaStream_t s) {
-  batch_update_kernel<<<1, 1024, 0, s>>>(k, phi, G, lambda, err);
-  ++g_launch_count;
-  return cudaGetLastError();
 }
 
 cudaError_t stpm_tensor_values(int k, float* phi, const float* G, double* lambda, cudaStream_t s,

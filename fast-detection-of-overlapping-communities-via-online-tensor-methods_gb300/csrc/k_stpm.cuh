@@ -61,9 +61,17 @@ struct StpmReduceArgs {
   const float* mu_out;  // plain mode
   double c1, c2;        // plain: d = c1 m1 m2 + c2 sum Z1Z2; adjoint/loss: p1, p2
   double scale;         // multiplies the contraction (adjoint: 1/count)
-  double count;         // nodes in the pass
+  double inv_count;     // 1 / nodes in the pass
   float* G;             // k x k column-major output
   double* loss_out;     // loss mode: sum_i That(phi_i,phi_i,phi_i)
+  // power iteration (lambda not null): lambda_i = ||G_i||^3, Phi_i = G_i / ||G_i||
+  // into phi_out, ||Phi - Phi_old||_F into err_out and, if not null, trace_out
+  double* lambda;
+  float* phi_out;
+  double* err_out;
+  double* trace_out;
+  double* parts;        // k doubles, and a counter that is 0 between launches
+  unsigned* done;       // (loss mode and power iteration)
 };
 
 struct StpmUpdateArgs {
@@ -121,8 +129,6 @@ cudaError_t stpm_partial_batched(int mode, int KP, const StpmPartialArgs* args, 
                                  int grid, bool bf16, cudaStream_t s);
 cudaError_t stpm_update_batched(int KP, const StpmUpdateArgs* args, int graphs, cudaStream_t s);
 cudaError_t stpm_update(const StpmUpdateArgs& a, cudaStream_t s);
-cudaError_t stpm_batch_update(int k, float* phi, const float* G, double* lambda, double* err,
-                              cudaStream_t s);
 // lambda_i = phi_i . G_i in FP64 (phi64: an FP64 copy of Phi to use for the
 // dot product, may be null), sign fixed so lambda_i > 0 (both copies flipped)
 cudaError_t stpm_tensor_values(int k, float* phi, const float* G, double* lambda, cudaStream_t s,

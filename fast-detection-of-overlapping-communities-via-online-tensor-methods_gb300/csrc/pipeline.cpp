@@ -682,8 +682,11 @@ static PartialOut stpm_partials(mmsb_ctx* c, int mode, int q1, int q2, int q3, i
   return PartialOut{gpart, grid / stpm_partial_cluster(), stride};
 }
 
+// power: a power iteration, Phi and lambda updated in place and the iterate's
+// change left in dscalar[0] and *power_trace (if not null)
 static void stpm_pass(mmsb_ctx* c, int mode, int q1, int q2, int q3, int64_t begin, int64_t count,
-                      double c0, double c1, double c2, double scale, float* G, double* loss) {
+                      double c0, double c1, double c2, double scale, float* G, double* loss,
+                      bool power = false, double* power_trace = nullptr) {
   const int k = c->k;
   PartialOut po = stpm_partials(c, mode, q1, q2, q3, begin, count, c0, c2);
   StpmReduceArgs r{};
@@ -700,9 +703,17 @@ static void stpm_pass(mmsb_ctx* c, int mode, int q1, int q2, int q3, int64_t beg
   r.c1 = c1;
   r.c2 = c2;
   r.scale = scale;
-  r.count = (double)count;
+  r.inv_count = 1.0 / (double)count;
   r.G = G;
   r.loss_out = loss;
+  r.parts = c->tbuf<double>("reduce_parts", 256);
+  r.done = c->flags + 1;
+  if (power) {
+    r.lambda = c->lambda;
+    r.phi_out = c->phi;
+    r.err_out = c->dscalar;
+    r.trace_out = power_trace;
+  }
   ck(stpm_reduce(r, c->s), "stpm_reduce");
 }
 
@@ -941,11 +952,9 @@ void pipeline_stpm(mmsb_ctx* c, const double* phi0) {
     c->conv_count = 0;
     for (int64_t it = 1;; ++it) {
       if (c->stop.load()) throw MmsbError(MMSB_ERR_STOPPED, "stop requested");
-      stpm_pass(c, kModePlain, 1, 2, 0, 0, nx, p_main, p_s0, p_s1, 1.0, G, nullptr);
-      ck(stpm_batch_update(k, c->phi, G, c->lambda, c->dscalar, s), "batch update");
-      if (c->conv_count < kConvCap)
-        ck(cudaMemcpyAsync(c->conv + c->conv_count++, c->dscalar, sizeof(double),
-                           cudaMemcpyDeviceToDevice, s), "trace");
+      c->ksample = it % 8 == 1;  // events between the kernels would break their chaining
+      stpm_pass(c, kModePlain, 1, 2, 0, 0, nx, p_main, p_s0, p_s1, 1.0, G, nullptr, true,
+                c->conv_count < kConvCap ? c->conv + c->conv_count++ : nullptr);
       c->stats.stpm_steps = it;
       if (it >= c->cfg.min_iter) {
         ck(cudaMemcpyAsync(&err, c->dscalar, sizeof(double), cudaMemcpyDeviceToHost, s), "err");
