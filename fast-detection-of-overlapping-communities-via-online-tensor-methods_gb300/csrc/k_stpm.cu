@@ -19,8 +19,8 @@
 // The contraction runs on the tensor cores (stpm_contract_kernel); partials
 // of 8-CTA clusters are summed through distributed shared memory and reduced
 // deterministically by stpm_reduce or by the step kernel.  The k x k update
-// (orthogonality term, step, Newton-Schulz polar orthonormalisation) runs on
-// one cluster of KP / 8 CTAs exchanging column blocks by bulk copies.
+// (orthogonality term, step, Cholesky QR) runs on one cluster that splits the
+// rows of the iterate and exchanges Gram blocks by bulk copies.
 #include "common.cuh"
 
 #include <cstdlib>
@@ -214,24 +214,35 @@ __global__ void __launch_bounds__(256) stpm_reduce_kernel(StpmReduceArgs a) {
 // computes the same Cholesky from the same data, so the pass count needs no
 // vote.
 //
-// Layout: every CTA holds whole k x k matrices (column-major, leading
-// dimension KP + 4) and owns NB = 8 or 16 columns.  The products
-// X^T Y[:, blk] (Gram) and X B_blk (times) run on the tensor cores as
-// warp-level m16n8k8 TF32 MMAs with the 3xTF32 split (a = a_hi + a_lo;
-// hi*hi + hi*lo + lo*hi accumulated in FP32, relative error ~1e-6 per
-// product; the first-order correction M F, |F| <= ~1e-5, as one TF32
-// product), one warp per 16 x 8 output tile.  A CTA's new column block is
-// staged in shared memory and sent to every CTA by bulk asynchronous copies
-// (cp.async.bulk shared::cta -> shared::cluster) that complete on the
-// receiver's per-block mbarrier; a CTA proceeds once all CL blocks have
-// arrived.  A staging tile used for broadcast n is rewritten at broadcast
-// n + 2 only, after every receiver has waited for broadcast n + 1 (sent by
-// each rank after it received all of broadcast n).
+// Split: the step is a chain of small dependent products, so what bounds it
+// is the number of exchanges and the Cholesky's pivots, not arithmetic.  CTA
+// q of the cluster owns RB = KP / CL ROWS of X.  A Gram is then the sum of
+// the CTAs' X_q^T X_q (a rank-RB product each): CTA q sends column block s of
+// its partial to CTA s, which adds the CL partials in rank order and sends
+// the finished block to everybody -- two one-way exchanges per Gram, no
+// cluster barrier.  Q1 = X R1^-1 needs no exchange at all: the rows of X ride
+// along as RB extra columns of the factorisation (R1^-T [A | X_q^T] leaves
+// (X_q R1^-1)^T), so neither R1^-1 nor Q1 is ever gathered, and the
+// first-order product is on the own rows as well.  (Owning columns instead
+// took an exchange of X, of A and of Q1 per pass, the triangular inverse and
+// three k^3 products: a minibatch step, contraction included, took 54 us at
+// k = 100, 20.6 us at k = 10 and 330 us at k = 200; 45, 15.3 and 295 us here.)  Up to KP = 64 one CTA holds everything and
+// nothing is exchanged.
 //
-// Hardware barriers of the step kernel's CTA: 0 = __syncthreads (whole CTA),
-// 1 = the four panel warps of inverse_columns (128 threads), 2 = the block-row
-// release of chol_blocked (warp 0 arrives, the other warps sync; whole CTA).
-// The three are never in use at the same time.
+// All products are FP32 FMAs (a thread per column, 8 rows at a time, the row
+// operand broadcast from shared memory): mma.sync TF32 in 3xTF32 form gives
+// ~50 multiply-adds per clock and SM here, FFMA up to 128, without the split.
+//
+// Exchanges are bulk asynchronous copies (cp.async.bulk shared::cta ->
+// shared::cluster) completing on the receiver's mbarrier of the source rank.
+// Buffers are reused without further synchronisation: a rank sends its
+// partials of Gram n + 1 only after it has all blocks of Gram n, and a block
+// of Gram n is sent only after its owner has consumed every partial of it.
+//
+// Hardware barriers of the step kernel's CTA: 0 = __syncthreads (whole CTA);
+// in chol_solve 1 = a diagonal block is factored (diagonal warp -> panel), 2 =
+// a block row is published and the previous trailing update complete (whole
+// CTA), 3 = the next block row is up to date (panel -> diagonal warp).
 
 // pivot ratio R_jj^2 / A_jj below which one more exact Cholesky QR pass runs
 // (one pass leaves Q1^T Q1 - I of about eps / ratio times a small constant, and
@@ -245,37 +256,40 @@ constexpr float kPivotFloor = 1e-7f;
 // the shift kShiftScale trace(A) (times 100 for each further restart, at
 // most kMaxShifts)
 constexpr float kShiftBelow = 1e-5f;
+// a first-order pass leaves about k |E|^2: it is repeated while an entry of E
+// is above this (the pivot ratios do not bound cond(X): with a few hundred
+// nodes per minibatch at k = 160 an exact pass left 0.1), at most 4 times
+constexpr float kFirstOrderBelow = 1e-4f;
 constexpr float kShiftScale = 1e-5f;
 constexpr int kMaxShifts = 3;
 
-// column stride of the k x k matrices: KP + 4 (== 4 mod 8 for KP a multiple
-// of 16) makes the fragment loads of the Gram product conflict-free
+// column stride of the k x k matrices and row blocks: KP + 4 floats, so that
+// columns stay 16-byte aligned and the 16-byte accesses of 8 consecutive
+// columns fall into different banks
 __host__ __device__ constexpr int step_xld(int KP) { return KP + 4; }
 
-// NB = 8 (one n-tile) when the cluster has KP / 8 CTAs, else 16.  Above
-// KP = 128 two FP32 copies of a k x k matrix no longer fit one SM (SB: a
-// single buffer, refilled after a cluster barrier, one staging tile, the
-// second tile holding the G block and then the inverse diagonal blocks of
-// the Cholesky factor; a matrix still needed after the buffer is refilled
-// is kept in global memory, StpmUpdateArgs::xstash).
+// CTAs of the step cluster: one up to KP = 64 (the exchanges would cost more
+// than the products they split), KP / 8 to 128, KP / 16 above (at most 16)
+__host__ __device__ constexpr int step_ctas(int KP) {
+  return KP <= 64 ? 1 : KP <= 128 ? KP / 8 : KP / 16;
+}
+
 template <int KP, int CL>
 struct StepSmem {
-  static constexpr int NB = KP / CL, XLD = step_xld(KP), MT = KP / 16, NT = NB / 8;
-  static constexpr int TILES = MT * NT, KS = TILES <= 8 ? 2 : 1;  // K split over warps
-  static constexpr bool SB = KP > 128;
-  static constexpr int NBK = KP / 8;  // 8-column blocks of the Cholesky factor
-  static constexpr size_t full = (size_t)(SB ? 1 : 2) * KP * XLD;
-  static constexpr size_t tiles = (size_t)4 * NB * XLD;  // B block, 2 staging tiles, G block
-  static constexpr size_t kpart = KS == 2 ? (size_t)TILES * 128 : 0;
-  // mean terms, d-sums, |phi_i|^2, mu1..3, tmp
-  static constexpr size_t small = 6 * KP + 4 * NB + 128 + 8;
-  // inverse diagonal blocks and superblock corners (SB: in the G block's tile)
-  static constexpr size_t tinv = SB ? 0 : (size_t)64 * NBK + 64 * (KP / 16);
-  static constexpr size_t floats = full + tiles - (SB ? NB * XLD : 0) + kpart + small + tinv +
-                                   2 * KP;  // original diagonal, 1 / R_jj
-  static_assert(!SB || (size_t)64 * NBK + 64 * (KP / 16) <= (size_t)NB * XLD,
-                "inverse blocks in the G tile");
-  static_assert(floats * sizeof(float) <= 227 * 1024 - 2048, "step kernel shared memory");
+  static constexpr int RB = KP / CL, XLD = step_xld(KP), NT = 512;
+  // above KP = 128 the partials of all ranks do not fit beside the matrix:
+  // each owner then reads them from the ranks' matrix buffers between two
+  // cluster barriers
+  static constexpr bool PULL = KP > 128;
+  static constexpr int PW = (KP + RB + 63) / 64, BW = NT / 32 - PW - 1;  // panel, bulk warps
+  static constexpr size_t recv = CL > 1 && !PULL ? (size_t)KP * XLD : 0;
+  static constexpr size_t rows = (size_t)RB * XLD;
+  // matrix, partials, X rows | Q1 rows | block to send, m1..3 and |phi_i|^2,
+  // mu1..3, d-sums, original diagonal, diagonal block
+  static constexpr size_t floats = (size_t)KP * XLD + recv + 3 * rows + 11 * KP + 128;
+  static_assert(KP % CL == 0 && RB % 8 == 0 && BW >= 4, "row blocks of whole 8-row blocks");
+  static_assert(KP <= 256 && (CL > 1 || KP <= 64), "16-byte words per column");
+  static_assert(floats * sizeof(float) <= 227 * 1024 - 1024, "step kernel shared memory");
 };
 
 __device__ __forceinline__ uint32_t tf32_round(float x) {
@@ -308,8 +322,6 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                : "memory");
 }
 
-// waits for the phase with the given parity to complete; false after `limit`
-// clock64 cycles (then the caller reports kFlagTimeout instead of hanging)
 // global -> this CTA's shared memory, completing on `bar` (16-byte aligned
 // addresses, bytes a multiple of 16)
 __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes,
@@ -321,6 +333,8 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
       : "memory");
 }
 
+// waits for the phase with the given parity to complete; false after `limit`
+// clock64 cycles (then the caller reports kFlagTimeout instead of hanging)
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
                                                   long long limit) {
   const long long start = clock64();
@@ -328,6 +342,22 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     uint32_t ok;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (clock64() - start > limit) return false;
+  }
+}
+
+__device__ __forceinline__ bool mbar_wait_cluster_bounded(uint64_t* bar, uint32_t parity,
+                                                          long long limit) {
+  const long long start = clock64();
+  while (true) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
         " selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(smem_addr(bar)), "r"(parity)
@@ -352,395 +382,247 @@ __device__ __forceinline__ void bulk_copy_to_rank(const void* dst_local, const v
       : "memory");
 }
 
-// One warp: acc = sum over k in [kb, ke) of A(m, k) B(k, n) for the 16 x 8
-// tile at pa = &A(0, 0) of the tile, pb = &B(0, 0) of the tile, with
-// A(m, k) = pa[m AM + k AK] and B(k, n) = pb[k BK + n BN].  Fragments of
-// m16n8k8 (g = lane / 4, t = lane % 4): a = A(g|g+8, t|t+4), b = B(t|t+4, g),
-// acc = C(g|g+8, 2t|2t+1).  SPLIT = false: one TF32 product (for a small
-// correction term whose relative error may be ~1e-3).
-template <int AM, int AK, int BK, int BN, bool SPLIT = true>
-__device__ __forceinline__ void warp_tile_3xtf32(const float* __restrict__ pa,
-                                                 const float* __restrict__ pb, int kb, int ke,
-                                                 float (&acc)[4]) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-  for (int k0 = kb; k0 < ke; k0 += 8) {
-    const float av[4] = {pa[g * AM + (k0 + t) * AK], pa[(g + 8) * AM + (k0 + t) * AK],
-                         pa[g * AM + (k0 + t + 4) * AK], pa[(g + 8) * AM + (k0 + t + 4) * AK]};
-    const float bv[2] = {pb[(k0 + t) * BK + g * BN], pb[(k0 + t + 4) * BK + g * BN]};
-    uint32_t ah[4], al[4], bh[2], bl[2];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      ah[q] = tf32_round(av[q]);
-      al[q] = __float_as_uint(av[q] - __uint_as_float(ah[q]));  // the MMA reads its top 19 bits
-    }
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      bh[q] = tf32_round(bv[q]);
-      bl[q] = __float_as_uint(bv[q] - __uint_as_float(bh[q]));
-    }
-    mma_tf32(c0, ah, bh);
-    if (SPLIT) {
-      mma_tf32(c1, ah, bl);
-      mma_tf32(c2, al, bh);
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) acc[q] = SPLIT ? c0[q] + (c1[q] + c2[q]) : c0[q];
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
 }
 
-// Tile products of the step.  Warp w < TILES * KS owns tile w % TILES and
-// half w / TILES of the K range (KS = 2); the halves meet in `part`.
-// kProdGram:  C_blk = X^T Y[:, c0 .. c0+NB)   (A(m=i, k=r) = X[i XLD + r], B = Y block)
-// kProdTimes: C_blk = X B_blk                 (A(m=r, k=i) = X[i XLD + r])
-// epi(acc, m0, n0) receives each finished 16 x 8 tile.
-enum StepProd : int { kProdGram = 0, kProdTimes = 1 };
+__device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
 
-template <int KP, int CL, int PROD, bool SPLIT = true, typename Epi>
-__device__ __forceinline__ void step_tiles(const float* __restrict__ X, const float* __restrict__ Bm,
-                                           float* part, Epi&& epi) {
-  using S = StepSmem<KP, CL>;
-  constexpr int XLD = S::XLD;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  auto product = [&](int tile, int kb, int ke, float (&acc)[4]) {
-    const int m0 = (tile % S::MT) * 16, n0 = (tile / S::MT) * 8;
-    if (PROD == kProdGram)
-      warp_tile_3xtf32<XLD, 1, 1, XLD, SPLIT>(X + m0 * XLD, Bm + n0 * XLD, kb, ke, acc);
-    else
-      warp_tile_3xtf32<1, XLD, 1, XLD, SPLIT>(X + m0, Bm + n0 * XLD, kb, ke, acc);
-  };
-  if (S::KS == 2) {
-    const int tile = warp % S::TILES, ks = warp / S::TILES;
-    const bool active = warp < S::TILES * S::KS;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    if (active) {
-      product(tile, ks * (KP / 2), ks * (KP / 2) + KP / 2, acc);
-      if (ks == 1) {
+// y_hi -= sum_b R(j0 + b, i0 + i) x_hb, i < 8: rows i0 .. i0+7 of H columns of
+// the trailing matrix (x_h: a column's entries of block row j0; Rj = &R(j0, i0)).
+// Every lane of a warp reads the same 16-byte words of R, which costs the
+// shared memory as much as different ones would: H columns share each.
+template <int XLD, int H>
+__device__ __forceinline__ void rank8(const float* Rj, const float (&x)[H][8], float (&y)[H][8]) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) part[tile * 128 + q * 32 + lane] = acc[q];
-      }
-    }
-    __syncthreads();
-    if (!active || ks != 0) return;
+  for (int i = 0; i < 8; ++i) {
+    float r[8];
+    load8(Rj + i * XLD, r);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] += part[tile * 128 + q * 32 + lane];
-    epi(acc, (tile % S::MT) * 16, (tile / S::MT) * 8);
-  } else {
-    for (int tile = warp; tile < S::TILES; tile += nw) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      product(tile, 0, KP, acc);
-      epi(acc, (tile % S::MT) * 16, (tile / S::MT) * 8);
-    }
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) y[h][i] = fmaf(-r[b], x[h][b], y[h][i]);
   }
 }
 
-// ---- Cholesky factor and its inverse on one CTA ----------------------------------
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// ---- Cholesky factorisation and forward substitution on one CTA -------------------
 //
-// A (KP x KP symmetric, column-major, leading dimension XLD, upper triangle
-// read) = R^T R with R upper triangular, blocked by 8 columns (right-looking,
-// one block of look-ahead).  Per block J: every thread forms one column of
-// the block row R_J = R_JJ^-T A_J by forward substitution; then warp 0,
-// which formed the block row's first 8 columns itself, goes straight on to
-// update the next 8 x 8 diagonal block, and one thread factors it in
-// registers (no shuffles on the pivot chain), while the other warps wait at
-// a named barrier for the whole block row and update the rest of the
-// trailing upper triangle with 3xTF32 tensor-core tiles (a rank-8 update is
-// one k-step); one CTA barrier closes the block.  R overwrites A's upper
-// triangle, 1 / R_jj goes to rd; the inverses T_JJ = R_JJ^-1 of the diagonal
-// blocks (tinv, 8 x 8 column-major each) are formed afterwards, one block per
-// thread, off the pivot chain.  Rows and columns >= k must hold the identity
-// (the caller sets their diagonal to 1; X's padding columns are zero).
-
-// One thread: the (already updated) 8 x 8 diagonal block at (j0, j0).  A
-// pivot that is not above kPivotFloor * dg (breakdown, or NaN) is raised to
-// it and counted as ratio 0.  Returns the smallest ratio R_jj^2 / dg[j] over
-// the live columns j0 + j < k.
-template <int XLD>
-__device__ __forceinline__ float factor_diag8(float* A, int j0, int k, float* rd, const float* dg) {
-  float a[8][8];
-#pragma unroll
-  for (int l = 0; l < 8; ++l)
-#pragma unroll
-    for (int i = 0; i <= l; ++i) a[i][l] = A[(j0 + i) + (j0 + l) * XLD];
-  float rmin = 1.f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float d = a[j][j];
-    const float d0 = dg[j0 + j];
-    float ratio = __fdividef(d, d0);
-    if (!(d > kPivotFloor * d0)) {
-      d = kPivotFloor * d0;
-      ratio = 0.f;
-    }
-    if (j0 + j < k) rmin = fminf(rmin, ratio);
-    const float ri = rsqrtf(d);
-    rd[j0 + j] = ri;
-    a[j][j] = d * ri;
-#pragma unroll
-    for (int l = j + 1; l < 8; ++l) a[j][l] *= ri;
-#pragma unroll
-    for (int i = j + 1; i < 8; ++i)
-#pragma unroll
-      for (int l = i; l < 8; ++l) a[i][l] = fmaf(-a[j][i], a[j][l], a[i][l]);
-  }
-#pragma unroll
-  for (int l = 0; l < 8; ++l)
-#pragma unroll
-    for (int i = 0; i <= l; ++i) A[(j0 + i) + (j0 + l) * XLD] = a[i][l];
-  return rmin;
-}
-
-// One thread: T = R_JJ^-1 (upper, 8 x 8 column-major into tb) of the
-// diagonal block at (j0, j0), column by column: T(j, j) = 1 / R_jj,
-// T(m, j) = -(sum_{m <= i < j} T(m, i) R(i, j)) / R(j, j).
-template <int XLD>
-__device__ __forceinline__ void invert_diag8(const float* A, int j0, const float* rd, float* tb) {
-  float r[8][8], t[8][8];
-#pragma unroll
-  for (int l = 0; l < 8; ++l)
-#pragma unroll
-    for (int i = 0; i < l; ++i) r[i][l] = A[(j0 + i) + (j0 + l) * XLD];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float rv = rd[j0 + j];
-    t[j][j] = rv;
-#pragma unroll
-    for (int m = 0; m < j; ++m) {
-      float s = 0.f;
-#pragma unroll
-      for (int i = m; i < j; ++i) s = fmaf(t[m][i], r[i][j], s);
-      t[m][j] = -s * rv;
-    }
-  }
-#pragma unroll
-  for (int l = 0; l < 8; ++l)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) tb[i + 8 * l] = i <= l ? t[i][l] : 0.f;
-}
-
-// Whole CTA.  Returns the smallest pivot ratio (the same value in every
-// thread: every CTA of a cluster factors the same matrix the same way).
+// Whole CTA.  A (symmetric, column-major, ld XLD, upper triangle read, rows
+// and columns < 8 nb, nb = ceil(k / 8)) = R^T R, and Y (RB columns, ld XLD, the
+// first `rows` of them not zero) becomes
+// R^-T Y: right-looking over 8-row blocks of the KP + RB columns.  The chain
+// that sets the time is that of the diagonal blocks, so one warp does nothing
+// else: it factors block J in registers (every lane the same), forward-
+// substitutes the 8 columns of block J + 1 and updates that diagonal block.
+// Panel warps (two columns per thread) take the factor for the other columns
+// of block row J and bring block row J + 1 up to date before the diagonal warp
+// asks for it; the bulk warps apply the block to the rows below.  The
+// entries of R stay in A above the diagonal blocks; the diagonal blocks are
+// not kept.  Rows and columns >= k hold the identity.  Returns the smallest
+// pivot ratio (the same in every thread: every CTA of a cluster factors the
+// same matrix the same way); a pivot that is not above kPivotFloor times its
+// original diagonal (breakdown, or NaN) is raised to that and counts as 0.
+// Measured per call at k = 100 (13 blocks): 21k cycles, 1.5k per block (factor
+// 0.65k, the rest round trips through shared memory and barriers), against
+// 30.7k for a single-thread diagonal factor plus about 5k for the triangular
+// inverse and product.
 // (No __restrict__ on these shared-memory pointers: other threads write what
 // a thread reads after each barrier, and the ratio decides the control flow
-// of the whole CTA, so no load may be moved across a barrier.  With
-// __restrict__ the compiler did move the read of the ratio above the
-// barrier: warps left the pass loop apart and the kernel hung.)
-template <int KP>
-__device__ float chol_blocked(float* A, int k, float* tinv, float* rd, float* dg,
-                              volatile float* s_ratio, float shift = 0.f) {
-  constexpr int XLD = step_xld(KP), NBK = KP / 8;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-  const int nw = blockDim.x >> 5;
-  for (int i = tid; i < KP; i += blockDim.x) {
+// of the whole CTA, so no load may be moved across a barrier.)
+template <int KP, int CL>
+__device__ float chol_solve(float* A, float* Y, int k, int rows, float* dg, float* dgi,
+                            float* dblk, float* rblk, volatile float* s_ratio, float shift) {
+  using S = StepSmem<KP, CL>;
+  constexpr int XLD = S::XLD, RB = S::RB, PW = S::PW, BW = S::BW;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nb = (k + 7) / 8, kk = 8 * nb;
+#pragma unroll 1
+  for (int i = tid; i < kk; i += S::NT) {
     float d = A[i + i * XLD] + shift;
     if (i >= k) d = 1.f;
     A[i + i * XLD] = d;
-    dg[i] = fmaxf(d, 1e-30f);
+    d = fmaxf(d, 1e-30f);
+    dg[i] = d;
+    dgi[i] = __fdividef(1.f, d);
   }
   __syncthreads();
-  float rmin = 1.f;
-  if (tid == 0) rmin = factor_diag8<XLD>(A, 0, k, rd, dg);
-  __syncthreads();
-  for (int J = 0; J + 1 < NBK; ++J) {
-    const int j0 = 8 * J, rest = KP - j0 - 8;
-    // block row: R(j0 + a, c) = (A(j0 + a, c) - sum_{b < a} R(j0 + b, j0 + a)
-    // R(j0 + b, c)) / R(j0 + a, j0 + a), c >= j0 + 8 (a thread per column)
-    for (int e = tid; e < rest; e += blockDim.x) {
-      const int c = j0 + 8 + e;
-      float x[8];
+  if (warp == 0) {
+    // the chain of diagonal blocks: factor block J (in every lane's
+    // registers), forward-substitute the next 8 columns (lane l: column n0 +
+    // l), update the next diagonal block
+    float rmin = 1.f;
 #pragma unroll
-      for (int b = 0; b < 8; ++b) x[b] = A[(j0 + b) + c * XLD];
-#pragma unroll
-      for (int aa = 0; aa < 8; ++aa) {
-        float s = x[aa];
-#pragma unroll
-        for (int b = 0; b < aa; ++b) s = fmaf(-A[(j0 + b) + (j0 + aa) * XLD], x[b], s);
-        x[aa] = s * rd[j0 + aa];
-      }
-#pragma unroll
-      for (int b = 0; b < 8; ++b) A[(j0 + b) + c * XLD] = x[b];
+    for (int h = 0; h < 2; ++h) {
+      const int e = lane + 32 * h;
+      dblk[e] = A[(e & 7) + (e >> 3) * XLD];
     }
-    // trailing update of the upper triangle, A(c, c') -= sum_b R(j0+b, c)
-    // R(j0+b, c') for j0 + 8 <= c <= c'
-    const int n0 = j0 + 8;
-    if (warp == 0) {
-      // the next diagonal block needs only the block row's columns n0 ..
-      // n0+7, which lanes 0-7 of this warp formed: the other warps are
-      // released through barrier 2 (arrive: release), and this warp goes on
-      // with the diagonal block and its factorisation at once
-      asm volatile("bar.arrive 2, %0;" ::"r"(nw * 32) : "memory");
+#pragma unroll 1
+    for (int J = 0; J < nb; ++J) {
+      const int j0 = 8 * J, n0 = j0 + 8;
       __syncwarp();
-      float sv[2];
+      float d[8][8], d0[8], di[8], ri[8];
+      load8(dg + j0, d0);
+      load8(dgi + j0, di);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int e = lane + 32 * h, i = e & 7, l = e >> 3;
-        sv[h] = A[(n0 + i) + (n0 + l) * XLD];
+      for (int l = 0; l < 8; ++l) {
+        float t[8];
+        load8(dblk + 8 * l, t);
 #pragma unroll
-        for (int b = 0; b < 8; ++b)
-          sv[h] = fmaf(-A[(j0 + b) + (n0 + i) * XLD], A[(j0 + b) + (n0 + l) * XLD], sv[h]);
+        for (int i = 0; i <= l; ++i) d[i][l] = t[i];
       }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int e = lane + 32 * h, i = e & 7, l = e >> 3;
-        if (i <= l) A[(n0 + i) + (n0 + l) * XLD] = sv[h];
+      for (int j = 0; j < 8; ++j) {
+        const float p = d[j][j], least = kPivotFloor * d0[j];
+        if (j0 + j < k) rmin = fminf(rmin, p > least ? p * di[j] : 0.f);
+        // (fmaxf: a NaN pivot is raised too)
+        ri[j] = rsqrt_ftz(fmaxf(p, least));
+#pragma unroll
+        for (int l = j + 1; l < 8; ++l) d[j][l] *= ri[j];
+#pragma unroll
+        for (int i = j + 1; i < 8; ++i)
+#pragma unroll
+          for (int l = i; l < 8; ++l) d[i][l] = fmaf(-d[j][i], d[j][l], d[i][l]);
+      }
+      // column a: R(b, a) for b < a, then 1 / R(a, a) (every lane stores the same)
+#pragma unroll
+      for (int l = 0; l < 8; ++l) {
+        float t[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t[i] = i < l ? d[i][l] : ri[l];
+        *reinterpret_cast<float4*>(rblk + 8 * l) = make_float4(t[0], t[1], t[2], t[3]);
+        if (l >= 4) *reinterpret_cast<float4*>(rblk + 8 * l + 4) = make_float4(t[4], t[5], t[6], t[7]);
       }
       __syncwarp();
-      if (lane == 0) rmin = fminf(rmin, factor_diag8<XLD>(A, n0, k, rd, dg));
-    } else {
-      asm volatile("bar.sync 2, %0;" ::"r"(nw * 32) : "memory");  // every block-row column
-    }
-    if (warp != 0 && rest > 8) {
-      // columns c' >= n0 + 8 in 8-wide tiles, rows c in [n0, c'] in 16-row
-      // tiles from mb; a last tile that would pass KP is computed at KP - 16
-      // (rows below mb not written), so no read leaves the matrix
-      const int mt = (rest + 15) / 16, ntl = (rest - 8) / 8;
-      for (int tl = warp - 1; tl < mt * ntl; tl += nw - 1) {
-        const int mb = n0 + 16 * (tl % mt), nc0 = n0 + 8 + 8 * (tl / mt);
-        if (mb > nc0 + 7) continue;  // entirely below the diagonal
-        const int m0 = min(mb, KP - 16);
-        float acc[4];
-        warp_tile_3xtf32<XLD, 1, 1, XLD>(A + j0 + m0 * XLD, A + j0 + nc0 * XLD, 0, 8, acc);
+      asm volatile("bar.arrive 1, %0;" ::"n"(32 * (PW + 1)) : "memory");
+      if (J + 1 < nb) {
+        // the panel has brought block row J of these columns up to date
+        if (J > 0) asm volatile("bar.sync 3, %0;" ::"n"(32 * (PW + 1)) : "memory");
+        if (lane < 8) {
+          float* col = A + j0 + (n0 + lane) * XLD;
+          float y[8];
+          load8(col, y);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int r = m0 + g + ((q & 2) ? 8 : 0), c = nc0 + 2 * t4 + (q & 1);
-          if (r >= mb && r <= c) A[r + c * XLD] -= acc[q];
+          for (int i = 0; i < 8; ++i) {
+            y[i] *= ri[i];
+#pragma unroll
+            for (int l = i + 1; l < 8; ++l) y[l] = fmaf(-d[i][l], y[i], y[l]);
+          }
+          store8(col, y);
+        }
+      }
+      asm volatile("bar.sync 2, %0;" ::"n"(S::NT) : "memory");
+      if (J + 1 < nb) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = lane + 32 * h, i = e & 7, l = e >> 3;
+          float xi[8], xl[8];
+          load8(A + j0 + (n0 + i) * XLD, xi);
+          load8(A + j0 + (n0 + l) * XLD, xl);
+          float v = A[(n0 + i) + (n0 + l) * XLD];
+#pragma unroll
+          for (int b = 0; b < 8; ++b) v = fmaf(-xi[b], xl[b], v);
+          dblk[e] = v;
         }
       }
     }
-    __syncthreads();
+    if (lane == 0) *s_ratio = rmin;
+  } else if (warp <= PW) {
+    // the panel, two columns per thread (of A, and past KP the rows of the
+    // block as columns): forward substitution of the columns past the diagonal
+    // warp's, then their next 8 entries
+    constexpr int H = 2;
+    float* col[H];
+    int cs[H];  // the column; a large number for a row of the block, -1: none
+    float y[H][8];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int c = tid - 32 + 32 * PW * h;
+      const bool aug = c >= KP && c < KP + rows;
+      cs[h] = c < kk ? c : aug ? 1 << 30 : -1;
+      col[h] = c < kk ? A + c * XLD : Y + (aug ? c - KP : 0) * XLD;
+      load8(col[h], y[h]);
+    }
+#pragma unroll 1
+    for (int J = 0; J < nb; ++J) {
+      const int j0 = 8 * J, n0 = j0 + 8;
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * (PW + 1)) : "memory");  // R_JJ published
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float r[8];  // R(0 .. i-1, i), 1 / R(i, i)
+        load8(rblk + 8 * i, r);
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+#pragma unroll
+          for (int l = 0; l < i; ++l) y[h][i] = fmaf(-r[l], y[h][l], y[h][i]);
+          y[h][i] *= r[i];
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+        if (cs[h] >= n0 + 8) store8(col[h] + j0, y[h]);
+      // block row J is complete, and the bulk warps are done with J - 1
+      asm volatile("bar.sync 2, %0;" ::"n"(S::NT) : "memory");
+      if (J + 1 < nb) {
+        float x[H][8];
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+#pragma unroll
+          for (int b = 0; b < 8; ++b) x[h][b] = y[h][b];
+          load8(col[h] + n0, y[h]);
+        }
+        rank8<XLD, H>(A + j0 + n0 * XLD, x, y);
+        if (J + 2 < nb) {
+#pragma unroll
+          for (int h = 0; h < H; ++h)
+            if (cs[h] >= n0 + 8 && cs[h] < n0 + 16) store8(col[h] + n0, y[h]);
+          asm volatile("bar.arrive 3, %0;" ::"n"(32 * (PW + 1)) : "memory");
+        }
+      }
+    }
+  } else {
+    // rows >= j0 + 16 (the panel threads update the 8 before): a warp per 8
+    // rows, the columns from the row block's diagonal on and then those of Y,
+    // 32 at a time; the row operand stays in registers (every lane the same
+    // words: a broadcast load costs the shared memory as much as any other).
+    // (mma.sync TF32 in 3xTF32 form took 3.2k cycles for the first block at k
+    // = 100.)
+#pragma unroll 1
+    for (int J = 0; J < nb; ++J) {
+      const int j0 = 8 * J;
+      asm volatile("bar.sync 2, %0;" ::"n"(S::NT) : "memory");
+#pragma unroll 1
+      for (int i0 = j0 + 16 + 8 * (warp - PW - 1); i0 < kk; i0 += 8 * BW) {
+        const int nc = kk - i0 + rows;
+        float r[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) load8(A + j0 + (i0 + i) * XLD, r[i]);
+#pragma unroll 1
+        for (int u = lane; u < nc; u += 32) {
+          float* col = u < kk - i0 ? A + (i0 + u) * XLD : Y + (u - (kk - i0)) * XLD;
+          float x[8], y[8];
+          load8(col + j0, x);
+          load8(col + i0, y);
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int b = 0; b < 8; ++b) y[i] = fmaf(-r[i][b], x[b], y[i]);
+          store8(col + i0, y);
+        }
+      }
+    }
   }
-  // the inverses of the diagonal blocks, one block per thread
-  for (int J = tid; J < NBK; J += blockDim.x) invert_diag8<XLD>(A, 8 * J, rd, tinv + 64 * J);
-  if (tid == 0) *s_ratio = rmin;
   __syncthreads();
   return *s_ratio;
-}
-
-// Columns c0 .. c0+NB of W = R^-1 (NB = 8 or 16: whole 8-column blocks) into
-// Wb (column jb at Wb + jb * XLD, rows past the diagonal block zero), by
-// block back substitution per 8-column block K: W_KK = T_KK, then upwards in
-// levels of 16 rows aligned to 16 (one 8-row level first when K is odd):
-// W_Q = -T_Q S_Q with S_Q = sum over the rows P below Q of R_QP W_PK, where
-// for a 16-row superblock Q = (a, b) of 8-row blocks T_Q = [T_a X; 0 T_b],
-// X = -T_a R_ab T_b (x16, 8 x 8 column-major per superblock, formed here
-// first).  One barrier per level: warps 0-3 add the last term of S_Q and
-// apply -T_Q (a named barrier between the two), while the other warps add
-// R_rP W_PK of the last level into the partial sums of the rows above
-// (held in Wb until their level).  The levels of the last column block are
-// about KP / 16 instead of KP / 8, which is what the cluster waits for.
-// Blocks that lie wholly in the padding (8K >= k: R is the identity there)
-// get unit columns.  tmp: 128 floats.  Whole CTA of at least 5 warps; ends
-// with a barrier.
-template <int KP, int NB>
-__device__ void inverse_columns(const float* R, const float* tinv, float* x16, int c0, int k,
-                                float* Wb, float* tmp) {
-  constexpr int XLD = step_xld(KP), NSB = KP / 16;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int e = tid; e < NB * XLD; e += nt) Wb[e] = 0.f;
-  // X(a, b) = -sum_i T_2m(a, i) sum_j R(16m + i, 16m + 8 + j) T_2m+1(j, b)
-  // (the T blocks hold explicit zeros below their diagonals; the R reads of
-  // a warp are broadcasts)
-  for (int e = tid; e < NSB * 64; e += nt) {
-    const int m = e >> 6, aa = e & 7, b = (e >> 3) & 7, r0 = 16 * m;
-    const float* ta = tinv + 64 * (2 * m);
-    const float* tb = ta + 64;
-    float tv[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) tv[j] = tb[j + 8 * b];
-    float x = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float y = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) y = fmaf(R[(r0 + i) + (r0 + 8 + j) * XLD], tv[j], y);
-      x = fmaf(ta[aa + 8 * i], y, x);
-    }
-    x16[e] = -x;
-  }
-#pragma unroll 1
-  for (int sb = 0; sb < NB / 8; ++sb) {
-    const int K = c0 / 8 + sb;
-    float* W = Wb + 8 * sb * XLD;
-    __syncthreads();  // zero fill, X and the previous column block done
-    if (8 * K >= k) {
-      if (tid < 8) W[8 * K + tid + tid * XLD] = 1.f;
-      continue;
-    }
-    for (int e = tid; e < 64; e += nt) {
-      const int aa = e & 7, jb = e >> 3;
-      W[8 * K + aa + jb * XLD] = tinv[64 * K + e];  // W_KK = T_KK (column-major)
-    }
-    __syncthreads();
-    int lo = 8 * K, h = 8;  // rows [lo, lo + h) were the last level
-    while (lo > 0) {
-      const int hn = (lo & 15) ? 8 : 16, nlo = lo - hn;
-      if (tid < 128) {
-        // S_Q (row i, column jb) = partial sum + R(nlo + i, lo ..) W(lo .., jb)
-        const int i = tid & 15, jb = tid >> 4;
-        if (i < hn) {
-          float sv = W[nlo + i + jb * XLD];
-#pragma unroll
-          for (int b = 0; b < 8; ++b) sv = fmaf(R[(nlo + i) + (lo + b) * XLD], W[lo + b + jb * XLD], sv);
-          if (h == 16) {
-#pragma unroll
-            for (int b = 8; b < 16; ++b) sv = fmaf(R[(nlo + i) + (lo + b) * XLD], W[lo + b + jb * XLD], sv);
-          }
-          tmp[i + 16 * jb] = sv;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (i < hn) {
-          const float* s = tmp + 16 * jb;
-          float w = 0.f;
-          // T rows from the diagonal on (zeros below it are stored)
-          const int ii = i & 7;
-          const float* t = tinv + 64 * (nlo / 8 + (i >> 3));
-          const float* sv = s + (i & 8);
-#pragma unroll
-          for (int b = 0; b < 8; ++b) w = fmaf(t[ii + 8 * b], sv[b], w);
-          if (hn == 16 && i < 8) {
-            const float* x = x16 + 64 * (nlo / 16) + i;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) w = fmaf(x[8 * j], s[8 + j], w);
-          }
-          W[nlo + i + jb * XLD] = -w;
-        }
-      } else {
-        // rows above the level accumulate R(r, lo ..) W(lo .., jb)
-        for (int e = tid - 128; e < nlo * 8; e += nt - 128) {
-          const int r = e % nlo, jb = e / nlo;
-          float sv = W[r + jb * XLD];
-#pragma unroll
-          for (int b = 0; b < 8; ++b) sv = fmaf(R[r + (lo + b) * XLD], W[lo + b + jb * XLD], sv);
-          if (h == 16) {
-#pragma unroll
-            for (int b = 8; b < 16; ++b) sv = fmaf(R[r + (lo + b) * XLD], W[lo + b + jb * XLD], sv);
-          }
-          W[r + jb * XLD] = sv;
-        }
-      }
-      __syncthreads();
-      h = hn;
-      lo = nlo;
-    }
-  }
-  __syncthreads();
-}
-
-__device__ __forceinline__ bool mbar_wait_cluster_bounded(uint64_t* bar, uint32_t parity,
-                                                          long long limit) {
-  const long long start = clock64();
-  while (true) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (clock64() - start > limit) return false;
-  }
 }
 
 template <int KP>
@@ -749,83 +631,87 @@ struct ContractTc;  // the tensor-core contraction's shared-memory layout (below
 template <int KP, int CL>
 __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
   using S = StepSmem<KP, CL>;
-  constexpr int NB = S::NB, XLD = S::XLD;
-  static_assert(NB == 8 || NB == 16, "column block of 8 or 16");
+  constexpr int RB = S::RB, XLD = S::XLD, NT = S::NT;
   // one warp of the 512 threads issues the copy to each rank
-  static_assert(CL <= 16 && S::TILES <= 32, "cluster or tile count");
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
+  static_assert(CL <= 16, "cluster size");
+  const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
   extern __shared__ __align__(16) float sm[];
-  float* Xa = sm;
-  float* Xb = S::SB ? Xa : Xa + KP * XLD;
-  float* Ab = Xa + S::full;                       // B block of the products, column jb at Ab + jb * XLD
-  float* Ot = Ab + NB * XLD;                      // staging tile(s) of the broadcasts
-  float* Gb = Ot + (S::SB ? 1 : 2) * NB * XLD;    // G block (online step)
-  float* part = Gb + NB * XLD;                    // K-split partial tiles
-  float* mv = part + S::kpart;                    // m1, m2, m3 of this block
-  float* dcol = mv + 3 * KP;                      // 3 * NB d-sums
-  float* nn = dcol + 3 * NB;                      // |phi_i|^2 of this block
-  float* mus = nn + NB;                           // mu1, mu2, mu3 (KP each)
-  float* tmp = mus + 3 * KP;                      // 128 (inverse columns)
-  float* tinv = S::SB ? Gb : tmp + 128 + 8;       // 8 x 8 inverse diagonal blocks
-  float* x16 = tinv + 64 * S::NBK;                // corners of the 16 x 16 inverse blocks
-  float* dg = (S::SB ? tmp + 128 + 8 : x16 + 64 * (KP / 16));  // original diagonal
-  float* rd = dg + KP;                            // 1 / R_jj
-  __shared__ float s_ratio;
+  float* A = sm;                       // Phi, then Grams and factors, columns at A + c XLD
+  float* Rv = A + KP * XLD;            // column block of the Gram partials of every rank
+  float* Xr = Rv + S::recv;            // own rows of X / Q1: row r at Xr + r XLD
+  float* Yr = Xr + S::rows;
+  float* St = Yr + S::rows;            // finished column block to send
+  float* mv = St + S::rows;            // m1 | m2 | m3 | |phi_i|^2 (KP each)
+  float* mus = mv + 4 * KP;            // mu1 | mu2 | mu3
+  float* dcol = mus + 3 * KP;          // d-sums (3 KP), later 1 / dg
+  float* dg = dcol + 3 * KP;           // original diagonal of the Gram
+  float* dblk = dg + KP;               // 8 x 8 diagonal block and its factor
+  __shared__ float s_ratio, s_shift;
   __shared__ float s_emax[16];
-  __shared__ __align__(8) uint64_t s_blk[2][16];  // block q of Xa / Xb arrived
-  __shared__ __align__(8) uint64_t s_csync;       // bounded cluster barrier
-  const int k = a.k;
-  const int c0 = rank * NB;
-  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  __shared__ __align__(8) uint64_t s_part[16], s_blk[16];  // partial / block of rank q arrived
+  __shared__ __align__(8) uint64_t s_csync[2];             // bounded cluster barrier, in turn
+  const int k = a.k, nb = (k + 7) / 8, kk = 8 * nb;
+  const int r0 = rank * RB, rows = max(0, min(RB, k - r0));  // own rows that are not padding
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long wl = tc::wait_limit_or_default(a.wait_limit);
   {
     // Phi: loads issued in batches of 8 per thread so that their latencies overlap
     constexpr int N = KP * XLD, B = 8;
-    for (int e0 = tid; e0 < N; e0 += 512 * B) {
+#pragma unroll 1
+    for (int e0 = tid; e0 < N; e0 += NT * B) {
       float v[B];
 #pragma unroll
       for (int u = 0; u < B; ++u) {
-        const int e = e0 + 512 * u, r = e % XLD, c = e / XLD;
+        const int e = e0 + NT * u, r = e % XLD, c = e / XLD;
         v[u] = (e < N && r < k && c < k) ? __ldg(a.phi + (int64_t)c * k + r) : 0.f;
       }
 #pragma unroll
       for (int u = 0; u < B; ++u)
-        if (e0 + 512 * u < N) {
-          Xa[e0 + 512 * u] = v[u];
-          if (!S::SB) Xb[e0 + 512 * u] = 0.f;
-        }
+        if (e0 + NT * u < N) A[e0 + NT * u] = v[u];
     }
   }
-  for (int e = tid; e < (S::SB ? 1 : 2) * NB * XLD; e += blockDim.x) Ot[e] = 0.f;
-  if (tid < 2 * CL) mbar_init(&s_blk[tid / CL][tid % CL], 1);
-  if (tid == 2 * CL) mbar_init(&s_csync, CL);
-  if (tid <= 2 * CL) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  __syncthreads();
-  if (a.step_mode == kStepOnline) {
-    // mu1..3 for the G block below, and the mean terms phi_i . mu and
-    // |phi_i|^2 of this block's columns (a warp per dot product, lanes along
-    // the k entries): Phi and mu only, so before the wait
-    for (int e = tid; e < 3 * KP; e += blockDim.x) {
+  const bool online = a.step_mode == kStepOnline;
+  if (online)
+#pragma unroll 1
+    for (int e = tid; e < 3 * KP; e += NT) {
       const int which = e / KP, j = e % KP;
       const float* mu = which == 0 ? a.mu1 : which == 1 ? a.mu2 : a.mu3;
       mus[e] = (mu && j < k) ? __ldg(mu + j) : 0.f;
     }
-    for (int e = tid / 32; e < 4 * NB; e += blockDim.x / 32) {
-      const int which = e / NB, jb = e % NB, i = c0 + jb;
-      const float* col = Xa + i * XLD;
-      const float* mu = which == 0 ? a.mu1 : which == 1 ? a.mu2 : which == 2 ? a.mu3 : col;
-      float sv = 0.f;
-      if (i < k && mu)
-        for (int j = lane; j < k; j += 32) sv = fmaf(col[j], mu[j], sv);
+  if (CL > 1) {
+    if (tid < CL) mbar_init(&s_part[tid], 1);
+    else if (tid < 2 * CL) mbar_init(&s_blk[tid - CL], 1);
+    else if (tid < 2 * CL + 2) mbar_init(&s_csync[tid - 2 * CL], CL);
+    if (tid < 2 * CL + 2) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (online) {
+    // mean terms phi_i . mu and |phi_i|^2 of all columns: Phi and mu only, so
+    // before the wait.  8 columns x 4 quarters of the rows per warp.
+    static_assert(KP % 16 == 0, "quarters of whole 16-byte words");
+#pragma unroll 1
+    for (int i0 = 8 * warp; i0 < KP; i0 += NT / 4) {
+      const int i = i0 + (lane & 7), h = lane >> 3;
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int j = h * (KP / 4); j < (h + 1) * (KP / 4); j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(A + i * XLD + j);
 #pragma unroll
-      for (int off = 16; off; off >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, off);
-      if (lane == 0) {
-        if (which < 3) mv[which * KP + jb] = sv; else nn[jb] = sv;
+        for (int q = 0; q < 3; ++q) {
+          const float4 m = *reinterpret_cast<const float4*>(mus + q * KP + j);
+          s[q] = fmaf(x.x, m.x, fmaf(x.y, m.y, fmaf(x.z, m.z, fmaf(x.w, m.w, s[q]))));
+        }
+        s[3] = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, s[3]))));
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        s[q] += __shfl_xor_sync(0xffffffffu, s[q], 8);
+        s[q] += __shfl_xor_sync(0xffffffffu, s[q], 16);
+        if (h == 0) mv[q * KP + i] = s[q];
       }
     }
   }
-  cluster.sync();  // Phi read and barriers initialised everywhere before any copy
+  if (CL > 1) cg::this_cluster().sync();  // barriers initialised everywhere before any copy
   // launched with programmatic serialization after the contraction, the
   // prologue above overlapped its tail (Phi is final: the contraction lets
   // this kernel start only after its own wait on the previous step); from
@@ -833,270 +719,391 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
   // next contraction be scheduled (it waits for this kernel in turn)
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  uint32_t parity = 0u;  // bit b: phase parity awaited on the barriers of buffer b
-  uint32_t csync_parity = 0u;
-  int nbcast = 0;
+  uint32_t par_part = 0u, par_blk = 0u, csync_n = 0u;
   bool timed_out = false;
-  constexpr uint32_t kBlockBytes = sizeof(float) * NB * XLD;
-  auto buf_of = [&](const float* b) { return b == Xa ? 0 : 1; };
-  // staging tile of the next broadcast (or of the final block)
-  auto stage_next = [&]() -> float* {
-    float* p = S::SB ? Ot : Ot + (nbcast & 1) * NB * XLD;
-    ++nbcast;
-    return p;
-  };
   // bounded cluster barrier: every thread of every CTA has passed the
   // __syncthreads before its rank's arrival (remote mbarrier arrives with
-  // release semantics, waited for with acquire); false after a timeout
+  // release semantics, waited for with acquire); false after a timeout.  Two
+  // mbarriers in turn: a rank past barrier n may arrive for n + 1 where phase
+  // n still misses an arrival.
   auto csync_arrive = [&]() {
     __syncthreads();
     if (tid < CL) {
       uint32_t remote;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(&s_csync)), "r"(tid));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                   : "=r"(remote)
+                   : "r"(smem_addr(&s_csync[csync_n & 1])), "r"(tid));
       asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
     }
   };
   auto csync_wait = [&]() -> bool {
     bool ok = true;
-    if (tid == 0) ok = mbar_wait_cluster_bounded(&s_csync, csync_parity, wl);
-    csync_parity ^= 1u;
+    if (tid == 0) ok = mbar_wait_cluster_bounded(&s_csync[csync_n & 1], (csync_n >> 1) & 1u, wl);
+    ++csync_n;
     return !__syncthreads_or(!ok);
   };
-  auto csync = [&]() -> bool {
-    csync_arrive();
-    return csync_wait();
-  };
-  // the staged block Otc (this CTA's columns) into `dst` of every rank,
-  // own copy included; sync_first: a cluster barrier first, because some
-  // rank may still be reading its `dst`
-  auto broadcast = [&](float* Otc, float* dst, bool sync_first) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // staging -> async proxy
-    if (sync_first) {
-      if (!csync()) timed_out = true;
-    } else {
-      __syncthreads();
-    }
-    float* own = dst + c0 * XLD;
-    for (int e = tid; e < NB * XLD; e += blockDim.x) own[e] = Otc[e];
-    const int bi = buf_of(dst), w = tid >> 5;
-    // one issuing thread per warp (copies issued by lanes of one warp
-    // serialise); rank q sends to q+1, q+2, ... first, so every rank receives
-    // its blocks spread over the exchange
-    if (lane == 0 && w < CL - 1)
-      bulk_copy_to_rank(own, Otc, kBlockBytes, &s_blk[bi][rank], (uint32_t)((rank + 1 + w) % CL));
-    if (tid < CL && tid != rank) mbar_arrive_expect_tx(&s_blk[bi][tid], kBlockBytes);
-  };
-  // every block of `buf` has arrived (false after a timeout of any wait);
-  // SB: then a cluster barrier, after which every copy of the broadcast has
-  // landed everywhere (the single staging tile and the G tile are free)
-  auto wait_buf = [&](const float* buf) -> bool {
-    const int bi = buf_of(buf);
-    bool ok = true;
-    if (tid < CL && tid != rank) ok = mbar_wait_bounded(&s_blk[bi][tid], (parity >> bi) & 1u, wl);
-    parity ^= 1u << bi;
-    ok = !__syncthreads_or(!ok);
-    if (S::SB) ok = csync() && ok;
-    return ok;
-  };
-  // Gram block C = P^T P[:, c0 .. c0+NB) into the staging tile, zero outside
-  // k x k; a non-finite entry raises kFlagNonFinite
-  auto gram_stage = [&](const float* P, float* Otc) {
-    bool bad = false;
-    step_tiles<KP, CL, kProdGram>(P, P + c0 * XLD, part, [&](const float (&acc)[4], int m0, int n0) {
+  constexpr uint32_t kBlockBytes = sizeof(float) * RB * XLD;
+
+  // X^T X of the CTA's rows X into A (upper triangle, 8-row blocks), summed
+  // over the cluster; first_order: F of E = X^T X - I instead.  Leaves the
+  // whole matrix in every CTA; false after a timeout.  (One call site: the
+  // step runs through its code once, and instruction fetch from L2 was its
+  // largest cost while the kernel had 88 KB of it.)
+  float emax = 0.f;
+  auto gram = [&](const float* X, bool first_order) -> bool {
+    __syncthreads();  // X complete, A free
+    // a warp per 8 rows, 4 columns per lane (the row operand is a broadcast:
+    // every load of it serves 4 columns)
+#pragma unroll 1
+    for (int i0 = 8 * warp; i0 < kk; i0 += 8 * (NT / 32)) {
+#pragma unroll 1
+      for (int c0 = i0; c0 < kk; c0 += 128) {
+        float acc[4][8];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = m0 + g + ((q & 2) ? 8 : 0), jb = n0 + 2 * t4 + (q & 1), col = c0 + jb;
-        const float v = acc[q];
-        if (!isfinite(v)) bad = true;
-        Otc[jb * XLD + i] = (i < k && col < k) ? v : 0.f;
+        for (int h = 0; h < 4; ++h)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[h][i] = 0.f;
+#pragma unroll 1
+        for (int rb = 0; rb < rows; rb += 8) {
+          // 8 rows apart from the sum so far: less round-off than one long chain
+          float part[4][8];
+#pragma unroll
+          for (int h = 0; h < 4; ++h)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) part[h][i] = 0.f;
+#pragma unroll 2
+          for (int r = rb; r < rb + 8; ++r) {
+            float w[8];
+            load8(X + r * XLD + i0, w);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              const int c = c0 + 32 * h + lane;
+              const float x = c < kk ? X[r * XLD + c] : 0.f;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) part[h][i] = fmaf(w[i], x, part[h][i]);
+            }
+          }
+#pragma unroll
+          for (int h = 0; h < 4; ++h)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[h][i] += part[h][i];
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const int c = c0 + 32 * h + lane;
+          if (c < kk) store8(A + c * XLD + i0, acc[h]);
+        }
       }
-    });
+    }
+    bool bad = false;
+    auto finish = [&](float4 v, int c, int i4) {
+      float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = 4 * i4 + u;
+        if (i <= c && !isfinite(w[u])) bad = true;  // (nothing below the diagonal is read)
+        if (first_order) {
+          const float e = i <= c && c < k ? w[u] - (i == c ? 1.f : 0.f) : 0.f;
+          emax = fmaxf(emax, fabsf(e));
+          w[u] = i < c ? e : 0.5f * e;
+        }
+      }
+      return make_float4(w[0], w[1], w[2], w[3]);
+    };
+    const int cols = max(0, min(RB, kk - r0)), n4 = kk / 4;
+    if (CL == 1) {
+      __syncthreads();
+#pragma unroll 1
+      for (int e = tid; e < cols * 16; e += NT) {  // (n4 <= 16)
+        const int c = e >> 4, i4 = e & 15;
+        float4* p = reinterpret_cast<float4*>(A + c * XLD) + i4;
+        if (i4 < n4) *p = finish(*p, c, i4);
+      }
+      if (bad) atomicOr(a.flags, kFlagNonFinite);
+      __syncthreads();
+      return true;
+    }
+    bool ok = true;
+    if (!S::PULL) {
+      // column block s of the partial to rank s, rank q's next neighbours
+      // first (copies issued by lanes of one warp serialise)
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncthreads();
+      if (lane == 0 && warp < CL - 1) {
+        const int to = (rank + 1 + warp) % CL;
+        bulk_copy_to_rank(Rv + rank * RB * XLD, A + to * RB * XLD, kBlockBytes, &s_part[rank],
+                          (uint32_t)to);
+      }
+      if (tid < CL && tid != rank) {
+        mbar_arrive_expect_tx(&s_part[tid], kBlockBytes);
+        ok = mbar_wait_bounded(&s_part[tid], par_part, wl);
+      }
+      par_part ^= 1u;
+      if (__syncthreads_or(!ok)) return false;
+    } else {
+      csync_arrive();
+      if (!csync_wait()) return false;
+    }
+    // own block: the ranks' partials added in rank order
+#pragma unroll 1
+    for (int e = tid; e < cols * 64; e += NT) {
+      const int c = e >> 6, i4 = e & 63;  // (n4 <= 52)
+      if (i4 >= n4) continue;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int q = 0; q < CL; ++q) {
+        const float* src;
+        if (S::PULL)
+          src = cg::this_cluster().map_shared_rank(A, q) + (r0 + c) * XLD;
+        else
+          src = q == rank ? A + (r0 + c) * XLD : Rv + (q * RB + c) * XLD;
+        const float4 t = reinterpret_cast<const float4*>(src)[i4];
+        v.x += t.x, v.y += t.y, v.z += t.z, v.w += t.w;
+      }
+      reinterpret_cast<float4*>(St + c * XLD)[i4] = finish(v, r0 + c, i4);
+    }
     if (bad) atomicOr(a.flags, kFlagNonFinite);
+    if (S::PULL) {
+      csync_arrive();  // every rank has read the partials: blocks may land on them
+      if (!csync_wait()) return false;
+    }
+    // (a flag in the padding of the block's first column: see more_orders)
+    const bool large = __syncthreads_or(first_order && emax > kFirstOrderBelow) != 0;
+    if (tid == 0) St[KP] = large ? 1.f : 0.f;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (lane == 0 && warp < CL - 1)
+      bulk_copy_to_rank(A + r0 * XLD, St, kBlockBytes, &s_blk[rank],
+                        (uint32_t)((rank + 1 + warp) % CL));
+#pragma unroll 1
+    for (int e = tid; e < cols * 64; e += NT)
+      if ((e & 63) < n4)
+        reinterpret_cast<float4*>(A + (r0 + (e >> 6)) * XLD)[e & 63] =
+            reinterpret_cast<const float4*>(St + (e >> 6) * XLD)[e & 63];
+    if (tid == 0) A[r0 * XLD + KP] = large ? 1.f : 0.f;
+    if (tid < CL && tid != rank) {
+      mbar_arrive_expect_tx(&s_blk[tid], kBlockBytes);
+      ok = mbar_wait_bounded(&s_blk[tid], par_blk, wl);
+    }
+    par_blk ^= 1u;
+    return !__syncthreads_or(!ok);
   };
 
-  float* M = Xa;               // the matrix to orthonormalise (full in every CTA)
-  float* F = S::SB ? Xa : Xb;  // the other buffer
-  if (a.step_mode == kStepOnline) {
-    // G block (columns c0 .. c0+NB) from the per-CTA partials.  The first 8
-    // partials of this thread's (up to) two G entries are loaded together
-    // with the d-sum partials, so that one round trip covers them all.
-    constexpr int kPre = 2, kPreParts = 8;
-    float gpre[kPre][kPreParts];
+  // whether any rank's block of E had an entry above kFirstOrderBelow (the
+  // same in every CTA: the blocks carry it in their padding)
+  auto more_orders = [&]() -> bool {
+    if (CL == 1) return __syncthreads_or(emax > kFirstOrderBelow) != 0;
+    bool more = false;
+    for (int q = 0; q < CL; ++q) more = more || A[q * RB * XLD + KP] != 0.f;
+    return more;
+  };
+
+  float* M = Xr;  // own rows of the matrix to orthonormalise
+  float* F = Yr;
+  if (online) {
+    // own rows of G from the contraction's partials, 4 rows of one column per
+    // item (a 16-byte load per partial where the rows allow it), and the
+    // d-sums of all columns (3 KP, zero past k).  The first 8 partials of a
+    // thread's first item and of its d-sum are loaded together: one L2 round
+    // trip (~1.7k cycles for lines another SM has just written) covers them.
+    const bool vec = ((k | (int)a.part_stride) & 3) == 0 && ((uintptr_t)a.gpart & 15) == 0;
+    constexpr int PRE = 8, ITEMS = KP * (RB / 4);
+    static_assert(3 * KP <= 2 * NT, "two d-sums per thread");
+    auto load4 = [&](const float* p, int j) {  // rows j .. j+3 of one partial
+      if (vec) return __ldg(reinterpret_cast<const float4*>(p));
+      float4 v = make_float4(__ldg(p), 0.f, 0.f, 0.f);
+      if (j + 1 < k) v.y = __ldg(p + 1);
+      if (j + 2 < k) v.z = __ldg(p + 2);
+      if (j + 3 < k) v.w = __ldg(p + 3);
+      return v;
+    };
+#pragma unroll 1
+    for (int e = tid; e < max(ITEMS, 3 * KP); e += NT) {
+      const int i = e / (RB / 4), rr = 4 * (e % (RB / 4)), j = r0 + rr;
+      const bool live = e < ITEMS && i < k && j < k;
+      const float* gp = a.gpart + (int64_t)i * k + j;
+      const int which = e / KP, di = e % KP;
+      const bool dlive = which < 3 && di < k && (which == 0 || a.mode == kModeAdjoint);
+      const float* dp = a.gpart + (int64_t)k * k + which * k + di;
+      float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+      float d = 0.f;
+#pragma unroll 1
+      for (int p0 = 0; p0 < a.nparts; p0 += PRE) {
+        float4 v[PRE];
+        float w[PRE];
 #pragma unroll
-    for (int h = 0; h < kPre; ++h) {
-      const int e = tid + h * (int)blockDim.x, jb = e / KP, j = e % KP, i = c0 + jb;
-      const bool live = e < NB * KP && i < k && j < k;
-#pragma unroll
-      for (int u = 0; u < kPreParts; ++u)
-        gpre[h][u] = (live && u < a.nparts)
-                         ? __ldg(a.gpart + (int64_t)u * a.part_stride + (int64_t)i * k + j)
-                         : 0.f;
-    }
-    // per-column sums of the d partials (3 x NB)
-    for (int e = tid / 32; e < 3 * NB; e += blockDim.x / 32) {
-      const int which = e / NB, jb = e % NB, i = c0 + jb;
-      float sd = 0.f;
-      if (i < k && (which == 0 || a.mode == kModeAdjoint))
-        for (int pp = tid % 32; pp < a.nparts; pp += 32)
-          sd += a.gpart[(int64_t)pp * a.part_stride + (int64_t)k * k + which * k + i];
-#pragma unroll
-      for (int off = 16; off; off >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, off);
-      if ((tid & 31) == 0) dcol[e] = sd;
-    }
-    __syncthreads();
-    for (int e = tid; e < NB * KP; e += blockDim.x) {
-      const int jb = e / KP, j = e % KP, i = c0 + jb;
-      float gval = 0.f;
-      if (i < k && j < k) {
-        const float* gp = a.gpart + (int64_t)i * k + j;
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-        int pp = 0;
-        const int h = (e - tid) / (int)blockDim.x;  // 0 or 1 for the preloaded entries
-        if (h < kPre) {
-#pragma unroll
-          for (int h2 = 0; h2 < kPre; ++h2)
-            if (h2 == h) {
-              s0 += gpre[h2][0] + gpre[h2][4];
-              s1 += gpre[h2][1] + gpre[h2][5];
-              s2 += gpre[h2][2] + gpre[h2][6];
-              s3 += gpre[h2][3] + gpre[h2][7];
-            }
-          pp = kPreParts;
+        for (int u = 0; u < PRE; ++u) {
+          const bool has = p0 + u < a.nparts;
+          v[u] = has && live ? load4(gp + (int64_t)(p0 + u) * a.part_stride, j)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+          w[u] = has && dlive ? __ldg(dp + (int64_t)(p0 + u) * a.part_stride) : 0.f;
         }
-        for (; pp + 8 <= a.nparts; pp += 8) {
-          float v[8];
+        // (8 partials as a tree: the sum's round-off grows with its depth)
 #pragma unroll
-          for (int u = 0; u < 8; ++u) v[u] = __ldg(gp + (int64_t)(pp + u) * a.part_stride);
-          s0 += v[0] + v[4];
-          s1 += v[1] + v[5];
-          s2 += v[2] + v[6];
-          s3 += v[3] + v[7];
-        }
-        for (; pp < a.nparts; ++pp) s0 += __ldg(gp + (int64_t)pp * a.part_stride);
-        float gv = ((s0 + s1) + (s2 + s3)) * (float)a.scale;
-        const float m1 = mv[jb], m2 = mv[KP + jb], m3 = mv[2 * KP + jb];
-        const float c1 = (float)a.c1, c2 = (float)a.c2;
-        if (a.mode == kModePlain) {
-          gv += mus[2 * KP + j] * (c1 * m1 * m2 + c2 * dcol[jb]);
-        } else {
-          const float ic = (float)(1.0 / a.count);
-          gv += mus[j] * (c2 * dcol[jb] * ic + c1 * m2 * m3) +
-                mus[KP + j] * (c2 * dcol[NB + jb] * ic + c1 * m1 * m3) +
-                mus[2 * KP + j] * (c2 * dcol[2 * NB + jb] * ic + c1 * m1 * m2);
-        }
-        gval = gv;
+        for (int h = PRE / 2; h; h >>= 1)
+#pragma unroll
+          for (int u = 0; u < h; ++u) {
+            v[u].x += v[u + h].x, v[u].y += v[u + h].y;
+            v[u].z += v[u + h].z, v[u].w += v[u + h].w;
+            w[u] += w[u + h];
+          }
+        g.x += v[0].x, g.y += v[0].y, g.z += v[0].z, g.w += v[0].w;
+        d += w[0];
       }
-      Gb[jb * XLD + j] = gval;
+      if (e < ITEMS) {
+        Xr[rr * XLD + i] = g.x;
+        Xr[(rr + 1) * XLD + i] = g.y;
+        Xr[(rr + 2) * XLD + i] = g.z;
+        Xr[(rr + 3) * XLD + i] = g.w;
+      }
+      if (which < 3) dcol[e] = d;
     }
     // X = Phi - beta (3 theta Phi (Phi^T Phi)^.2 - gscale G)   (Util.cpp:259-272)
-    float* Otc;
     const float alpha = -a.beta * a.theta3, gamma = a.beta * a.gscale;
     if (a.phi_general) {
-      // the literal product (first step of a run: Phi0 need not be orthonormal)
-      step_tiles<KP, CL, kProdGram>(M, M + c0 * XLD, part, [&](const float (&acc)[4], int m0, int n0) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int i = m0 + g + ((q & 2) ? 8 : 0), jb = n0 + 2 * t4 + (q & 1);
-          Ab[jb * XLD + i] = acc[q] * acc[q];
+      // the literal product (first step of a run: Phi0 need not be
+      // orthonormal), 16 columns of (Phi^T Phi)^.2 at a time (in Yr | St); every
+      // CTA forms all of them, once per run.  Xr then holds both terms.
+      float* S2 = Yr;
+      static_assert(2 * RB * XLD >= 16 * XLD, "16 columns in Q1's rows and the staged block");
+      constexpr int PER = (16 * RB + NT - 1) / NT;  // products per thread and 16 columns
+#pragma unroll 1
+      for (int i0 = 0; i0 < KP; i0 += 16) {
+        __syncthreads();
+#pragma unroll 1
+        for (int e = tid; e < KP * 16; e += NT) {
+          const int l = e % KP, i = i0 + e / KP;
+          float s = 0.f;
+#pragma unroll 1
+          for (int j = 0; j < KP; j += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(A + l * XLD + j);
+            const float4 y = *reinterpret_cast<const float4*>(A + i * XLD + j);
+            s = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, s))));
+          }
+          S2[(i - i0) * XLD + l] = s * s;
         }
-      });
-      __syncthreads();
-      Otc = stage_next();
-      step_tiles<KP, CL, kProdTimes>(M, Ab, part, [&](const float (&acc)[4], int m0, int n0) {
+        __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int r = m0 + g + ((q & 2) ? 8 : 0), jb = n0 + 2 * t4 + (q & 1), col = c0 + jb;
-          const float v = alpha * acc[q] + M[col * XLD + r] + gamma * Gb[jb * XLD + r];
-          Otc[jb * XLD + r] = (r < k && col < k) ? v : 0.f;
+        for (int t = 0; t < PER; ++t) {
+          const int e = tid + NT * t, r = e % RB, ii = e / RB, i = i0 + ii;
+          if (e < 16 * RB) {
+            float s = 0.f;
+#pragma unroll 1
+            for (int l = 0; l < k; ++l) s = fmaf(A[l * XLD + r0 + r], S2[ii * XLD + l], s);
+            Xr[r * XLD + i] = fmaf(alpha, s, gamma * (Xr[r * XLD + i] * a.scale));
+          }
         }
-      });
-    } else {
-      // Phi is the previous step's Q: Phi^T Phi = I to ~1e-7, so
-      // (Phi^T Phi)^.2 = diag(|phi_i|^4) + O(1e-14) and Phi times it is
-      // phi_i |phi_i|^4, column by column
-      __syncthreads();
-      Otc = stage_next();
-      for (int e = tid; e < NB * XLD; e += blockDim.x) {
-        const int r = e % XLD, jb = e / XLD, col = c0 + jb;
-        const float n2 = nn[jb] * nn[jb];
-        Otc[e] = (r < k && col < k) ? M[col * XLD + r] * (1.f + alpha * n2) + gamma * Gb[e] : 0.f;
       }
-    }
-    broadcast(Otc, F, S::SB);
-    if (!wait_buf(F)) timed_out = true;
-    float* t = M;
-    M = F;
-    F = t;
-  }
-  // Cholesky QR passes on M: A = M^T M gathered into F, R = chol(A) and the
-  // columns of R^-1 this CTA needs (computed by every CTA from the same A),
-  // M R^-1 gathered into F, which becomes M.  (SB: M is kept in global
-  // memory while its buffer holds A.)
-  int passes = 0, shifts = 0, plain_left = a.max_passes;
-  float shift = 0.f;
-  bool resync = false;  // a rank may still be factoring the last Gram in F
-  __shared__ float s_shift;
-  // SB: the buffer (R, read by no one now) gets M back from the stash
-  // (written before the barrier of the last broadcast)
-  auto restore_m = [&]() {
-    for (int e = tid; e < KP * KP; e += blockDim.x) {
-      const int r = e % KP, c = e / KP;
-      M[c * XLD + r] = __ldcg(a.xstash + (int64_t)c * KP + r);
     }
     __syncthreads();
-  };
-  while (!timed_out) {
-    float* Otc = stage_next();
-    gram_stage(M, Otc);
-    if (S::SB) {
-      // M's own columns to the stash (every rank's are read back below)
-      for (int e = tid; e < NB * KP; e += blockDim.x) {
-        const int r = e % KP, jb = e / KP;
-        a.xstash[(int64_t)(c0 + jb) * KP + r] = M[(c0 + jb) * XLD + r];
+#pragma unroll 1
+    for (int e = tid; e < RB * XLD; e += NT) {
+      const int r = e / XLD, i = e % XLD, j = r0 + r;
+      float x = 0.f;
+      if (i < k && j < k) {
+        const float m1 = mv[i], m2 = mv[KP + i], m3 = mv[2 * KP + i];
+        const float c1 = a.c1, c2 = a.c2;
+        // (explicit fmaf here: the single and the batched kernel must round alike)
+        float gm;  // the mean terms of the gradient
+        if (a.mode == kModePlain) {
+          gm = mus[2 * KP + j] * fmaf(c1 * m1, m2, c2 * dcol[i]);
+        } else {
+          const float c2n = c2 * a.inv_count;
+          gm = fmaf(mus[j], fmaf(c1 * m2, m3, c2n * dcol[i]),
+                    fmaf(mus[KP + j], fmaf(c1 * m1, m3, c2n * dcol[KP + i]),
+                         mus[2 * KP + j] * fmaf(c1 * m1, m2, c2n * dcol[2 * KP + i])));
+        }
+        const float phi = A[i * XLD + j], g = Xr[e];
+        if (a.phi_general) {
+          x = phi + fmaf(gamma, gm, g);
+        } else {
+          // Phi is the previous step's Q: Phi^T Phi = I to ~1e-7, so
+          // (Phi^T Phi)^.2 = diag(|phi_i|^4) + O(1e-14) and Phi times it is
+          // phi_i |phi_i|^4, column by column
+          const float n2 = mv[3 * KP + i] * mv[3 * KP + i];
+          x = fmaf(phi, fmaf(alpha, n2, 1.f), gamma * fmaf(g, a.scale, gm));
+        }
       }
+      Xr[e] = x;
     }
-    broadcast(Otc, F, S::SB || resync);
-    resync = false;
-    if (!wait_buf(F)) {
+  } else {
+#pragma unroll 1
+    for (int e = tid; e < RB * XLD; e += NT) {
+      const int r = e / XLD, i = e % XLD;
+      Xr[e] = i < KP ? A[i * XLD + r0 + r] : 0.f;
+    }
+  }
+  // Cholesky QR passes: A = M^T M, M <- M R^-1
+  int passes = 0, shifts = 0, plain_left = a.max_passes;
+  float shift = 0.f;
+  bool first_order = false;  // the second pass: E = M^T M - I, Phi = M (I - F)
+  int orders = 0;
+  float emax_all = 0.f;
+  while (true) {
+    if (!gram(M, first_order)) {
       timed_out = true;
       break;
     }
-    const float ratio = chol_blocked<KP>(F, k, tinv, rd, dg, &s_ratio, shift);
+    if (first_order) {
+      const bool more = more_orders() && orders < 4;
+      ++orders;
+      // no copy to this CTA is outstanding after the last pass; its own may
+      // still be read by others, so it stays until every rank has arrived here
+      if (CL > 1 && !more) csync_arrive();
+      // own rows of M - M F: RT rows of one column per item, F's column in
+      // 16-byte words down to the diagonal
+      constexpr int RT = RB >= 32 ? 4 : 2;
+#pragma unroll 1
+      for (int e = tid; e < KP * (RB / RT); e += NT) {
+        const int c = e % KP, r = RT * (e / KP);
+        float s[RT];
+#pragma unroll
+        for (int u = 0; u < RT; ++u) s[u] = 0.f;
+        if (c < k && r < rows)
+#pragma unroll 2
+          for (int i = 0; i <= c; i += 4) {
+            const float4 f = *reinterpret_cast<const float4*>(A + c * XLD + i);
+#pragma unroll
+            for (int u = 0; u < RT; ++u) {
+              const float4 m = *reinterpret_cast<const float4*>(M + (r + u) * XLD + i);
+              s[u] = fmaf(m.x, f.x, fmaf(m.y, f.y, fmaf(m.z, f.z, fmaf(m.w, f.w, s[u]))));
+            }
+          }
+#pragma unroll
+        for (int u = 0; u < RT; ++u) {
+          const int j = r0 + r + u;
+          const float v = c < k && j < k ? M[(r + u) * XLD + c] - s[u] : 0.f;
+          F[(r + u) * XLD + c] = v;
+        }
+      }
+      if (!more) break;
+      emax_all = fmaxf(emax_all, emax);
+      emax = 0.f;
+      float* t = M;
+      M = F;
+      F = t;
+      continue;
+    }
+#pragma unroll 1
+    for (int e = tid; e < RB * XLD; e += NT) F[e] = M[e];
+    const float ratio = chol_solve<KP, CL>(A, F, k, rows, dg, dcol, dblk, dblk + 64, &s_ratio, shift);
     if (__syncthreads_or(ratio < kShiftBelow) && shifts < kMaxShifts) {
       // near breakdown: the Gram again, factored with a diagonal shift
       if (tid == 0) {
         float tr = 0.f;
+#pragma unroll 1
         for (int i = 0; i < k; ++i) tr += dg[i];
         s_shift = shift > 0.f ? 100.f * shift : kShiftScale * tr;
       }
       __syncthreads();
       shift = s_shift;
       ++shifts;
-      if (S::SB) restore_m();
-      resync = true;
       continue;
     }
-    inverse_columns<KP, NB>(F, tinv, x16, c0, k, Ab, tmp);
     ++passes;
-    if (S::SB) restore_m();
-    Otc = stage_next();
-    step_tiles<KP, CL, kProdTimes>(M, Ab, part, [&](const float (&acc)[4], int m0, int n0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = m0 + g + ((q & 2) ? 8 : 0), jb = n0 + 2 * t4 + (q & 1), col = c0 + jb;
-        Otc[jb * XLD + r] = (r < k && col < k) ? acc[q] : 0.f;
-      }
-    });
-    // every rank has finished its Cholesky in F (and, SB, its product on M)
-    // before any block of M R^-1 is written there
-    broadcast(Otc, F, true);
-    if (!wait_buf(F)) {
-      timed_out = true;
-      break;
-    }
     float* t = M;
     M = F;
-    F = S::SB ? M : t;
+    F = t;
     if (shift > 0.f) {
       // Q1 of a shifted factor is well conditioned, not orthonormal: plain
       // passes follow
@@ -1110,119 +1117,83 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
     const bool again = __syncthreads_or(ratio < kQrExactBelow) != 0;
     if (!again || plain_left <= 0) {
       if (again && rank == 0 && tid == 0) atomicOr(a.flags, kFlagNoConvergence);
-      break;
+      first_order = true;
     }
   }
-  // every copy of the last exchange has landed in this CTA, and each rank
-  // sent its blocks only after the barrier that opened that exchange, so
-  // every rank's phase of that barrier is complete: this CTA's arrival at
-  // the closing barrier (no remote access follows) goes out now, its wait
-  // comes at the end
-  const bool early_arrive = !timed_out;
-  if (early_arrive) csync_arrive();
-  // first-order second pass: E = M^T M - I, F = strict upper part of E plus
-  // half its diagonal (this CTA's columns, in Ab), Phi = M (I - F)
-  float emax = 0.f;
   if (!timed_out) {
-    step_tiles<KP, CL, kProdGram>(M, M + c0 * XLD, part, [&](const float (&acc)[4], int m0, int n0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = m0 + g + ((q & 2) ? 8 : 0), jb = n0 + 2 * t4 + (q & 1), col = c0 + jb;
-        const bool live = i < k && col < k;
-        const float e = live ? acc[q] - (i == col ? 1.f : 0.f) : 0.f;
-        emax = fmaxf(emax, fabsf(e));
-        Ab[jb * XLD + i] = i < col ? e : i == col ? 0.5f * e : 0.f;
-      }
-    });
+    emax = fmaxf(emax, emax_all);
 #pragma unroll
     for (int off = 16; off; off >>= 1) emax = fmaxf(emax, __shfl_xor_sync(0xffffffffu, emax, off));
-    if (lane == 0) s_emax[tid >> 5] = emax;
+    if (lane == 0) s_emax[warp] = emax;
     __syncthreads();
-    float* Otc = stage_next();
-    // |F| is at most ~1e-5 here (an exact pass left M orthonormal to u times
-    // at most 1 / the pivot ratio bound), so a single TF32 product keeps
-    // M F to ~1e-9, below the FP32 resolution of Phi's entries
-    step_tiles<KP, CL, kProdTimes, false>(M, Ab, part, [&](const float (&acc)[4], int m0, int n0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = m0 + g + ((q & 2) ? 8 : 0), jb = n0 + 2 * t4 + (q & 1), col = c0 + jb;
-        Otc[jb * XLD + r] = (r < k && col < k) ? M[col * XLD + r] - acc[q] : 0.f;
-      }
-    });
-    __syncthreads();
+#pragma unroll 1
+    for (int e = tid; e < KP * RB; e += NT) {
+      const int r = e % RB, c = e / RB;
+      if (c < k && r0 + r < k) a.phi[(int64_t)c * k + r0 + r] = F[r * XLD + c];
+    }
     if (tid == 0) {
       float m = 0.f;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, s_emax[w]);
+#pragma unroll 1
+      for (int w = 0; w < NT / 32; ++w) m = fmaxf(m, s_emax[w]);
       if (a.orth_err) atomicMax(reinterpret_cast<int*>(a.orth_err), __float_as_int(m));
-    }
-    for (int e = tid; e < KP * NB; e += blockDim.x) {
-      const int r = e % KP, jb = e / KP, col = c0 + jb;
-      if (r < k && col < k) a.phi[(int64_t)col * k + r] = Otc[jb * XLD + r];
     }
     if constexpr (KP <= 112) {
       if (a.phi_img) {
-        // the next contraction's operand image of this CTA's columns i (rows
-        // of its A operand, K = j): TF32 hi / lo in the core-matrix layout,
-        // then Phi^T mu1, Phi^T mu2 of the columns
+        // the next contraction's operand image (rows i of its A operand, K =
+        // j): TF32 hi / lo of the own 16-byte words along j, in the core-matrix
+        // layout
         using CT = ContractTc<KP>;
         unsigned char* img = static_cast<unsigned char*>(a.phi_img);
-        for (int e = tid; e < NB * (KP / 4); e += blockDim.x) {
-          const int jb = e / (KP / 4), jq = e % (KP / 4), i = c0 + jb;
+#pragma unroll 1
+        for (int e = tid; e < KP * (RB / 4); e += NT) {
+          const int i = e % KP, r = 4 * (e / KP);
           float v[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) v[u] = Otc[jb * XLD + 4 * jq + u];  // zero past k
+          for (int u = 0; u < 4; ++u) v[u] = F[(r + u) * XLD + i];  // zero past k
           uint4 h;
           float4 l;
           tc::split4(v, h, l);
-          const uint32_t off = tc::kmajor_off(i, 4 * jq, CT::SBOJ);
+          const uint32_t off = tc::kmajor_off(i, r0 + r, CT::SBOJ);
           *reinterpret_cast<uint4*>(img + CT::PH + off) = h;
           *reinterpret_cast<float4*>(img + CT::PL + off) = l;
         }
-        float* mimg = reinterpret_cast<float*>(img + 2 * CT::PSZ);
-        for (int e = tid >> 5; e < 2 * NB; e += blockDim.x >> 5) {
-          const int which = e / NB, jb = e % NB, i = c0 + jb;
-          const float* mu = which == 0 ? a.mu1 : a.mu2;
-          float sv = 0.f;
-          if (mu && i < k)
-            for (int j = lane; j < k; j += 32) sv = fmaf(Otc[jb * XLD + j], mu[j], sv);
-#pragma unroll
-          for (int off = 16; off; off >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, off);
-          if (lane == 0) mimg[which * KP + i] = sv;
-        }
       }
     }
-    if (a.trace_out) {  // ||Phi_new - snapshot||_F^2 over this CTA's columns, fixed order
+    if (a.trace_out) {  // ||Phi_new - snapshot||_F^2 over this CTA's rows, fixed order
       double d2 = 0.0;
-      for (int e = tid; e < KP * NB; e += blockDim.x) {
-        const int r = e % KP, jb = e / KP, col = c0 + jb;
-        if (r < k && col < k) {
-          const float v = Otc[jb * XLD + r];
-          const double d = (double)v - (double)a.trace_snap[(int64_t)col * k + r];
+#pragma unroll 1
+      for (int e = tid; e < KP * RB; e += NT) {
+        const int r = e % RB, c = e / RB, j = r0 + r;
+        if (j < k && c < k) {
+          const float v = F[r * XLD + c];
+          const double d = (double)v - (double)a.trace_snap[(int64_t)c * k + j];
           d2 = fma(d, d, d2);
-          a.trace_snap[(int64_t)col * k + r] = v;
+          a.trace_snap[(int64_t)c * k + j] = v;
         }
       }
 #pragma unroll
       for (int off = 16; off; off >>= 1) d2 += __shfl_xor_sync(0xffffffffu, d2, off);
       __shared__ double tpart[16];
-      if (lane == 0) tpart[tid >> 5] = d2;
+      if (lane == 0) tpart[warp] = d2;
       __syncthreads();
       if (tid == 0) {
         double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += tpart[w];
+#pragma unroll 1
+        for (int w = 0; w < NT / 32; ++w) t += tpart[w];
         a.trace_out[rank] = t;
       }
     }
   }
-  if (timed_out) {
-    if (tid == 0) atomicOr(a.flags, kFlagTimeout);
-  }
+  if (timed_out && tid == 0) atomicOr(a.flags, kFlagTimeout);
   if (rank == 0 && tid == 0 && a.orth_passes) atomicAdd(a.orth_passes, passes);
-  // keep shared memory alive until remote writers are done (bounded: after a
-  // timeout the ranks may stand at different barriers)
-  if (!(early_arrive ? csync_wait() : csync())) {
-    if (tid == 0) atomicOr(a.flags, kFlagTimeout);
-    __nanosleep(100000);  // let copies a stalled exchange left in flight land
+  if (CL > 1) {
+    // keep shared memory alive until remote readers and writers are done
+    // (bounded: after a timeout the ranks may stand at different barriers)
+    if (timed_out) csync_arrive();
+    if (!csync_wait()) {
+      if (tid == 0) atomicOr(a.flags, kFlagTimeout);
+      __nanosleep(100000);  // let copies a stalled exchange left in flight land
+    }
   }
 }
 
@@ -1260,8 +1231,11 @@ __global__ void __launch_bounds__(512, 1) stpm_step_batched(const StpmUpdateArgs
 //   [Z1 Z2] = Phi^T [y1 y2]      A = Phi  (M = i, K = j), B = y1 | y2 (N = 2 TM, K = j)
 //   C   = c0 Z1 Z2 + c2 (Z1 m2 + m1 Z2)   (TMEM -> registers -> shared)
 //   G  += y3^T C                 A = y3   (M = j, K = x), B = C   (N = i, K = x)
-// Z1, Z2 and G live in tensor memory (columns [0, TM), [TM, 2 TM),
-// [2 TM, 2 TM + KP)); G accumulates over the CTA's tiles.  Operands are
+// Z1, Z2 and G live in tensor memory (columns [0, TM), [TM, 2 TM), the hi hi
+// products of G in [2 TM, 2 TM + KP) and the others in the KP columns after);
+// G accumulates over the CTA's tiles.  (Apart, because every accumulation
+// truncates: with one accumulator lambda at k = 100 was 2.7e-6 off after 5
+// tiles per CTA and 4.4e-6 after 13; 1.6e-6 after 13 here.)  Operands are
 // staged hi / lo in shared memory, K-major without swizzle; y3 is staged
 // transposed (node index along K).  An M = 128 operand of KP < 128 rows
 // reads its rows past KP from the buffer after it: their products land in
@@ -1286,7 +1260,8 @@ struct ContractTc {
   static constexpr uint32_t REGION = ((REGION0 > STAGE ? REGION0 : STAGE) + 127) / 128 * 128;
   // alignment slack, m1 | m2, d-sums of the 4 node groups
   static constexpr size_t smem = 1024 + REGION + sizeof(float) * (2 * KP + 4 * KP);
-  static constexpr uint32_t TMEM_COLS = 256;
+  static constexpr uint32_t TMEM_COLS = KP <= 32 ? 128 : KP <= 96 ? 256 : 512;
+  static_assert(2 * TM + 2 * KP <= (int)TMEM_COLS, "tensor memory columns");
   static_assert(KP % 16 == 0 && KP >= 32 && KP <= 112, "tensor-core contraction: KP in [32, 112]");
   static_assert(smem <= 227 * 1024, "tensor-core contraction shared memory");
 };
@@ -1583,9 +1558,24 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
   float* part = reinterpret_cast<float*>(base + C::CH);  // [q][i][jq]
   static_assert(2 * KP * NQ * 4 <= 2 * C::TSZ, "partials fit the C area");
   bool img_timed_out = false;
+  // part -> m_q (mv and mus share storage)
+  auto finish_means = [&]() {
+    __syncthreads();
+    float m = 0.f;
+    if (tid < 2 * KP) {
+      const float* pp = part + (tid / KP) * KP * NQ + (tid % KP) * NQ;
+#pragma unroll 4
+      for (int jq = 0; jq < NQ; ++jq) m += pp[jq];
+    }
+    __syncthreads();  // every read of mus done
+    if (tid < 2 * KP) mv[tid] = m;
+    __syncthreads();
+  };
+  bool need_means = a.phi_img != nullptr;
   if (a.phi_img) {
-    // the previous step kernel wrote Phi's operand image and Phi^T mu1|2:
-    // bulk copies of the hi | lo image (in 4 pieces) and plain loads of m
+    // the previous step kernel wrote Phi's operand image: bulk copies of the
+    // hi | lo image (in 4 pieces); Phi^T mu_q is formed behind the first
+    // tile's Z products
     __syncthreads();  // every thread past its first-tile stores (the barrier init is ordered)
     if (tid == 0) {
       constexpr uint32_t bytes = 2 * C::PSZ, piece = bytes / 4;
@@ -1596,12 +1586,6 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
         bulk_copy_g2s(base + C::PH + q * piece, static_cast<const unsigned char*>(a.phi_img) + q * piece,
                       piece, &bars[2]);
     }
-    const float* mimg = reinterpret_cast<const float*>(static_cast<const unsigned char*>(a.phi_img) +
-                                                       2 * C::PSZ);
-    float m = 0.f;
-    if (tid < 2 * KP) m = mimg[tid];
-    __syncthreads();  // every read of mus done (mv and mus share storage)
-    if (tid < 2 * KP) mv[tid] = m;
     if (!tc::mbar_wait(&bars[2], 0u, tc::wait_limit_or_default(a.wait_limit))) img_timed_out = true;
   } else {
     float v[PT][4];
@@ -1638,15 +1622,7 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
         part[KP * NQ + i * NQ + jq] = p2;
       }
     }
-    __syncthreads();
-    float m = 0.f;
-    if (tid < 2 * KP) {
-      const float* pp = part + (tid / KP) * KP * NQ + (tid % KP) * NQ;
-#pragma unroll 4
-      for (int jq = 0; jq < NQ; ++jq) m += pp[jq];
-    }
-    __syncthreads();  // every read of mus done
-    if (tid < 2 * KP) mv[tid] = m;
+    finish_means();
   }
 
   tc::fence_before_sync();
@@ -1683,14 +1659,42 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       const uint64_t dpl = tc::smem_desc(sbase + C::PL, 128, C::SBOJ);
       const uint64_t dyh = tc::smem_desc(sbase + C::Y1H, 128, C::SBOJ);
       const uint64_t dyl = tc::smem_desc(sbase + C::Y1L, 128, C::SBOJ);
+      // the small products first: every accumulation truncates, so only the
+      // KP / 8 of the hi hi products do so at Z's full size
 #pragma unroll
       for (int ks = 0; ks < KP / 8; ++ks) {
         const uint64_t ko = 16u * ks;
-        tc::mma_tf32(tmem, dph + ko, dyh + ko, iz, ks > 0 ? 1u : 0u);
-        tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, 1u);
+        tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, ks > 0 ? 1u : 0u);
         tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
       }
+#pragma unroll
+      for (int ks = 0; ks < KP / 8; ++ks)
+        tc::mma_tf32(tmem, dph + 16u * ks, dyh + 16u * ks, iz, 1u);
       tc::commit(&bars[0]);
+    }
+    if (need_means) {  // from the image in shared memory (hi + lo = Phi), behind the MMAs
+      need_means = false;
+#pragma unroll
+      for (int t = 0; t < PT; ++t) {
+        const int e = tid + NT * t;
+        int i, jq;
+        task_phi(e, i, jq);
+        if (e < KP * NQ) {
+          const uint32_t off = tc::kmajor_off(i, 4 * jq, C::SBOJ);
+          const float4 h = *reinterpret_cast<const float4*>(base + C::PH + off);
+          const float4 l = *reinterpret_cast<const float4*>(base + C::PL + off);
+          const float v[4] = {h.x + l.x, h.y + l.y, h.z + l.z, h.w + l.w};
+          float p1 = 0.f, p2 = 0.f;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            p1 = fmaf(v[u], mus[4 * jq + u], p1);
+            p2 = fmaf(v[u], mus[KP + 4 * jq + u], p2);
+          }
+          part[i * NQ + jq] = p1;
+          part[KP * NQ + i * NQ + jq] = p2;
+        }
+      }
+      finish_means();
     }
     if (!tc::mbar_wait(&bars[0], ph_z, tc::wait_limit_or_default(a.wait_limit))) timed_out = true;
     ph_z ^= 1u;
@@ -1738,9 +1742,10 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
 #pragma unroll
       for (int ks = 0; ks < TM / 8; ++ks) {
         const uint64_t ko = 16u * ks;
-        tc::mma_tf32(d, dah + ko, dbh + ko, ig, (any || ks > 0) ? 1u : 0u);
-        tc::mma_tf32(d, dah + ko, dbl + ko, ig, 1u);
-        tc::mma_tf32(d, dal + ko, dbh + ko, ig, 1u);
+        const uint32_t acc = (any || ks > 0) ? 1u : 0u;
+        tc::mma_tf32(d, dah + ko, dbh + ko, ig, acc);
+        tc::mma_tf32(d + KP, dah + ko, dbl + ko, ig, acc);
+        tc::mma_tf32(d + KP, dal + ko, dbh + ko, ig, 1u);
       }
       tc::commit(&bars[1]);
     }
@@ -1759,7 +1764,14 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
     for (int c4 = 0; c4 < NQ; c4 += 4) {
       const int ic = cg4 * NQ + c4;
       float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (ok && any) tc::tmem_ld4(tmem + ((uint32_t)(32 * sub) << 16) + (uint32_t)(2 * TM + ic), v);
+      if (ok && any) {
+        const uint32_t at = tmem + ((uint32_t)(32 * sub) << 16) + (uint32_t)(2 * TM + ic);
+        float lo[4];
+        tc::tmem_ld4(at, v);
+        tc::tmem_ld4(at + KP, lo);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] += lo[u];
+      }
       if (j < KP)
 #pragma unroll
         for (int u = 0; u < 4; ++u) stage[(ic + u) * KP + j] = v[u];
@@ -2552,17 +2564,16 @@ cudaError_t launch_step_t(const StpmUpdateArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// step_ctas(KP) CTAs (up to 16, a non-portable cluster size) where the device
+// can co-schedule them, else KP / 16 of 16 rows
 template <int KP>
 cudaError_t launch_step_k(const StpmUpdateArgs& a, cudaStream_t s) {
-  // KP / 8 CTAs (8 columns each; up to 16, a non-portable cluster size) where
-  // the device can co-schedule them, else KP / 16 CTAs of 16 columns; above
-  // KP = 128 always KP / 16 (a cluster holds at most 16 CTAs)
-  if constexpr (KP > 128) {
-    return launch_step_t<KP, KP / 16>(a, s);
+  if constexpr (KP <= 64 || KP > 128) {
+    return launch_step_t<KP, step_ctas(KP)>(a, s);
   } else {
     static int wide = -1;
     if (wide != 0) {
-      cudaError_t e = launch_step_t<KP, KP / 8>(a, s);
+      cudaError_t e = launch_step_t<KP, step_ctas(KP)>(a, s);
       if (e == cudaSuccess) {
         wide = 1;
         return e;
@@ -2606,18 +2617,22 @@ cudaError_t launch_step_batched_t(const StpmUpdateArgs* args, int graphs, cudaSt
 
 template <int KP>
 cudaError_t launch_step_batched_k(const StpmUpdateArgs* args, int graphs, cudaStream_t s) {
-  static int wide = -1;
-  if (wide != 0) {
-    cudaError_t e = launch_step_batched_t<KP, KP / 8>(args, graphs, s);
-    if (e == cudaSuccess) {
-      wide = 1;
-      return e;
+  if constexpr (KP <= 64) {
+    return launch_step_batched_t<KP, step_ctas(KP)>(args, graphs, s);
+  } else {
+    static int wide = -1;
+    if (wide != 0) {
+      cudaError_t e = launch_step_batched_t<KP, step_ctas(KP)>(args, graphs, s);
+      if (e == cudaSuccess) {
+        wide = 1;
+        return e;
+      }
+      if (wide == 1) return e;
+      cudaGetLastError();
+      wide = 0;
     }
-    if (wide == 1) return e;
-    cudaGetLastError();
-    wide = 0;
+    return launch_step_batched_t<KP, KP / 16>(args, graphs, s);
   }
-  return launch_step_batched_t<KP, KP / 16>(args, graphs, s);
 }
 
 }  // namespace
@@ -2708,7 +2723,7 @@ int stpm_step_kp(int k) { return stpm_kp(k); }
 size_t stpm_phi_image_bytes(int k) {
   const int kp = stpm_kp(k);
   if (kp < 32 || kp > 112) return 0;
-  return (size_t)8 * kp * kp + (size_t)8 * kp;  // hi | lo (ContractTc<KP>::PSZ each), m1 | m2
+  return (size_t)8 * kp * kp;  // hi | lo (ContractTc<KP>::PSZ each)
 }
 
 cudaError_t stpm_partial_batched(int mode, int KP, const StpmPartialArgs* args, int graphs,

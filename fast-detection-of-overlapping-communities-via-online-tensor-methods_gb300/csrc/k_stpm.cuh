@@ -38,9 +38,8 @@ struct StpmPartialArgs {
   unsigned* flags;       // device flag word (MMSB_ERR_TIMEOUT of a bounded wait), may be null
   long long wait_limit;  // clock64 cycles a bounded wait may take (0: about one second)
   // tensor-core plain FP32 form (KP <= 112): Phi already split into its TF32
-  // hi / lo operand image, followed by Phi^T mu1 | Phi^T mu2 (2 KP floats),
-  // as the previous step kernel wrote it (stpm_phi_image_bytes); null: the
-  // contraction stages Phi itself
+  // hi / lo operand image, as the previous step kernel wrote it
+  // (stpm_phi_image_bytes); null: the contraction stages Phi itself
   const void* phi_img;
 };
 
@@ -87,7 +86,7 @@ struct StpmUpdateArgs {
   const float* mu1;
   const float* mu2;
   const float* mu3;     // plain: mu_out
-  double c1, c2, scale, count;
+  float c1, c2, scale, inv_count;  // (in FP32: a conversion per thread costs the FP64 pipe)
   float beta;
   float theta3;         // 3 * theta
   float gscale;         // 3 (plain) or 1 (adjoint: G already holds dT)
@@ -95,7 +94,6 @@ struct StpmUpdateArgs {
   unsigned* flags;
   int* orth_passes;      // accumulates the exact Cholesky QR passes (may be null)
   float* orth_err;       // max |Q1^T Q1 - I| before the first-order pass, max over steps (may be null)
-  float* xstash;         // KP x KP scratch in global memory (KP > 128 only)
   long long wait_limit;  // clock64 cycles a bounded wait may take (0: about one second)
   int active;            // batched launches: 0 = no update for this graph in this round
   // online steps: 1 = form Phi (Phi^T Phi)^.2 literally (the first step of a
@@ -105,7 +103,7 @@ struct StpmUpdateArgs {
   // the contraction's operand image of the new Phi (stpm_phi_image_bytes), or
   // null
   void* phi_img;
-  // convergence trace (may be null): CTA q writes sum over its columns of
+  // convergence trace (may be null): CTA q writes sum over its rows of
   // (Phi_new - trace_snap)^2 to trace_out[q] and sets trace_snap = Phi_new there
   float* trace_snap;
   double* trace_out;

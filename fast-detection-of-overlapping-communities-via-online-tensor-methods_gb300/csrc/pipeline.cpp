@@ -729,8 +729,6 @@ static StpmUpdateArgs step_args(mmsb_ctx* c, int step_mode, bool counted) {
     u.orth_passes = c->tbuf<int>("orth_passes", 4);
     u.orth_err = c->tbuf<float>("orth_err", 4);
   }
-  const int kp = stpm_step_kp(c->k);
-  if (kp > 128) u.xstash = c->tbuf<float>("xstash", (size_t)kp * kp);
   u.wait_limit = c->wait_limit;
   u.active = 1;
   return u;
@@ -758,10 +756,10 @@ StpmUpdateArgs stpm_online_update_args(mmsb_ctx* c, const OnlineRound& rd, float
   u.mu1 = c->ymu;
   u.mu2 = c->ymu + k;
   u.mu3 = c->ymu + 2 * k;
-  u.c1 = rd.c1;
-  u.c2 = rd.c2;
-  u.scale = rd.scale;
-  u.count = (double)rd.cnt;
+  u.c1 = (float)rd.c1;
+  u.c2 = (float)rd.c2;
+  u.scale = (float)rd.scale;
+  u.inv_count = (float)(1.0 / (double)rd.cnt);
   u.beta = (float)rd.beta;
   u.gscale = (float)rd.gscale;
   u.phi_general = rd.r == 0 ? 1 : 0;
