@@ -131,7 +131,7 @@ void fill_args(mmsb_batch* B, Bucket& b, int ctas, int64_t rounds) {
       p[G] = StpmPartialArgs{};
       u = StpmUpdateArgs{};
       if (!stpm_online_round(c, r, &rd)) continue;
-      const int need = stpm_partial_grid(rd.cnt, rd.bf16);
+      const int need = stpm_partial_grid(rd.mode, c->k, rd.cnt, rd.bf16);
       const int nb = std::min(ctas, need);
       p[rd.bf16 ? G : 0] =
           stpm_partial_args(c, 0, 1, 2, rd.x0, rd.cnt, rd.c0, rd.c2, rd.bf16, gp, stride, nb);
@@ -179,8 +179,11 @@ void launch_round(mmsb_batch* B, Bucket& b, int64_t r) {
 void autotune(mmsb_batch* B, Bucket& b) {
   int need = 8;
   OnlineRound rd;
-  for (int gi : b.graphs)
-    if (stpm_online_round(B->g[(size_t)gi], 0, &rd)) need = std::max(need, stpm_partial_grid(rd.cnt, rd.bf16));
+  for (int gi : b.graphs) {
+    const mmsb_ctx* c = B->g[(size_t)gi];
+    if (stpm_online_round(c, 0, &rd))
+      need = std::max(need, stpm_partial_grid(rd.mode, c->k, rd.cnt, rd.bf16));
+  }
   std::vector<int> cand;
   for (int c = 8; c < need; c *= 2) cand.push_back(c);
   cand.push_back(need);

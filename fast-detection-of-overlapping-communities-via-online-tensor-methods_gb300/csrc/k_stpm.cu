@@ -1231,11 +1231,12 @@ __global__ void __launch_bounds__(512, 1) stpm_step_batched(const StpmUpdateArgs
 //   [Z1 Z2] = Phi^T [y1 y2]      A = Phi  (M = i, K = j), B = y1 | y2 (N = 2 TM, K = j)
 //   C   = c0 Z1 Z2 + c2 (Z1 m2 + m1 Z2)   (TMEM -> registers -> shared)
 //   G  += y3^T C                 A = y3   (M = j, K = x), B = C   (N = i, K = x)
-// Z1, Z2 and G live in tensor memory (columns [0, TM), [TM, 2 TM), the hi hi
-// products of G in [2 TM, 2 TM + KP) and the others in the KP columns after);
-// G accumulates over the CTA's tiles.  (Apart, because every accumulation
-// truncates: with one accumulator lambda at k = 100 was 2.7e-6 off after 5
-// tiles per CTA and 4.4e-6 after 13; 1.6e-6 after 13 here.)  Operands are
+// Z1, Z2 and G live in tensor memory (columns [0, TM), [TM, 2 TM),
+// [2 TM, 2 TM + KP)); G accumulates over the CTA's tiles.  Every accumulation
+// truncates, so from KP = 64 the small products (hi lo, lo hi) of Z come first
+// and those of G have an accumulator of their own (the next KP columns): lambda
+// at k = 100 was 2.7e-6 off with all in one after 5 tiles per CTA, and is 1.6e-6
+// off after 13.  Below, the chains are short (k = 10: 0.8e-6).  Operands are
 // staged hi / lo in shared memory, K-major without swizzle; y3 is staged
 // transposed (node index along K).  An M = 128 operand of KP < 128 rows
 // reads its rows past KP from the buffer after it: their products land in
@@ -1260,7 +1261,8 @@ struct ContractTc {
   static constexpr uint32_t REGION = ((REGION0 > STAGE ? REGION0 : STAGE) + 127) / 128 * 128;
   // alignment slack, m1 | m2, d-sums of the 4 node groups
   static constexpr size_t smem = 1024 + REGION + sizeof(float) * (2 * KP + 4 * KP);
-  static constexpr uint32_t TMEM_COLS = KP <= 32 ? 128 : KP <= 96 ? 256 : 512;
+  static constexpr bool APART = KP >= 64;
+  static constexpr uint32_t TMEM_COLS = KP <= 96 ? 256 : 512;
   static_assert(2 * TM + 2 * KP <= (int)TMEM_COLS, "tensor memory columns");
   static_assert(KP % 16 == 0 && KP >= 32 && KP <= 112, "tensor-core contraction: KP in [32, 112]");
   static_assert(smem <= 227 * 1024, "tensor-core contraction shared memory");
@@ -1319,10 +1321,10 @@ struct Contract {
   static constexpr int NZ = MODE == kModePlain ? 2 : 3;
   static constexpr int NC = MODE == kModePlain ? 1 : MODE == kModeAdjoint ? 3 : 0;
   // columns i of Phi handled by one CTA: all of them up to KP = 128, above
-  // that blocks of 64 (blockIdx.y), so that Phi's block, the G accumulators
-  // and the staged partial fit one SM; Z, C, G and the d-sums are separable
-  // by column
-  static constexpr int IB = KP <= 128 ? KP : 64;
+  // that halves in FP32 and blocks of 64 in BF16 (blockIdx.y), so that Phi's
+  // block, the G accumulators and the staged partial fit one SM; Z, C, G and
+  // the d-sums are separable by column
+  static constexpr int IB = KP <= 128 ? KP : BF ? 64 : KP / 2;
   static constexpr int NBC = (KP + IB - 1) / IB;  // column blocks (<= 4: one loss slot each)
   static constexpr int PAD = BF ? 8 : 4;   // row strides == 4 words mod 8: conflict-free fragments
   static constexpr int PLD = KP + PAD, LDY = KP + PAD, LDC = TM + PAD;
@@ -1336,9 +1338,22 @@ struct Contract {
   static constexpr int NPHI = BF ? 2 : 1;
   static constexpr size_t tile_bytes =
       sizeof(T) * ((size_t)NPHI * IB * PLD + (size_t)3 * TM * LDY + (size_t)NC * IB * LDC);
-  static constexpr size_t stage_bytes = sizeof(float) * ((size_t)KP * IB + 3 * IB + 4);
+  // the staged partial; the FP32 form's d-sums of the node groups follow it
+  static constexpr size_t DPART = ((size_t)KP * IB + 3 * IB + 4 + 3) / 4 * 4;
+  static constexpr size_t stage_bytes =
+      sizeof(float) * (DPART + (BF ? 0 : (size_t)(TM / 2) * 3 * IB));
   static constexpr size_t region = ((tile_bytes > stage_bytes ? tile_bytes : stage_bytes) + 15) / 16 * 16;
-  static constexpr size_t smem_mma = region + sizeof(float) * (3 * IB + NW + NW * 3 * IB);
+  // m1..3, loss partials, and the warps' d-sums (BF16) or mu1..3 (FP32)
+  static constexpr size_t smem_mma =
+      region + sizeof(float) * (3 * IB + NW + (BF ? NW * 3 * IB : 3 * KP));
+  static_assert(TC || TCBF || smem_mma <= 227 * 1024 - 1024, "contraction shared memory");
+  // FP32 form on the CUDA cores (contract_ffma): thread tiles of the Z products
+  // (4 columns i x XT nodes) and of the G products (8 j x GI columns i)
+  static constexpr int XT = KP >= 96 ? 4 : 2;
+  static constexpr int ZTH = (IB / 4) * (TM / XT);
+  static constexpr int GI = (KP / 8) * (IB / 4) <= NT ? 4 : 8;
+  static constexpr int GTH = (KP / 8) * (IB / GI);
+  static_assert(BF || (ZTH <= NT && GTH <= NT && IB % 8 == 0), "thread tiles");
   static constexpr size_t smem = contract_smem<KP, TC, TCBF>(smem_mma);
   static_assert(NBC <= 4, "one loss slot per column block");
 };
@@ -1659,17 +1674,25 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       const uint64_t dpl = tc::smem_desc(sbase + C::PL, 128, C::SBOJ);
       const uint64_t dyh = tc::smem_desc(sbase + C::Y1H, 128, C::SBOJ);
       const uint64_t dyl = tc::smem_desc(sbase + C::Y1L, 128, C::SBOJ);
-      // the small products first: every accumulation truncates, so only the
-      // KP / 8 of the hi hi products do so at Z's full size
+      if constexpr (C::APART) {  // the small products first
 #pragma unroll
-      for (int ks = 0; ks < KP / 8; ++ks) {
-        const uint64_t ko = 16u * ks;
-        tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, ks > 0 ? 1u : 0u);
-        tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
+        for (int ks = 0; ks < KP / 8; ++ks) {
+          const uint64_t ko = 16u * ks;
+          tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, ks > 0 ? 1u : 0u);
+          tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
+        }
+#pragma unroll
+        for (int ks = 0; ks < KP / 8; ++ks)
+          tc::mma_tf32(tmem, dph + 16u * ks, dyh + 16u * ks, iz, 1u);
+      } else {
+#pragma unroll
+        for (int ks = 0; ks < KP / 8; ++ks) {
+          const uint64_t ko = 16u * ks;
+          tc::mma_tf32(tmem, dph + ko, dyh + ko, iz, ks > 0 ? 1u : 0u);
+          tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, 1u);
+          tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
+        }
       }
-#pragma unroll
-      for (int ks = 0; ks < KP / 8; ++ks)
-        tc::mma_tf32(tmem, dph + 16u * ks, dyh + 16u * ks, iz, 1u);
       tc::commit(&bars[0]);
     }
     if (need_means) {  // from the image in shared memory (hi + lo = Phi), behind the MMAs
@@ -1742,10 +1765,10 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
 #pragma unroll
       for (int ks = 0; ks < TM / 8; ++ks) {
         const uint64_t ko = 16u * ks;
-        const uint32_t acc = (any || ks > 0) ? 1u : 0u;
+        const uint32_t acc = (any || ks > 0) ? 1u : 0u, dl = C::APART ? d + KP : d;
         tc::mma_tf32(d, dah + ko, dbh + ko, ig, acc);
-        tc::mma_tf32(d + KP, dah + ko, dbl + ko, ig, acc);
-        tc::mma_tf32(d + KP, dal + ko, dbh + ko, ig, 1u);
+        tc::mma_tf32(dl, dah + ko, dbl + ko, ig, C::APART ? acc : 1u);
+        tc::mma_tf32(dl, dal + ko, dbh + ko, ig, 1u);
       }
       tc::commit(&bars[1]);
     }
@@ -1766,11 +1789,13 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       float v[4] = {0.f, 0.f, 0.f, 0.f};
       if (ok && any) {
         const uint32_t at = tmem + ((uint32_t)(32 * sub) << 16) + (uint32_t)(2 * TM + ic);
-        float lo[4];
         tc::tmem_ld4(at, v);
-        tc::tmem_ld4(at + KP, lo);
+        if constexpr (C::APART) {
+          float lo[4];
+          tc::tmem_ld4(at + KP, lo);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] += lo[u];
+          for (int u = 0; u < 4; ++u) v[u] += lo[u];
+        }
       }
       if (j < KP)
 #pragma unroll
@@ -2079,6 +2104,242 @@ __device__ __forceinline__ void contract_tc_bf(const StpmPartialArgs& a, int nbl
   if (warp == 0) tc::tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
+// FP32 contraction on the CUDA cores, for the forms that do not fit the
+// tensor-core one (plain above KP = 112, adjoint and loss).  Register-tiled
+// FFMA from shared memory, K (= j, then nodes) in 16-byte words: 4 i x XT nodes
+// x NZ per thread for Z (4 + XT NZ words per 16 XT NZ products), 8 j x GI i for
+// G, accumulated in registers over the CTA's tiles.  It is bound by the shared
+// memory's bandwidth.  The mma.sync form in 3xTF32 that it replaces issues one
+// m16n8k8 per 22 cycles and SM: the adjoint form of 8,192 nodes at k = 100 took
+// 94 us (69 us here), a minibatch step of 8,192 nodes at k = 200 295 us (250 us).
+// And the FFMA sums round to nearest, where the tensor cores' accumulators
+// truncate: the loss's gradient was 1.9e-6 off, 0.07e-6 here.
+template <int KP, int MODE>
+__device__ __forceinline__ void contract_ffma(const StpmPartialArgs& a, int nblocks,
+                                              unsigned char* smraw) {
+  using Cfg = Contract<KP, MODE, false>;
+  constexpr int TM = Cfg::TM, NZ = Cfg::NZ, NC = Cfg::NC, PLD = Cfg::PLD, LDY = Cfg::LDY,
+                LDC = Cfg::LDC, IB = Cfg::IB, NT = Cfg::NT, XT = Cfg::XT, GI = Cfg::GI;
+  // programmatic serialization: wait for the previous kernel (the step that
+  // wrote Phi), then let the next one be scheduled early
+  const int cb = (Cfg::NBC > 1) ? (int)blockIdx.y : 0, i0 = cb * IB;
+  float* Phis = reinterpret_cast<float*>(smraw);  // Phis[ii PLD + j] = Phi_j,i0+ii
+  float* Ys = Phis + IB * PLD;                    // 3 node-major tiles: Ys[q TM LDY + x LDY + j]
+  float* CT = Ys + 3 * TM * LDY;                  // CT[c IB LDC + ii LDC + x]
+  float* mv = reinterpret_cast<float*>(smraw + Cfg::region);  // m1 | m2 | m3 (IB each)
+  float* tred = mv + 3 * IB;
+  float* mus = tred + Cfg::NW;  // mu1..3 (3 KP), then d-sums
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = a.k;
+#pragma unroll 1
+  for (int e = tid; e < 3 * KP; e += NT) {
+    const int which = e / KP, j = e % KP;
+    const float* mu = which == 0 ? a.mu1 : which == 1 ? a.mu2 : a.mu3;
+    mus[e] = (mu && j < k) ? mu[j] : 0.f;
+  }
+  const int64_t ntiles = ceil_div_dev(a.count, TM);
+  auto load_tile = [&](int64_t tile) {  // 16-byte words; columns past the stored row are zero
+    const int64_t x0 = a.begin + tile * TM;
+    const int64_t left = a.begin + a.count - x0;
+    const int nvalid = left < TM ? (int)left : TM;
+    constexpr int NCH = KP / 4, N = 3 * TM * NCH, B = 4;
+#pragma unroll 1
+    for (int e0 = tid; e0 < N; e0 += NT * B) {
+      float4 v[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        const int e = e0 + NT * u, q = e / (TM * NCH), rem = e % (TM * NCH), xx = rem / NCH,
+                  c = rem % NCH;
+        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* Y = q == 0 ? a.y1 : q == 1 ? a.y2 : a.y3;
+        if (e < N && xx < nvalid && 4 * c < a.ldy)
+          v[u] = __ldg(reinterpret_cast<const float4*>(Y + (x0 + xx) * a.ldy + 4 * c));
+      }
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        const int e = e0 + NT * u, q = e / (TM * NCH), rem = e % (TM * NCH), xx = rem / NCH,
+                  c = rem % NCH;
+        if (e < N) *reinterpret_cast<float4*>(Ys + q * TM * LDY + xx * LDY + 4 * c) = v[u];
+      }
+    }
+    return nvalid;
+  };
+  int nvalid = 0;
+  if ((int64_t)blockIdx.x < ntiles) nvalid = load_tile(blockIdx.x);  // (y only: before the wait)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // Phi: loads issued in batches of 8 per thread so that their latencies overlap
+  {
+    constexpr int N = IB * PLD, B = 8;
+#pragma unroll 1
+    for (int e0 = tid; e0 < N; e0 += NT * B) {
+      float v[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        const int e = e0 + NT * u, i = i0 + e / PLD, j = e % PLD;
+        v[u] = (e < N && i < k && j < k) ? __ldg(a.phi + (int64_t)i * k + j) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (e0 + NT * u < N) Phis[e0 + NT * u] = v[u];
+    }
+  }
+  __syncthreads();
+  // m_q = Phi^T mu_q: a column i per 4 lanes
+#pragma unroll 1
+  for (int e = tid >> 2; e < 3 * IB; e += NT / 4) {
+    const float* mu = mus + (e / IB) * KP;
+    const float* ph = Phis + (e % IB) * PLD;
+    float s = 0.f;
+#pragma unroll 4
+    for (int j = tid & 3; j < KP; j += 4) s = fmaf(ph[j], mu[j], s);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if ((tid & 3) == 0) mv[e] = s;
+  }
+  // this thread's Z tile: columns zi + (IB / 4) u, nodes zx .. zx + XT - 1
+  const int zi = tid % (IB / 4), zx = (tid / (IB / 4)) * XT;
+  const bool zlive = tid < Cfg::ZTH;
+  // and G tile: rows 8 gj .. + 7, columns gi + (IB / GI) u
+  const int gj = tid / (IB / GI), gi = tid % (IB / GI);
+  const bool glive = tid < Cfg::GTH;
+  float gacc[8][GI];
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int u = 0; u < GI; ++u) gacc[j][u] = 0.f;
+  float dl[MODE == kModePlain ? 1 : 3][4] = {};
+  float tsum = 0.f;
+  const float cc0 = a.c0, cc2 = a.c2;
+#pragma unroll 1
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += nblocks) {
+    if (tile != (int64_t)blockIdx.x) nvalid = load_tile(tile);
+    __syncthreads();
+    // ---- Z, C and the d-sums
+    if (zlive) {
+      float z[NZ][4][XT];
+#pragma unroll
+      for (int q = 0; q < NZ; ++q)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int x = 0; x < XT; ++x) z[q][u][x] = 0.f;
+#pragma unroll 2
+      for (int j = 0; j < KP; j += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          p[u] = *reinterpret_cast<const float4*>(Phis + (zi + (IB / 4) * u) * PLD + j);
+#pragma unroll
+        for (int q = 0; q < NZ; ++q)
+#pragma unroll
+          for (int x = 0; x < XT; ++x) {
+            const float4 y = *reinterpret_cast<const float4*>(Ys + (q * TM + zx + x) * LDY + j);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              z[q][u][x] = fmaf(p[u].x, y.x, fmaf(p[u].y, y.y, fmaf(p[u].z, y.z, fmaf(p[u].w, y.w, z[q][u][x]))));
+          }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = zi + (IB / 4) * u;
+        const float m1 = mv[i], m2 = mv[IB + i], m3 = mv[2 * IB + i];
+#pragma unroll
+        for (int x = 0; x < XT; ++x) {
+          const bool valid = zx + x < nvalid && i0 + i < k;
+          const float z1 = z[0][u][x], z2 = z[1][u][x];
+          if (MODE == kModePlain) {
+            CT[i * LDC + zx + x] = valid ? cc0 * z1 * z2 + cc2 * (z1 * m2 + m1 * z2) : 0.f;
+            if (valid) dl[0][u] = fmaf(z1, z2, dl[0][u]);
+          } else {
+            const float z3 = z[NZ - 1][u][x];
+            if (MODE == kModeAdjoint) {
+              CT[i * LDC + zx + x] = valid ? cc0 * z2 * z3 + cc2 * (z2 * m3 + m2 * z3) : 0.f;
+              CT[(IB + i) * LDC + zx + x] = valid ? cc0 * z1 * z3 + cc2 * (z1 * m3 + m1 * z3) : 0.f;
+              CT[(2 * IB + i) * LDC + zx + x] = valid ? cc0 * z1 * z2 + cc2 * (z1 * m2 + m1 * z2) : 0.f;
+            }
+            if (valid) {
+              dl[0][u] = fmaf(z2, z3, dl[0][u]);
+              dl[MODE == kModePlain ? 0 : 1][u] = fmaf(z1, z3, dl[MODE == kModePlain ? 0 : 1][u]);
+              dl[MODE == kModePlain ? 0 : 2][u] = fmaf(z1, z2, dl[MODE == kModePlain ? 0 : 2][u]);
+              if (MODE == kModeLoss)
+                tsum += cc0 * z1 * z2 * z3 + cc2 * (z1 * z2 * m3 + z1 * m2 * z3 + m1 * z2 * z3);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+    // ---- G (8 j x GI i per thread) += Yout^T C over this tile's nodes
+    if (NC > 0 && glive) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const float* Yo = Ys + (MODE == kModePlain ? 2 : c) * TM * LDY + 8 * gj;
+        const float* Cc = CT + c * IB * LDC;
+#pragma unroll 2
+        for (int x = 0; x < TM; x += 4) {
+          float4 cv[GI];
+#pragma unroll
+          for (int u = 0; u < GI; ++u)
+            cv[u] = *reinterpret_cast<const float4*>(Cc + (gi + (IB / GI) * u) * LDC + x);
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            float y[8];
+            load8(Yo + (x + h) * LDY, y);
+#pragma unroll
+            for (int u = 0; u < GI; ++u) {
+              const float cx = h == 0 ? cv[u].x : h == 1 ? cv[u].y : h == 2 ? cv[u].z : cv[u].w;
+#pragma unroll
+              for (int j = 0; j < 8; ++j) gacc[j][u] = fmaf(y[j], cx, gacc[j][u]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (MODE == kModeLoss) {
+#pragma unroll
+    for (int off = 16; off; off >>= 1) tsum += __shfl_xor_sync(0xffffffffu, tsum, off);
+    if (lane == 0) tred[warp] = tsum;
+  }
+  // stage this CTA's partial over the dead tiles for the cluster sum
+  // (partial_cluster_sum): G column-major, 3 d-sums, loss
+  float* stage = reinterpret_cast<float*>(smraw);
+  float* dpart = stage + Cfg::DPART;  // d-sums of the TM / XT node groups
+  constexpr int ND = MODE == kModePlain ? 1 : 3;
+  if (NC > 0 && glive) {
+#pragma unroll
+    for (int u = 0; u < GI; ++u) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = gacc[j][u];
+      store8(stage + (gi + (IB / GI) * u) * KP + 8 * gj, v);
+    }
+  }
+  if (zlive) {
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        dpart[((tid / (IB / 4)) * ND + d) * IB + zi + (IB / 4) * u] = dl[d][u];
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int e = tid; e < 3 * IB; e += NT) {
+    float v = 0.f;
+    if (e < ND * IB)
+      for (int x = 0; x < TM / XT; ++x) v += dpart[x * ND * IB + e];
+    stage[KP * IB + e] = v;
+  }
+  if (tid == 0) {
+    float t = 0.f;
+    if (MODE == kModeLoss)
+      for (int w = 0; w < Cfg::NW; ++w) t += tred[w];
+    stage[KP * IB + 3 * IB] = t;
+  }
+  partial_cluster_sum<KP, IB, Cfg::NBC, MODE>(a, stage, cb, i0);
+}
+
 template <int KP, int MODE, bool BF>
 __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblocks) {
   using Cfg = Contract<KP, MODE, BF>;
@@ -2100,7 +2361,11 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
     contract_tc_bf<KP>(a, nblocks, smraw, stage);
     partial_cluster_sum<KP, IB, Cfg::NBC, MODE>(a, stage, 0, 0);
     return;
+  } else if constexpr (!BF) {
+    contract_ffma<KP, MODE>(a, nblocks, smraw);
+    return;
   }
+  if constexpr (BF) {
   // programmatic serialization: wait for the previous kernel (the step that
   // wrote Phi), then let the next one be scheduled early
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -2192,15 +2457,9 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
           const int q = e / (TM * NCH), rem = e % (TM * NCH), xx = rem / NCH, c = rem % NCH;
           v[u] = make_uint4(0u, 0u, 0u, 0u);
           if (e < N) {
-            if (BF) {
-              const T* Y = static_cast<const T*>(q == 0 ? a.yh1 : q == 1 ? a.yh2 : a.yh3);
-              if (xx < nvalid && c * CH < a.ldyh)
-                v[u] = __ldg(reinterpret_cast<const uint4*>(Y + (x0 + xx) * a.ldyh + c * CH));
-            } else {
-              const float* Y = q == 0 ? a.y1 : q == 1 ? a.y2 : a.y3;
-              if (xx < nvalid && c * CH < a.ldy)
-                v[u] = __ldg(reinterpret_cast<const uint4*>(Y + (x0 + xx) * a.ldy + c * CH));
-            }
+            const T* Y = static_cast<const T*>(q == 0 ? a.yh1 : q == 1 ? a.yh2 : a.yh3);
+            if (xx < nvalid && c * CH < a.ldyh)
+              v[u] = __ldg(reinterpret_cast<const uint4*>(Y + (x0 + xx) * a.ldyh + c * CH));
           }
         }
 #pragma unroll
@@ -2222,7 +2481,7 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
       for (int q = 0; q < NZ; ++q)
 #pragma unroll
         for (int r = 0; r < 4; ++r) z[q][r] = 0.f;
-      if (BF) {
+      {
 #pragma unroll 2
         for (int k0 = 0; k0 < KP; k0 += 16) {
           const T* pa = Phis + m0 * PLD + k0 + 2 * t4;
@@ -2239,35 +2498,6 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
             mma_bf16(z[q], afl, bf);
           }
         }
-      } else {
-        float zc[NZ][4];
-#pragma unroll
-        for (int q = 0; q < NZ; ++q)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) zc[q][r] = 0.f;
-#pragma unroll 2
-        for (int k0 = 0; k0 < KP; k0 += 8) {
-          const float* pa = reinterpret_cast<const float*>(Phis) + m0 * PLD + k0 + t4;
-          uint32_t ah[4], al[4];
-          split_tf32(pa[g * PLD], ah[0], al[0]);
-          split_tf32(pa[(g + 8) * PLD], ah[1], al[1]);
-          split_tf32(pa[g * PLD + 4], ah[2], al[2]);
-          split_tf32(pa[(g + 8) * PLD + 4], ah[3], al[3]);
-#pragma unroll
-          for (int q = 0; q < NZ; ++q) {
-            const float* pb = reinterpret_cast<const float*>(Ys) + q * TM * LDY + (n0 + g) * LDY + k0 + t4;
-            uint32_t bh[2], bl[2];
-            split_tf32(pb[0], bh[0], bl[0]);
-            split_tf32(pb[4], bh[1], bl[1]);
-            mma_tf32(z[q], ah, bh);
-            mma_tf32(zc[q], ah, bl);
-            mma_tf32(zc[q], al, bh);
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < NZ; ++q)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) z[q][r] += zc[q][r];
       }
       // epilogue: fragment r holds (i = m0 + g + 8 (r >> 1), x = n0 + 2 t4 + (r & 1))
       float dl[3][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
@@ -2302,11 +2532,7 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           T* dst = CT + c * IB * LDC + (m0 + g + 8 * h) * LDC + n0 + 2 * t4;
-          if (BF) {
-            *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(cv[c][2 * h], cv[c][2 * h + 1]);
-          } else {
-            *reinterpret_cast<float2*>(dst) = make_float2(cv[c][2 * h], cv[c][2 * h + 1]);
-          }
+          *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(cv[c][2 * h], cv[c][2 * h + 1]);
         }
 #pragma unroll
       for (int qd = 0; qd < 3; ++qd) {
@@ -2335,27 +2561,13 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
           for (int c = 0; c < NC; ++c) {
             const T* Yo = Ys + (MODE == kModePlain ? 2 : c) * TM * LDY;
             const T* Cc = CT + c * IB * LDC;
-            if (BF) {
+            {
               uint32_t af[4];
               const int q = lane >> 3, rr = lane & 7;
               ldsm_x4_trans(af, Yo + (k0 + (q >> 1) * 8 + rr) * LDY + m0 + (q & 1) * 8);
               const T* pb = Cc + (n0 + g) * LDC + k0 + 2 * t4;
               const uint32_t bf[2] = {ld_b32(pb), ld_b32(pb + 8)};
               mma_bf16(gacc[u], af, bf);
-            } else {
-              const float* pa = reinterpret_cast<const float*>(Yo) + (k0 + t4) * LDY + m0 + g;
-              uint32_t ah[4], al[4];
-              split_tf32(pa[0], ah[0], al[0]);
-              split_tf32(pa[8], ah[1], al[1]);
-              split_tf32(pa[4 * LDY], ah[2], al[2]);
-              split_tf32(pa[4 * LDY + 8], ah[3], al[3]);
-              const float* pb = reinterpret_cast<const float*>(Cc) + (n0 + g) * LDC + k0 + t4;
-              uint32_t bh[2], bl[2];
-              split_tf32(pb[0], bh[0], bl[0]);
-              split_tf32(pb[4], bh[1], bl[1]);
-              mma_tf32(gacc[u], ah, bh);
-              mma_tf32(gacc[u], ah, bl);
-              mma_tf32(gacc[u], al, bh);
             }
           }
         }
@@ -2401,6 +2613,7 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
     stage[KP * IB + 3 * IB] = t;
   }
   partial_cluster_sum<KP, IB, Cfg::NBC, MODE>(a, stage, cb, i0);
+  }
 }
 
 template <int KP, int MODE, bool BF>
@@ -2437,8 +2650,10 @@ __global__ void tensor_value_kernel(int k, float* __restrict__ phi, const float*
     }
 }
 
+// launch configuration of the contraction; attr holds 2 attributes
 template <int KP, int MODE, bool BF>
-cudaError_t launch_partial_t(const StpmPartialArgs& a, int grid, cudaStream_t s) {
+cudaError_t partial_config(int grid, cudaStream_t s, cudaLaunchConfig_t* cfg,
+                           cudaLaunchAttribute* attr) {
   const size_t smem = Contract<KP, MODE, BF>::smem;
   static bool set = false;
   if (!set) {
@@ -2446,23 +2661,72 @@ cudaError_t launch_partial_t(const StpmPartialArgs& a, int grid, cudaStream_t s)
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     set = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid, (unsigned)Contract<KP, MODE, BF>::NBC, 1);
-  cfg.blockDim = dim3(Contract<KP, MODE, BF>::NT, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[2];
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3((unsigned)grid, (unsigned)Contract<KP, MODE, BF>::NBC, 1);
+  cfg->blockDim = dim3(Contract<KP, MODE, BF>::NT, 1, 1);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = s;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = kPartialCluster;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see contract_body
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg->attrs = attr;
+  cfg->numAttrs = 2;
+  return cudaSuccess;
+}
+
+template <int KP, int MODE, bool BF>
+cudaError_t launch_partial_t(const StpmPartialArgs& a, int grid, cudaStream_t s) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  MMSB_CUDA_TRY((partial_config<KP, MODE, BF>(grid, s, &cfg, attr)));
   MMSB_CUDA_TRY(cudaLaunchKernelEx(&cfg, stpm_contract_kernel<KP, MODE, BF>, a));
   ++g_launch_count;
   return cudaGetLastError();
+}
+
+// CTAs (per column block, a multiple of the cluster size) that run at the
+// same time: clusters of 8 pack into the GPCs, so this is less than one per SM
+// (120 of 152 for the forms that fill an SM)
+template <int KP, int MODE, bool BF>
+int partial_resident_t() {
+  static const int ctas = []() {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    cudaError_t e = partial_config<KP, MODE, BF>(kPartialCluster, nullptr, &cfg, attr);
+    cfg.numAttrs = 1;
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveClusters(&n, stpm_contract_kernel<KP, MODE, BF>, &cfg);
+    if (e != cudaSuccess) cudaGetLastError();
+    n = e == cudaSuccess ? n / Contract<KP, MODE, BF>::NBC : 0;
+    return kPartialCluster * std::max(1, n);
+  }();
+  return ctas;
+}
+
+template <int MODE, bool BF>
+int partial_resident_m(int KP) {
+  switch (KP) {
+    case 32: return partial_resident_t<32, MODE, BF>();
+    case 48: return partial_resident_t<48, MODE, BF>();
+    case 64: return partial_resident_t<64, MODE, BF>();
+    case 80: return partial_resident_t<80, MODE, BF>();
+    case 96: return partial_resident_t<96, MODE, BF>();
+    case 112: return partial_resident_t<112, MODE, BF>();
+    case 128: return partial_resident_t<128, MODE, BF>();
+    case 160: return partial_resident_t<160, MODE, BF>();
+    default: return partial_resident_t<208, MODE, BF>();
+  }
+}
+
+template <bool BF>
+int partial_resident_p(int mode, int KP) {
+  return mode == kModePlain     ? partial_resident_m<kModePlain, BF>(KP)
+         : mode == kModeAdjoint ? partial_resident_m<kModeAdjoint, BF>(KP)
+                                : partial_resident_m<kModeLoss, BF>(KP);
 }
 
 template <int MODE, bool BF>
@@ -2650,18 +2914,16 @@ int stpm_kp(int k) {
   return -1;
 }
 
-int stpm_partial_grid(int64_t count, bool bf16) {
+int stpm_partial_grid(int mode, int k, int64_t count, bool bf16) {
   // at least 64 nodes per CTA (two FP32 tiles, one BF16 tile): measured on
   // 4,096-node minibatches at k = 100, 64 CTAs beat 128 (44 vs 53 us in FP32;
   // staging Phi and the cluster reduction are per-CTA costs)
-  (void)bf16;
   // MMSB_CONTRACT_NODES overrides the 64 nodes per CTA (a tuning override)
   static const int64_t per_cta = []() {
     const char* e = std::getenv("MMSB_CONTRACT_NODES");
     const long v = e ? std::strtol(e, nullptr, 10) : 0;
     return v >= 16 ? (int64_t)v : (int64_t)64;
   }();
-  const int64_t tiles = ceil_div(count, per_cta);
   // MMSB_CONTRACT_CTAS caps the contraction CTAs of single-graph runs (a
   // tuning override; default 2 per SM)
   static const int64_t cap = []() {
@@ -2669,7 +2931,21 @@ int stpm_partial_grid(int64_t count, bool bf16) {
     const long v = e ? std::strtol(e, nullptr, 10) : 0;
     return v > 0 ? (int64_t)v : (int64_t)2 * kNumSMs;
   }();
-  const int64_t g = std::max<int64_t>(1, std::min<int64_t>(tiles, cap));
+  int64_t g = std::max<int64_t>(1, std::min<int64_t>(ceil_div(count, per_cta), cap));
+  // one wave: a second one repeats the per-CTA costs for a few CTAs (8,192
+  // nodes, k = 100: 128 CTAs where 120 fit took 55 / 95 us in the loss and
+  // adjoint forms, 39 / 69 us with 88).  As few CTAs as keep the largest share
+  // of tiles per CTA.  Not the tensor-core plain form with one accumulator
+  // (KP <= 48), where more tiles per CTA cost accuracy.
+  const int KP = stpm_kp(k);
+  const bool truncating = !bf16 && mode == kModePlain && KP <= 48;
+  const int64_t resident = KP < 0 || truncating ? 0
+                           : bf16               ? partial_resident_p<true>(mode, KP)
+                                                : partial_resident_p<false>(mode, KP);
+  if (resident > 0 && g > resident) {
+    const int64_t tiles = ceil_div(count, bf16 ? 64 : 32);
+    g = ceil_div(tiles, ceil_div(tiles, resident));
+  }
   return (int)round_up(g, kPartialCluster);
 }
 

@@ -113,7 +113,7 @@ int stpm_kp(int k);
 int stpm_step_kp(int k);
 // grid of the partial kernel (a multiple of its cluster size); partial
 // blocks written = grid / stpm_partial_cluster()
-int stpm_partial_grid(int64_t count, bool bf16);
+int stpm_partial_grid(int mode, int k, int64_t count, bool bf16);
 int stpm_partial_cluster();
 // bf16: y read from yh1..yh3 and Phi rounded to BF16 (FP32 accumulation);
 // otherwise FP32 operands through the 3xTF32 split

@@ -671,7 +671,7 @@ static PartialOut stpm_partials(mmsb_ctx* c, int mode, int q1, int q2, int q3, i
                                 int64_t count, double c0, double c2, bool bf16 = false,
                                 const void* phi_img = nullptr) {
   const int k = c->k;
-  const int grid = stpm_partial_grid(count, bf16);
+  const int grid = stpm_partial_grid(mode, k, count, bf16);
   const int64_t stride = (int64_t)k * k + 3 * k + 4;
   float* gpart = c->tbuf<float>("gpart", (size_t)grid * stride);
   StpmPartialArgs a = stpm_partial_args(c, q1, q2, q3, begin, count, c0, c2, bf16, gpart, stride, grid);
