@@ -73,6 +73,13 @@ struct mmsb_ctx {
   // (0: about one second); mmsb_set_wait_limit
   long long wait_limit = 0;
 
+  // page-locked slots that large results pass through on their way into
+  // pageable memory (made on first use, freed with the context)
+  static constexpr size_t kHostSlotBytes = (size_t)1 << 20;
+  static constexpr int kHostSlots = 8;
+  void* host_slots = nullptr;
+  cudaEvent_t host_ev[kHostSlots] = {};
+
   ~mmsb_ctx();
   // grow-only named workspace buffer of at least `bytes` bytes
   void* buf(const std::string& name, size_t bytes);

@@ -27,6 +27,9 @@ mmsb_ctx::~mmsb_ctx() {
       cudaEventDestroy(pr.first);
       cudaEventDestroy(pr.second);
     }
+  if (host_slots) cudaFreeHost(host_slots);
+  for (auto& e : host_ev)
+    if (e) cudaEventDestroy(e);
   if (fork_ev) cudaEventDestroy(fork_ev);
   if (join_ev) cudaEventDestroy(join_ev);
   if (s4) cudaStreamDestroy(s4);
