@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(256) stpm_reduce_kernel(StpmReduceArgs a) {
 // first-order product is on the own rows as well.  (Owning columns instead
 // took an exchange of X, of A and of Q1 per pass, the triangular inverse and
 // three k^3 products: a minibatch step, contraction included, took 54 us at
-// k = 100, 20.6 us at k = 10 and 330 us at k = 200; 45, 15.3 and 295 us here.)  Up to KP = 64 one CTA holds everything and
-// nothing is exchanged.
+// k = 100, 20.6 us at k = 10 and 330 us at k = 200; 45, 15.3 and 295 us here.)  At KP = 32 one CTA holds everything
+// and nothing is exchanged.
 //
 // All products are FP32 FMAs (a thread per column, 8 rows at a time, the row
 // operand broadcast from shared memory): mma.sync TF32 in 3xTF32 form gives
@@ -268,10 +268,12 @@ constexpr int kMaxShifts = 3;
 // columns fall into different banks
 __host__ __device__ constexpr int step_xld(int KP) { return KP + 4; }
 
-// CTAs of the step cluster: one up to KP = 64 (the exchanges would cost more
-// than the products they split), KP / 8 to 128, KP / 16 above (at most 16)
+// CTAs of the step cluster: one at KP = 32 (the exchanges would cost more than
+// the products they split), KP / 8 to 128, KP / 16 above (at most 16).  A step of
+// 4,000 nodes at k = 45, contraction included: 35.8 us with one CTA, 29.4 us
+// with KP / 16, 27.8 us with KP / 8; 5,000 nodes at k = 64: 43.6, 33.2, 31.3 us.
 __host__ __device__ constexpr int step_ctas(int KP) {
-  return KP <= 64 ? 1 : KP <= 128 ? KP / 8 : KP / 16;
+  return KP <= 32 ? 1 : KP <= 128 ? KP / 8 : KP / 16;
 }
 
 template <int KP, int CL>
@@ -288,24 +290,9 @@ struct StepSmem {
   // mu1..3, d-sums, original diagonal, diagonal block
   static constexpr size_t floats = (size_t)KP * XLD + recv + 3 * rows + 11 * KP + 128;
   static_assert(KP % CL == 0 && RB % 8 == 0 && BW >= 4, "row blocks of whole 8-row blocks");
-  static_assert(KP <= 256 && (CL > 1 || KP <= 64), "16-byte words per column");
+  static_assert(KP <= 256 && (CL > 1 || KP <= 32), "16-byte words per column");
   static_assert(floats * sizeof(float) <= 227 * 1024 - 1024, "step kernel shared memory");
 };
-
-__device__ __forceinline__ uint32_t tf32_round(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4],
-                                         const uint32_t (&b)[2]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-      "{%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -443,7 +430,7 @@ template <int KP, int CL>
 __device__ float chol_solve(float* A, float* Y, int k, int rows, float* dg, float* dgi,
                             float* dblk, float* rblk, volatile float* s_ratio, float shift) {
   using S = StepSmem<KP, CL>;
-  constexpr int XLD = S::XLD, RB = S::RB, PW = S::PW, BW = S::BW;
+  constexpr int XLD = S::XLD, PW = S::PW, BW = S::BW;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nb = (k + 7) / 8, kk = 8 * nb;
 #pragma unroll 1
@@ -1233,10 +1220,12 @@ __global__ void __launch_bounds__(512, 1) stpm_step_batched(const StpmUpdateArgs
 //   G  += y3^T C                 A = y3   (M = j, K = x), B = C   (N = i, K = x)
 // Z1, Z2 and G live in tensor memory (columns [0, TM), [TM, 2 TM),
 // [2 TM, 2 TM + KP)); G accumulates over the CTA's tiles.  Every accumulation
-// truncates, so from KP = 64 the small products (hi lo, lo hi) of Z come first
-// and those of G have an accumulator of their own (the next KP columns): lambda
-// at k = 100 was 2.7e-6 off with all in one after 5 tiles per CTA, and is 1.6e-6
-// off after 13.  Below, the chains are short (k = 10: 0.8e-6).  Operands are
+// truncates (about 0.3 of an ulp each), so past KP = 32 the products are spread:
+// the small ones (hi lo, lo hi) of Z come first, its large ones go to two or
+// three accumulators, and the small products of G have one of their own.  The
+// first steps of a run, where the iterate is near singular, multiply that error
+// by 10 to 50: after 4 of them Phi was 3.6e-5 off at k = 100 (median of 8 runs)
+// with one chain of each and 1.5e-5 here, 0.9e-5 and 0.6e-5 at k = 33.  Operands are
 // staged hi / lo in shared memory, K-major without swizzle; y3 is staged
 // transposed (node index along K).  An M = 128 operand of KP < 128 rows
 // reads its rows past KP from the buffer after it: their products land in
@@ -1261,9 +1250,13 @@ struct ContractTc {
   static constexpr uint32_t REGION = ((REGION0 > STAGE ? REGION0 : STAGE) + 127) / 128 * 128;
   // alignment slack, m1 | m2, d-sums of the 4 node groups
   static constexpr size_t smem = 1024 + REGION + sizeof(float) * (2 * KP + 4 * KP);
-  static constexpr bool APART = KP >= 64;
-  static constexpr uint32_t TMEM_COLS = KP <= 96 ? 256 : 512;
-  static_assert(2 * TM + 2 * KP <= (int)TMEM_COLS, "tensor memory columns");
+  static constexpr bool SPREAD = KP > 32;
+  // further accumulators of Z1 | Z2: two, or one where two CTAs share an SM
+  static constexpr int NZX = !SPREAD ? 0 : KP <= 64 ? 1 : 2;
+  static constexpr uint32_t ZX = 2 * TM + 2 * KP;
+  static constexpr uint32_t TMEM_COLS = KP <= 64 ? 256 : 512;
+  static_assert(ZX + NZX * 2 * TM <= TMEM_COLS, "tensor memory columns");
+  static_assert(KP <= 64 || smem > 114 * 1024, "512 tensor memory columns: one CTA per SM");
   static_assert(KP % 16 == 0 && KP >= 32 && KP <= 112, "tensor-core contraction: KP in [32, 112]");
   static_assert(smem <= 227 * 1024, "tensor-core contraction shared memory");
 };
@@ -1317,6 +1310,10 @@ struct Contract {
   static constexpr bool TC = MODE == kModePlain && !BF && KP <= 112;
   static constexpr bool TCBF = MODE == kModeAdjoint && BF && KP <= 112;
   using T = typename std::conditional<BF, __nv_bfloat16, float>::type;
+  // two CTAs per SM up to KP = 64 (64 registers a thread: without the bound the
+  // compiler takes 82 at KP = 48, and an iteration of the power method at k = 33,
+  // 10,000 nodes, took 28.8 us against 23.1 us)
+  static constexpr int CTAS = TC && KP <= 64 ? 2 : 1;
   static constexpr int TM = BF ? 64 : 32;  // nodes per tile
   static constexpr int NZ = MODE == kModePlain ? 2 : 3;
   static constexpr int NC = MODE == kModePlain ? 1 : MODE == kModeAdjoint ? 3 : 0;
@@ -1338,22 +1335,27 @@ struct Contract {
   static constexpr int NPHI = BF ? 2 : 1;
   static constexpr size_t tile_bytes =
       sizeof(T) * ((size_t)NPHI * IB * PLD + (size_t)3 * TM * LDY + (size_t)NC * IB * LDC);
-  // the staged partial; the FP32 form's d-sums of the node groups follow it
-  static constexpr size_t DPART = ((size_t)KP * IB + 3 * IB + 4 + 3) / 4 * 4;
-  static constexpr size_t stage_bytes =
-      sizeof(float) * (DPART + (BF ? 0 : (size_t)(TM / 2) * 3 * IB));
-  static constexpr size_t region = ((tile_bytes > stage_bytes ? tile_bytes : stage_bytes) + 15) / 16 * 16;
-  // m1..3, loss partials, and the warps' d-sums (BF16) or mu1..3 (FP32)
-  static constexpr size_t smem_mma =
-      region + sizeof(float) * (3 * IB + NW + (BF ? NW * 3 * IB : 3 * KP));
-  static_assert(TC || TCBF || smem_mma <= 227 * 1024 - 1024, "contraction shared memory");
   // FP32 form on the CUDA cores (contract_ffma): thread tiles of the Z products
   // (4 columns i x XT nodes) and of the G products (8 j x GI columns i)
   static constexpr int XT = KP >= 96 ? 4 : 2;
   static constexpr int ZTH = (IB / 4) * (TM / XT);
   static constexpr int GI = (KP / 8) * (IB / 4) <= NT ? 4 : 8;
   static constexpr int GTH = (KP / 8) * (IB / GI);
+  // the nodes of a tile go to GPARTS thread groups where one leaves most idle
+  // (an adjoint step of 16,384 nodes at k = 20: 36.7 us with one, 29.7 us)
+  static constexpr int GPARTS = NC == 0 ? 1 : 8 * GTH <= NT ? 8 : 4 * GTH <= NT ? 4 : 2 * GTH <= NT ? 2 : 1;
   static_assert(BF || (ZTH <= NT && GTH <= NT && IB % 8 == 0), "thread tiles");
+  // the staged partial; the FP32 form's d-sums of the node groups and the other
+  // thread groups' G follow it
+  static constexpr size_t DPART = ((size_t)KP * IB + 3 * IB + 4 + 3) / 4 * 4;
+  static constexpr size_t stage_bytes =
+      sizeof(float) *
+      (DPART + (BF ? 0 : (size_t)(TM / 2) * 3 * IB + (size_t)(GPARTS - 1) * KP * IB));
+  static constexpr size_t region = ((tile_bytes > stage_bytes ? tile_bytes : stage_bytes) + 15) / 16 * 16;
+  // m1..3, loss partials, and the warps' d-sums (BF16) or mu1..3 (FP32)
+  static constexpr size_t smem_mma =
+      region + sizeof(float) * (3 * IB + NW + (BF ? NW * 3 * IB : 3 * KP));
+  static_assert(TC || TCBF || smem_mma <= 227 * 1024 - 1024, "contraction shared memory");
   static constexpr size_t smem = contract_smem<KP, TC, TCBF>(smem_mma);
   static_assert(NBC <= 4, "one loss slot per column block");
 };
@@ -1382,14 +1384,6 @@ __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(smem_addr(p)));
-}
-
-// v = hi + lo with hi rounded to TF32; lo is passed as full FP32 bits: a TF32
-// MMA reads only the top 19 bits of an operand, so lo enters truncated to
-// TF32 (|error| <= 2^-10 |lo| <= 2^-21 |v|) without a second conversion
-__device__ __forceinline__ void split_tf32(float v, uint32_t& hi, uint32_t& lo) {
-  hi = tf32_round(v);
-  lo = __float_as_uint(v - __uint_as_float(hi));
 }
 
 // The cluster's CTAs staged their partials (column block cb: G block, 3
@@ -1674,16 +1668,22 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       const uint64_t dpl = tc::smem_desc(sbase + C::PL, 128, C::SBOJ);
       const uint64_t dyh = tc::smem_desc(sbase + C::Y1H, 128, C::SBOJ);
       const uint64_t dyl = tc::smem_desc(sbase + C::Y1L, 128, C::SBOJ);
-      if constexpr (C::APART) {  // the small products first
+      if constexpr (C::SPREAD) {
+        // the small products, then the first share of the large ones; the other
+        // shares in accumulators of their own (added in the epilogue)
 #pragma unroll
         for (int ks = 0; ks < KP / 8; ++ks) {
           const uint64_t ko = 16u * ks;
           tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, ks > 0 ? 1u : 0u);
           tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
         }
+        constexpr int SHARE = (KP / 8 + C::NZX) / (C::NZX + 1);
 #pragma unroll
-        for (int ks = 0; ks < KP / 8; ++ks)
-          tc::mma_tf32(tmem, dph + 16u * ks, dyh + 16u * ks, iz, 1u);
+        for (int ks = 0; ks < KP / 8; ++ks) {
+          const int part = ks / SHARE;
+          tc::mma_tf32(tmem + (part > 0 ? C::ZX + 2 * TM * (part - 1) : 0), dph + 16u * ks,
+                       dyh + 16u * ks, iz, part > 0 && ks % SHARE == 0 ? 0u : 1u);
+        }
       } else {
 #pragma unroll
         for (int ks = 0; ks < KP / 8; ++ks) {
@@ -1729,6 +1729,14 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       float z1[8], z2[8];
       tc::tmem_ld8(lb, z1);
       tc::tmem_ld8(lb + TM, z2);
+#pragma unroll
+      for (int part = 0; part < C::NZX; ++part) {
+        float x1[8], x2[8];
+        tc::tmem_ld8(lb + C::ZX + 2 * TM * part, x1);
+        tc::tmem_ld8(lb + C::ZX + 2 * TM * part + TM, x2);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) z1[u] += x1[u], z2[u] += x2[u];
+      }
       if (i < KP) {
         const float m1 = mv[i], m2 = mv[KP + i];
         float cv[8], d = 0.f;
@@ -1765,9 +1773,9 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
 #pragma unroll
       for (int ks = 0; ks < TM / 8; ++ks) {
         const uint64_t ko = 16u * ks;
-        const uint32_t acc = (any || ks > 0) ? 1u : 0u, dl = C::APART ? d + KP : d;
+        const uint32_t acc = (any || ks > 0) ? 1u : 0u, dl = C::SPREAD ? d + KP : d;
         tc::mma_tf32(d, dah + ko, dbh + ko, ig, acc);
-        tc::mma_tf32(dl, dah + ko, dbl + ko, ig, C::APART ? acc : 1u);
+        tc::mma_tf32(dl, dah + ko, dbl + ko, ig, C::SPREAD ? acc : 1u);
         tc::mma_tf32(dl, dal + ko, dbh + ko, ig, 1u);
       }
       tc::commit(&bars[1]);
@@ -1790,7 +1798,7 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       if (ok && any) {
         const uint32_t at = tmem + ((uint32_t)(32 * sub) << 16) + (uint32_t)(2 * TM + ic);
         tc::tmem_ld4(at, v);
-        if constexpr (C::APART) {
+        if constexpr (C::SPREAD) {
           float lo[4];
           tc::tmem_ld4(at + KP, lo);
 #pragma unroll
@@ -2200,8 +2208,8 @@ __device__ __forceinline__ void contract_ffma(const StpmPartialArgs& a, int nblo
   const int zi = tid % (IB / 4), zx = (tid / (IB / 4)) * XT;
   const bool zlive = tid < Cfg::ZTH;
   // and G tile: rows 8 gj .. + 7, columns gi + (IB / GI) u
-  const int gj = tid / (IB / GI), gi = tid % (IB / GI);
-  const bool glive = tid < Cfg::GTH;
+  const int gpart = tid / Cfg::GTH, gt = tid % Cfg::GTH, gj = gt / (IB / GI), gi = gt % (IB / GI);
+  const bool glive = gpart < Cfg::GPARTS;
   float gacc[8][GI];
 #pragma unroll
   for (int j = 0; j < 8; ++j)
@@ -2276,7 +2284,7 @@ __device__ __forceinline__ void contract_ffma(const StpmPartialArgs& a, int nblo
         const float* Yo = Ys + (MODE == kModePlain ? 2 : c) * TM * LDY + 8 * gj;
         const float* Cc = CT + c * IB * LDC;
 #pragma unroll 2
-        for (int x = 0; x < TM; x += 4) {
+        for (int x = 4 * gpart; x < TM; x += 4 * Cfg::GPARTS) {
           float4 cv[GI];
 #pragma unroll
           for (int u = 0; u < GI; ++u)
@@ -2306,6 +2314,7 @@ __device__ __forceinline__ void contract_ffma(const StpmPartialArgs& a, int nblo
   // (partial_cluster_sum): G column-major, 3 d-sums, loss
   float* stage = reinterpret_cast<float*>(smraw);
   float* dpart = stage + Cfg::DPART;  // d-sums of the TM / XT node groups
+  float* gmore = dpart + (TM / 2) * 3 * IB;  // G of the thread groups past the first
   constexpr int ND = MODE == kModePlain ? 1 : 3;
   if (NC > 0 && glive) {
 #pragma unroll
@@ -2313,7 +2322,7 @@ __device__ __forceinline__ void contract_ffma(const StpmPartialArgs& a, int nblo
       float v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = gacc[j][u];
-      store8(stage + (gi + (IB / GI) * u) * KP + 8 * gj, v);
+      store8((gpart ? gmore + (gpart - 1) * KP * IB : stage) + (gi + (IB / GI) * u) * KP + 8 * gj, v);
     }
   }
   if (zlive) {
@@ -2330,6 +2339,21 @@ __device__ __forceinline__ void contract_ffma(const StpmPartialArgs& a, int nblo
     if (e < ND * IB)
       for (int x = 0; x < TM / XT; ++x) v += dpart[x * ND * IB + e];
     stage[KP * IB + e] = v;
+  }
+  if (Cfg::GPARTS > 1) {
+#pragma unroll 1
+    for (int e = 4 * tid; e < KP * IB; e += 4 * NT) {
+      float4 v = *reinterpret_cast<const float4*>(stage + e);
+#pragma unroll
+      for (int q = 0; q < Cfg::GPARTS - 1; ++q) {
+        const float4 w = *reinterpret_cast<const float4*>(gmore + q * KP * IB + e);
+        v.x += w.x;
+        v.y += w.y;
+        v.z += w.z;
+        v.w += w.w;
+      }
+      *reinterpret_cast<float4*>(stage + e) = v;
+    }
   }
   if (tid == 0) {
     float t = 0.f;
@@ -2617,14 +2641,14 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
 }
 
 template <int KP, int MODE, bool BF>
-__global__ void __launch_bounds__(Contract<KP, MODE, BF>::NT) stpm_contract_kernel(StpmPartialArgs a) {
+__global__ void __launch_bounds__(Contract<KP, MODE, BF>::NT, Contract<KP, MODE, BF>::CTAS) stpm_contract_kernel(StpmPartialArgs a) {
   contract_body<KP, MODE, BF>(a, gridDim.x);
 }
 
 // blockIdx.y selects the graph; its first a.nblocks CTAs (a multiple of the
 // cluster size) work, the rest and graphs without nodes this round leave
 template <int KP, int MODE, bool BF>
-__global__ void __launch_bounds__(Contract<KP, MODE, BF>::NT) stpm_contract_batched(const StpmPartialArgs* __restrict__ args) {
+__global__ void __launch_bounds__(Contract<KP, MODE, BF>::NT, Contract<KP, MODE, BF>::CTAS) stpm_contract_batched(const StpmPartialArgs* __restrict__ args) {
   const StpmPartialArgs a = args[blockIdx.y];
   if ((int)blockIdx.x >= a.nblocks || a.count <= 0) return;
   contract_body<KP, MODE, BF>(a, a.nblocks);
@@ -2935,10 +2959,10 @@ int stpm_partial_grid(int mode, int k, int64_t count, bool bf16) {
   // one wave: a second one repeats the per-CTA costs for a few CTAs (8,192
   // nodes, k = 100: 128 CTAs where 120 fit took 55 / 95 us in the loss and
   // adjoint forms, 39 / 69 us with 88).  As few CTAs as keep the largest share
-  // of tiles per CTA.  Not the tensor-core plain form with one accumulator
-  // (KP <= 48), where more tiles per CTA cost accuracy.
+  // of tiles per CTA.  Not the tensor-core plain form with one chain per sum
+  // (KP = 32), where more tiles per CTA cost accuracy.
   const int KP = stpm_kp(k);
-  const bool truncating = !bf16 && mode == kModePlain && KP <= 48;
+  const bool truncating = !bf16 && mode == kModePlain && KP <= 32;
   const int64_t resident = KP < 0 || truncating ? 0
                            : bf16               ? partial_resident_p<true>(mode, KP)
                                                 : partial_resident_p<false>(mode, KP);

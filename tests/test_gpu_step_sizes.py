@@ -1,6 +1,6 @@
 """The k x k step kernel and the reduction behind the power iteration at the
 sizes where their layouts change: k at and beside multiples of 8 (blocks of the
-Cholesky factorisation) and of the padded sizes (32 .. 208: one CTA up to 64,
+Cholesky factorisation) and of the padded sizes (32 .. 208: one CTA at 32,
 KP / 8 CTAs to 128, KP / 16 above).  Whitened data of the model with unit
 noise, started near its components; device against the FP64 oracle.
 
@@ -73,3 +73,18 @@ def test_power_iterations(mm, oracle, k):
     assert abs(trace[-1] - err) < 1e-4 * max(err, 1e-2) + 2e-5 * np.sqrt(k)
     assert rel(phi, phi_o) < max(2e-5, 5 * rel(phi_n, phi_o))
     assert rel(lam, lam_o) < max(6e-5, 5 * rel(lam_n, lam_o))
+
+
+# the adjoint contraction's thread groups: 8 up to k = 32, 4 to 64, 2 to 80
+@pytest.mark.parametrize("k,nx", [(1, 65), (32, 431), (33, 500), (48, 1025), (64, 801), (65, 1000),
+                                  (80, 1300)])
+def test_adjoint_steps(mm, oracle, k, nx):
+    b = -(-nx // 2)
+    y, noisy, phi0 = data(oracle, k, nx, 2000 + k)
+    with pipeline(mm, k, nx, y, stpm_method=mm.STPM_ADJOINT, sweeps=4, minibatch=b) as p:
+        p.stpm(phi0)
+        lam, phi = p.lam(), p.phi()
+    lam_o, phi_o, _ = oracle.stpm_online(y, 1.0, phi0, sweeps=4, minibatch=b, adjoint=True)
+    lam_n, phi_n, _ = oracle.stpm_online(noisy, 1.0, phi0, sweeps=4, minibatch=b, adjoint=True)
+    assert rel(phi, phi_o) < max(2e-5, 5 * rel(phi_n, phi_o))
+    assert rel(lam, lam_o) < max(2e-5, 5 * rel(lam_n, lam_o))
