@@ -26,9 +26,44 @@ __device__ __forceinline__ void fma4(float4& a, float v, const float4& x) {
   a.w = fmaf(v, x.w, a.w);
 }
 
+// a0 (a1) += val P[ci, ch0 (ch1)] over nonzeros j .. j + U - 1, in order, with
+// all U gathers in flight
+template <int U>
+__device__ __forceinline__ void gather_add(const int32_t* __restrict__ ci,
+                                           const float* __restrict__ val, int64_t j,
+                                           const float4* __restrict__ P, int c4, int ch0, int ch1,
+                                           bool h0, bool h1, float4& a0, float4& a1) {
+  int64_t c[U];
+  float v[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    c[u] = ci[j + u];
+    v[u] = 1.f;
+  }
+  if (val) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = val[j + u];
+  }
+  float4 x[U];
+  if (h0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = ldg4(P + c[u] * c4 + ch0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) fma4(a0, v[u], x[u]);
+  }
+  if (h1) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = ldg4(P + c[u] * c4 + ch1);
+#pragma unroll
+    for (int u = 0; u < U; ++u) fma4(a1, v[u], x[u]);
+  }
+}
+
 // G lanes per row; every lane accumulates chunks (base + gl) and (base + G + gl)
-// of the 16-byte column chunks [cb, ce) (rows of P and Y have c4 chunks).
-template <int G>
+// of the 16-byte column chunks [cb, ce) (rows of P and Y have c4 chunks).  U
+// nonzeros' gathers are in flight per lane; an entry is one chain over its
+// row's nonzeros in order, whatever U is.
+template <int G, int U>
 __global__ void __launch_bounds__(256) spmm_rows_kernel(
     const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
     const float* __restrict__ val, int64_t n_rows, const float4* __restrict__ P, int c4,
@@ -43,52 +78,37 @@ __global__ void __launch_bounds__(256) spmm_rows_kernel(
     const bool h0 = ch0 < ce, h1 = ch1 < ce;
     float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
     int64_t j = beg;
-    for (; j + 4 <= end; j += 4) {
-      const int64_t c_0 = ci[j], c_1 = ci[j + 1], c_2 = ci[j + 2], c_3 = ci[j + 3];
-      float v0 = 1.f, v1 = 1.f, v2 = 1.f, v3 = 1.f;
-      if (val) {
-        v0 = val[j];
-        v1 = val[j + 1];
-        v2 = val[j + 2];
-        v3 = val[j + 3];
-      }
-      if (h0) {
-        float4 x0 = ldg4(P + c_0 * c4 + ch0), x1 = ldg4(P + c_1 * c4 + ch0);
-        float4 x2 = ldg4(P + c_2 * c4 + ch0), x3 = ldg4(P + c_3 * c4 + ch0);
-        fma4(a0, v0, x0);
-        fma4(a0, v1, x1);
-        fma4(a0, v2, x2);
-        fma4(a0, v3, x3);
-      }
-      if (h1) {
-        float4 x0 = ldg4(P + c_0 * c4 + ch1), x1 = ldg4(P + c_1 * c4 + ch1);
-        float4 x2 = ldg4(P + c_2 * c4 + ch1), x3 = ldg4(P + c_3 * c4 + ch1);
-        fma4(a1, v0, x0);
-        fma4(a1, v1, x1);
-        fma4(a1, v2, x2);
-        fma4(a1, v3, x3);
-      }
-    }
-    for (; j < end; ++j) {
-      const int64_t c = ci[j];
-      const float v = val ? val[j] : 1.f;
-      if (h0) fma4(a0, v, ldg4(P + c * c4 + ch0));
-      if (h1) fma4(a1, v, ldg4(P + c * c4 + ch1));
-    }
+    for (; j + U <= end; j += U) gather_add<U>(ci, val, j, P, c4, ch0, ch1, h0, h1, a0, a1);
+    if (U > 4)
+      for (; j + 4 <= end; j += 4) gather_add<4>(ci, val, j, P, c4, ch0, ch1, h0, h1, a0, a1);
+    for (; j < end; ++j) gather_add<1>(ci, val, j, P, c4, ch0, ch1, h0, h1, a0, a1);
     if (h0) Y[row * c4 + ch0] = make_float4(alpha * a0.x, alpha * a0.y, alpha * a0.z, alpha * a0.w);
     if (h1) Y[row * c4 + ch1] = make_float4(alpha * a1.x, alpha * a1.y, alpha * a1.z, alpha * a1.w);
   }
 }
 
+// Threads below which a gather kernel leaves the SMs so few warps that the
+// latency of its chains of loads sets the time: then 16 gathers in flight per
+// lane (a row of 250 nonzeros in 16 round trips instead of 63; SpMM of a
+// 1,000 x 1,000 block with 10 columns 34 us -> 11.5 us), else 4 (more cost
+// registers and occupancy: 3,117 -> 2,956 GB/s on 400-column panels).
+constexpr int64_t kFewThreads = (int64_t)kNumSMs * 1024;
+
 template <int G>
 cudaError_t launch_spmm(const int64_t* rp, const int32_t* ci, const float* val, int64_t n_rows,
                         const float* P, int c4, float alpha, float* Y, cudaStream_t s,
                         int cb = 0, int ce = -1) {
-  const int threads = 256;
+  // small grids in small CTAs, so that they spread over the SMs
+  const bool few = n_rows * G < kFewThreads;
+  const int threads = few ? 64 : 256;
   const int64_t blocks = ceil_div(n_rows * G, threads);
-  spmm_rows_kernel<G><<<(unsigned)blocks, threads, 0, s>>>(
-      rp, ci, val, n_rows, reinterpret_cast<const float4*>(P), c4, alpha,
-      reinterpret_cast<float4*>(Y), cb, ce < 0 ? c4 : ce);
+  const float4* p4 = reinterpret_cast<const float4*>(P);
+  float4* y4 = reinterpret_cast<float4*>(Y);
+  if (ce < 0) ce = c4;
+  if (few)
+    spmm_rows_kernel<G, 16><<<(unsigned)blocks, threads, 0, s>>>(rp, ci, val, n_rows, p4, c4, alpha, y4, cb, ce);
+  else
+    spmm_rows_kernel<G, 4><<<(unsigned)blocks, threads, 0, s>>>(rp, ci, val, n_rows, p4, c4, alpha, y4, cb, ce);
   ++g_launch_count;
   return cudaGetLastError();
 }
@@ -241,6 +261,8 @@ __global__ void row_sums_kernel(const int64_t* __restrict__ rp, const float* __r
 
 // ---- unwhitening + normProbVector + threshold ------------------------------
 
+// (U nonzeros' gathers in flight; the sums are one chain per entry in order)
+template <int U>
 __global__ void __launch_bounds__(256) unwhiten_normprob_kernel(
     const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
     const float* __restrict__ val, int64_t n_rows, const float4* __restrict__ P, int c4, int k,
@@ -253,12 +275,12 @@ __global__ void __launch_bounds__(256) unwhiten_normprob_kernel(
   const int ch0 = lane, ch1 = lane + 32;
   const bool h0 = ch0 < c4, h1 = ch1 < c4;
   float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-  for (int64_t j = beg; j < end; ++j) {
-    const int64_t c = ci[j];
-    const float v = val ? val[j] : 1.f;
-    if (h0) fma4(a0, v, ldg4(P + c * c4 + ch0));
-    if (h1) fma4(a1, v, ldg4(P + c * c4 + ch1));
+  int64_t j = beg;
+  if (U > 1) {
+    for (; j + U <= end; j += U) gather_add<U>(ci, val, j, P, c4, ch0, ch1, h0, h1, a0, a1);
+    for (; j + 4 <= end; j += 4) gather_add<4>(ci, val, j, P, c4, ch0, ch1, h0, h1, a0, a1);
   }
+  for (; j < end; ++j) gather_add<1>(ci, val, j, P, c4, ch0, ch1, h0, h1, a0, a1);
   float x[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
   // entries beyond k (panel padding) do not take part
   float pos = 0.f, neg = 0.f;
@@ -437,10 +459,16 @@ cudaError_t unwhiten_normprob(const int64_t* rp, const int32_t* ci, const float*
                               float raw_scale) {
   if (ldp % 4 != 0 || k > 256 || k > ldp) return cudaErrorInvalidValue;
   if (n_rows == 0) return cudaSuccess;
-  const int T = 256;
-  unwhiten_normprob_kernel<<<(unsigned)ceil_div(n_rows * 32, T), T, 0, s>>>(
-      rp, ci, val, n_rows, reinterpret_cast<const float4*>(P), ldp / 4, k, tau, row_offset, pi,
-      bits, raw_scale);
+  const bool few = n_rows * 32 < kFewThreads;
+  const int T = few ? 64 : 256;
+  const unsigned grid = (unsigned)ceil_div(n_rows * 32, T);
+  const float4* p4 = reinterpret_cast<const float4*>(P);
+  if (few)
+    unwhiten_normprob_kernel<16><<<grid, T, 0, s>>>(rp, ci, val, n_rows, p4, ldp / 4, k, tau,
+                                                    row_offset, pi, bits, raw_scale);
+  else
+    unwhiten_normprob_kernel<1><<<grid, T, 0, s>>>(rp, ci, val, n_rows, p4, ldp / 4, k, tau,
+                                                   row_offset, pi, bits, raw_scale);
   ++g_launch_count;
   return cudaGetLastError();
 }
