@@ -120,9 +120,10 @@ cudaError_t colmajor64_to_panel(const double* A, int64_t rows, int cols, int64_t
                                 int ldp, cudaStream_t s);
 cudaError_t panel_to_colmajor64(const float* P, int ldp, int64_t rows, int cols, double* A,
                                 int64_t lda, cudaStream_t s);
-// Scale columns: P[:, j] *= d[j] (row-major panel, FP64 factors).
-cudaError_t panel_scale_cols(float* P, int ldp, int64_t n, int q, const double* d,
-                             cudaStream_t s);
+// out[:, j] = P[:, j] d[j], j < q, the padding columns copied (row-major panels
+// of leading dimension ldp, a multiple of 4; FP64 factors; out == P allowed).
+cudaError_t panel_scale_cols(const float* P, int ldp, int64_t n, int q, const double* d,
+                             float* out, cudaStream_t s);
 cudaError_t fill_f32(float* p, int64_t n, float v, cudaStream_t s);
 cudaError_t fill_f64(double* p, int64_t n, double v, cudaStream_t s);
 // dst[j] = src[j] (FP64 vector ops on device, tiny)

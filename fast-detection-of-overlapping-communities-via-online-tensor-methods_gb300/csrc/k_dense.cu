@@ -12,6 +12,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <type_traits>
 
 namespace mmsb {
 
@@ -43,15 +44,30 @@ __global__ void __launch_bounds__(256) gram_partial_kernel(
       acc[i][j] = 0.f;
     }
   int since = 0;
-  for (int64_t rb = r0; rb < r1; rb += GR) {
-    for (int e = tid; e < GR * GT; e += 256) {
-      const int rr = e / GT, cc = e % GT;
+  // the next stage's rows are loaded while this one is summed (23.4 us -> 20.7 us
+  // for 5,000 rows of 50 columns, where a split has 8 stages)
+  constexpr int PER = GR * GT / 256;
+  float va[PER], vb[PER];
+  auto load = [&](int64_t rb) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = tid + 256 * u, rr = e / GT, cc = e % GT;
       const int64_t row = rb + rr;
       const int ca = ta * GT + cc, cb = tb * GT + cc;
-      As[rr][cc] = (row < r1 && ca < pa) ? A[row * lda + ca] : 0.f;
-      Bs[rr][cc] = (row < r1 && cb < pb) ? B[row * ldb + cb] : 0.f;
+      va[u] = (row < r1 && ca < pa) ? __ldg(A + row * lda + ca) : 0.f;
+      vb[u] = (row < r1 && cb < pb) ? __ldg(B + row * ldb + cb) : 0.f;
+    }
+  };
+  load(r0);
+  for (int64_t rb = r0; rb < r1; rb += GR) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = tid + 256 * u;
+      As[e / GT][e % GT] = va[u];
+      Bs[e / GT][e % GT] = vb[u];
     }
     __syncthreads();
+    if (rb + GR < r1) load(rb + GR);
 #pragma unroll 4
     for (int rr = 0; rr < GR; ++rr) {
       float a[4], b[4];
@@ -88,12 +104,21 @@ __global__ void __launch_bounds__(256) gram_partial_kernel(
     }
 }
 
+// (the splits in order, 8 loads in flight: the FP64 sums stay one chain)
 __global__ void gram_reduce_kernel(const double* __restrict__ partials, int nsplit, int64_t m,
                                    double alpha, double* __restrict__ S) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m;
        e += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int t = 0; t < nsplit; ++t) s += partials[(int64_t)t * m + e];
+    int t = 0;
+    for (; t + 8 <= nsplit; t += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = __ldg(partials + (int64_t)(t + u) * m + e);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    for (; t < nsplit; ++t) s += __ldg(partials + (int64_t)t * m + e);
     S[e] = alpha * s;
   }
 }
@@ -107,13 +132,27 @@ int gram_nsplit(int64_t n, int pa, int pb) {
 
 // ---- M (n x p, FP32 row-major) * F (p x q, FP64 column-major) ----------------
 
+// (float)x in integer arithmetic (round to nearest even): a conversion costs
+// the FP64 unit 64 cycles per warp and SM quarter, and F is converted again in
+// every CTA (with that, and 16-byte loads of F, two concurrent products of n =
+// 50,000, p = q = 200 went from 271 to 258 us; the shared memory's bandwidth sets
+// the rest).  Results outside the normal FP32 range take the conversion.
+__device__ __forceinline__ float narrow(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned e = (hi >> 20) & 0x7ffu;
+  if (e - 897u > 253u) return x == 0.0 ? __uint_as_float(hi & 0x80000000u) : (float)x;
+  const unsigned m = ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+  const unsigned rem = lo & 0x1fffffffu;
+  return __uint_as_float((hi & 0x80000000u) | (m + (rem + (m & 1u) > 0x10000000u ? 1u : 0u)));
+}
+
 constexpr int PT_R = 64, PT_C = 64, PT_K = 32;
 
 __global__ void __launch_bounds__(256) panel_small_kernel(
     const float* __restrict__ M, int ldm, int p, int64_t n, const double* __restrict__ F,
     int ldf, int q, float* __restrict__ Y, int ldy) {
   __shared__ float Ms[PT_R][PT_K + 1];
-  __shared__ float Fs[PT_K][PT_C + 1];
+  __shared__ __align__(16) float Fs[PT_K][PT_C + 4];
   const int tid = threadIdx.x;
   const int tx = tid % 16, ty = tid / 16;
   const int64_t row0 = (int64_t)blockIdx.x * PT_R;
@@ -126,8 +165,8 @@ __global__ void __launch_bounds__(256) panel_small_kernel(
       Ms[rr][kk] = (row < n && k0 + kk < p) ? M[row * ldm + k0 + kk] : 0.f;
     }
     for (int e = tid; e < PT_K * PT_C; e += 256) {
-      const int kk = e / PT_C, cc = e % PT_C;
-      Fs[kk][cc] = (k0 + kk < p && col0 + cc < q) ? (float)F[(int64_t)(col0 + cc) * ldf + k0 + kk]
+      const int kk = e % PT_K, cc = e / PT_K;
+      Fs[kk][cc] = (k0 + kk < p && col0 + cc < q) ? narrow(F[(int64_t)(col0 + cc) * ldf + k0 + kk])
                                                   : 0.f;
     }
     __syncthreads();
@@ -136,8 +175,7 @@ __global__ void __launch_bounds__(256) panel_small_kernel(
       float a[4], b[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) a[i] = Ms[ty * 4 + i][kk];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Fs[kk][tx * 4 + j];
+      *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Fs[kk][tx * 4]);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -303,7 +341,55 @@ __global__ void __launch_bounds__(256, 1) chol_upper_cluster_kernel(int p, const
       DJ[e] = v;
     }
     __syncthreads();
-    if (warp == 0) {  // upper Cholesky of the diagonal block with the drop rule
+    if constexpr (std::is_same<T, double>::value) {
+      // FP64: 4 warps, 2 entries per thread, root-free: entry (i, l) -= a_ci (a_cl
+      // / a_cc), the reciprocal from an FP32 start and formed by every thread (a
+      // warp's FP64 instruction takes 64 cycles here whatever its lanes do, and
+      // a square root and a division per pivot took 1.3k); the rows are scaled by
+      // 1 / sqrt(a_cc) at the end.
+      if (tid < 128) {
+        static_assert(KB == 16, "two entries per thread");
+        for (int c = 0; c < bs; ++c) {
+          const double d = DJ[c * KB + c];
+          double inv = 0.0;
+          if (d > drop2) {
+            if (d > 1e-30 && d < 1e30) {
+              const double y = (double)__frcp_rn((float)d), e = fma(-d, y, 1.0);
+              inv = fma(y * e, 1.0 + e, y);  // e ~ 2^-24: the error is e^3
+            } else {
+              inv = 1.0 / d;
+            }
+          }
+          double v[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int e = tid + 128 * h, i = e % KB, l = e / KB;
+            v[h] = DJ[e];
+            if (i > c && i <= l && l < bs) v[h] = fma(-DJ[i * KB + c], DJ[l * KB + c] * inv, v[h]);
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {  // (row c, read by others, is not written)
+            const int e = tid + 128 * h, i = e % KB, l = e / KB;
+            if (i > c && i <= l && l < bs) DJ[e] = v[h];
+          }
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
+        if (tid < bs) {
+          const double d = DJ[tid * KB + tid];
+          if (!(d == d)) atomicOr(flags, kFlagNonFinite);
+          DI[tid] = d > drop2 ? 1.0 / sqrt(d) : 0.0;
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        double v[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = tid + 128 * h, i = e % KB, l = e / KB;
+          v[h] = i <= l && l < bs ? DJ[e] * DI[i] : 0.0;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) DJ[tid + 128 * h] = v[h];
+      }
+    } else if (warp == 0) {  // upper Cholesky of the diagonal block with the drop rule
       for (int c = 0; c < bs; ++c) {
         if (lane == 0) {
           const T d = DJ[c * KB + c];
@@ -331,6 +417,25 @@ __global__ void __launch_bounds__(256, 1) chol_upper_cluster_kernel(int p, const
     // row block J of this CTA's columns past the block: the forward
     // substitution R_JJ^T x = S_J,l (a thread per column)
     const int i0 = jb + bs;
+    if constexpr (std::is_same<T, double>::value) {
+      // (FP64: 16 lanes per column, lane c its entry c: 16 steps of a product
+      // and an update instead of a chain of 136)
+      for (int l0 = 0; l0 < ncl; l0 += nt / KB) {
+        const int lc = l0 + tid / KB, c = tid % KB, l = lc * CL + rank;
+        const bool live = lc < ncl && l >= i0 && l < p;
+        T* col = Rl + (size_t)(live ? lc : 0) * p + jb;
+        T v = live && c < bs ? col[c] : (T)0;
+        const unsigned half = (lane & 16) ? 0xffff0000u : 0x0000ffffu;
+        if (__any_sync(0xffffffffu, live)) {
+          for (int c2 = 0; c2 < bs; ++c2) {
+            if (c == c2) v *= DI[c2];
+            const T x = __shfl_sync(half, v, c2, KB);
+            if (c > c2) v = fma(-DJ[c * KB + c2], x, v);
+          }
+        }
+        if (live && c < bs) col[c] = v;
+      }
+    } else {
     for (int lc = tid; lc < ncl; lc += nt) {
       const int l = lc * CL + rank;
       if (l < i0 || l >= p) continue;
@@ -340,6 +445,7 @@ __global__ void __launch_bounds__(256, 1) chol_upper_cluster_kernel(int p, const
         for (int c2 = 0; c2 < c; ++c2) x = fma(-DJ[c * KB + c2], col[c2], x);
         col[c] = x * DI[c];
       }
+    }
     }
     // every CTA has gathered S_JJ and row block J is complete everywhere;
     // only now may the owners overwrite the block's own columns with R_JJ
@@ -352,9 +458,15 @@ __global__ void __launch_bounds__(256, 1) chol_upper_cluster_kernel(int p, const
       for (int c = 0; c <= cc; ++c) col[c] = DJ[cc * KB + c];
     }
     if (i0 >= p) break;
-    for (int e = tid; e < bs * (p - i0); e += nt) {
-      const int c = e / (p - i0), i = i0 + e % (p - i0);
-      BR[(size_t)c * p + i] = cluster.map_shared_rank(Rl, i % CL)[(size_t)(i / CL) * p + jb + c];
+    // (a thread per row i, its entries of the block loaded together)
+    for (int i = i0 + (tid >> 1); i < p; i += nt >> 1) {
+      const T* src = cluster.map_shared_rank(Rl, i % CL) + (size_t)(i / CL) * p + jb;
+      T v[KB / 2];
+#pragma unroll
+      for (int u = 0; u < KB / 2; ++u) v[u] = 2 * u + (tid & 1) < bs ? src[2 * u + (tid & 1)] : (T)0;
+#pragma unroll
+      for (int u = 0; u < KB / 2; ++u)
+        if (2 * u + (tid & 1) < bs) BR[(size_t)(2 * u + (tid & 1)) * p + i] = v[u];
     }
     __syncthreads();
     // trailing update of this CTA's columns: a warp per column, lanes on rows
@@ -385,46 +497,61 @@ __global__ void __launch_bounds__(256, 1) chol_upper_cluster_kernel(int p, const
 // Column j of T solves R t = e_j by back substitution in column (axpy) form:
 // for l = j..0: t_l = b_l / R_ll (0 where R_ll == 0), then b_i -= t_l R_il for
 // i < l.  Column l of R is contiguous, so each step is one coalesced axpy;
-// lane i % 32 keeps b_i (and then t_i) in register slot i / 32 (p <= 512).
-__global__ void __launch_bounds__(256) trinv_upper_kernel(int p, const double* __restrict__ R,
-                                                          double* __restrict__ T) {
-  constexpr int kSlots = 16;
+// lane i % 32 keeps b_i (and then t_i) in register slot i / 32 (p <= 32 SLOTS),
+// and column l - 1 is loaded while step l runs: with the load inside the step
+// its latency set the time (144 us at p = 200, 95 us here).
+template <int SLOTS>
+__global__ void __launch_bounds__(64) trinv_upper_kernel(int p, const double* __restrict__ R,
+                                                         double* __restrict__ T) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int j = blockIdx.x * (blockDim.x >> 5) + w;
   if (j >= p) return;
-  double b[kSlots], rinv[kSlots];
+  double b[SLOTS], rinv[SLOTS], next[SLOTS];
+  auto load = [&](int l) {
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q)
+      if (32 * q <= l) next[q] = lane + 32 * q < l ? __ldg(R + (int64_t)l * p + lane + 32 * q) : 0.0;
+  };
+#pragma unroll
+  for (int q = 0; q < SLOTS; ++q) next[q] = 0.0;
+  load(j);
   // 1 / R_ll of the rows this lane holds, all divisions issued together (the
   // FP64 pipe is ~2 operations per clock per SM): the back substitution's
   // dependent chain then has multiplications only
 #pragma unroll
-  for (int q = 0; q < kSlots; ++q) {
+  for (int q = 0; q < SLOTS; ++q) {
     const int i = lane + 32 * q;
     b[q] = i == j ? 1.0 : 0.0;
-    const double rii = i <= j ? R[(int64_t)i * p + i] : 0.0;
-    rinv[q] = rii != 0.0 ? 1.0 / rii : 0.0;
+    rinv[q] = 0.0;
+    if (32 * q <= j) {
+      const double rii = i <= j ? R[(int64_t)i * p + i] : 0.0;
+      rinv[q] = rii != 0.0 ? 1.0 / rii : 0.0;
+    }
   }
   for (int l = j; l >= 0; --l) {
     const int ql = l >> 5, ll = l & 31;
+    double rc[SLOTS];
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) rc[q] = next[q];
+    if (l > 0) load(l - 1);
     double bl = 0.0, il = 0.0;
 #pragma unroll
-    for (int q = 0; q < kSlots; ++q)
+    for (int q = 0; q < SLOTS; ++q)
       if (q == ql) bl = b[q], il = rinv[q];
     bl = __shfl_sync(0xffffffffu, bl, ll);
     il = __shfl_sync(0xffffffffu, il, ll);
-    const double* rc = R + (int64_t)l * p;
     const double tl = bl * il;
     // only slots holding rows i <= l take part: a warp-uniform branch per
     // slot, so the FP64 pipe (~2 DFMA per clock per SM) does no dead work
 #pragma unroll
-    for (int q = 0; q < kSlots; ++q) {
+    for (int q = 0; q < SLOTS; ++q) {
       if (q > ql) break;
-      const int i = lane + 32 * q;
       if (q == ql && lane == ll) b[q] = tl;
-      if (i < l) b[q] = fma(-tl, rc[i], b[q]);
+      if (lane + 32 * q < l) b[q] = fma(-tl, rc[q], b[q]);
     }
   }
 #pragma unroll
-  for (int q = 0; q < kSlots; ++q) {
+  for (int q = 0; q < SLOTS; ++q) {
     const int i = lane + 32 * q;
     if (i < p) T[(int64_t)j * p + i] = i <= j ? b[q] : 0.0;
   }
@@ -1205,29 +1332,38 @@ __global__ void __launch_bounds__(256) oa_correction_kernel(int n, const double*
   E[e] = v;
 }
 
-// columns of X reordered by descending lam (stable on ties by index)
-// (descending, ties by index; NaN ranks last so the ranks always form a
-// permutation, and is reported through the flag word)
-__global__ void sort_eigen_kernel(int n, const double* __restrict__ lam, const double* __restrict__ X,
-                                  double* __restrict__ evals, double* __restrict__ evecs,
-                                  unsigned* flags) {
-  extern __shared__ int order[];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double ki = isnan(lam[i]) ? -INFINITY : lam[i];
-    if (!isfinite(lam[i]) && flags) atomicOr(flags, kFlagNonFinite);
-    int rank = 0;
-    for (int j = 0; j < n; ++j) {
-      const double kj = isnan(lam[j]) ? -INFINITY : lam[j];
-      rank += (kj > ki) || (kj == ki && j < i);
-    }
-    order[rank] = i;
+// Columns of X reordered by descending lam (ties by index; NaN ranks last so
+// the ranks always form a permutation, and is reported through the flag word).
+// A warp per column: its rank, then the copy.  (One CTA for all took 51 us at n =
+// 200, most of it FP64 comparisons at 2 per clock: the keys compare as integers
+// whose order is that of the values.)
+__device__ __forceinline__ long long order_key(double v) {
+  if (isnan(v)) v = -INFINITY;
+  if (v == 0.0) v = 0.0;  // -0 ties with +0
+  const long long b = __double_as_longlong(v);
+  return b < 0 ? (long long)0x8000000000000000ull - b : b;
+}
+
+__global__ void __launch_bounds__(256) sort_eigen_kernel(int n, const double* __restrict__ lam,
+                                                         const double* __restrict__ X,
+                                                         double* __restrict__ evals,
+                                                         double* __restrict__ evecs,
+                                                         unsigned* flags) {
+  const int lane = threadIdx.x & 31, i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i >= n) return;
+  const double li = lam[i];
+  const long long ki = order_key(li);
+  int rank = 0;
+  for (int j = lane; j < n; j += 32) {
+    const long long kj = order_key(lam[j]);
+    rank += (kj > ki) || (kj == ki && j < i);
   }
-  __syncthreads();
-  for (int64_t e = threadIdx.x; e < (int64_t)n * n; e += blockDim.x) {
-    const int r = (int)(e % n), c = (int)(e / n);
-    evecs[e] = X[(int64_t)order[c] * n + r];
+  rank = __reduce_add_sync(0xffffffffu, rank);
+  if (lane == 0) {
+    evals[rank] = li;
+    if (!isfinite(li) && flags) atomicOr(flags, kFlagNonFinite);
   }
-  for (int c = threadIdx.x; c < n; c += blockDim.x) evals[c] = lam[order[c]];
+  for (int r = lane; r < n; r += 32) evecs[(int64_t)rank * n + r] = X[(int64_t)i * n + r];
 }
 
 // P (rows x q, row-major panel ld) gets column `col` = v (FP64 vector, length rows)
@@ -1316,14 +1452,35 @@ __global__ void panel_to_colmajor_kernel(const float* __restrict__ P, int ldp, i
   }
 }
 
-__global__ void scale_cols_kernel(float* __restrict__ P, int ldp, int64_t n, int q,
-                                  const double* __restrict__ d) {
-  const int64_t total = n * q;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = e / q;
-    const int c = (int)(e % q);
-    P[r * ldp + c] = (float)(P[r * ldp + c] * d[c]);
+// out = P with column j < q scaled by d[j] (row-major, ld a multiple of 4, also
+// in place).  A warp per row, 16 bytes per lane; the factor as a pair of floats,
+// P dh + P dl in one fma, rounds as the FP64 product does but for its ties (an
+// FP64 multiplication and two conversions per entry made it 35 us for 50,000 x
+// 100; 15 us here, the copy before it included).
+__global__ void __launch_bounds__(256) scale_cols_kernel(const float4* __restrict__ P, int ld4,
+                                                         int64_t n, int q,
+                                                         const double* __restrict__ d,
+                                                         float4* __restrict__ out) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int c0 = 0; c0 < ld4; c0 += 32) {
+    const int c4 = c0 + lane;
+    float dh[4], dl[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int c = 4 * c4 + u;
+      const double v = c4 < ld4 && c < q ? d[c] : 1.0;
+      dh[u] = (float)v;
+      dl[u] = (float)(v - (double)dh[u]);
+    }
+    if (c4 >= ld4) continue;
+    for (int64_t r = (int64_t)blockIdx.x * nw + (threadIdx.x >> 5); r < n; r += (int64_t)gridDim.x * nw) {
+      float4 x = P[r * ld4 + c4];
+      x.x = fmaf(x.x, dh[0], x.x * dl[0]);
+      x.y = fmaf(x.y, dh[1], x.y * dl[1]);
+      x.z = fmaf(x.z, dh[2], x.z * dl[2]);
+      x.w = fmaf(x.w, dh[3], x.w * dl[3]);
+      out[r * ld4 + c4] = x;
+    }
   }
 }
 
@@ -1439,8 +1596,15 @@ static cudaError_t chol_upper_drop_t(int p, const double* S, int lds, double* R,
   // columns and one row block fit shared memory, else one CTA
   constexpr int KB = 16;
   static int wide = -1;
+  if (p <= 64) {
+    // the blocked form on one CTA, in FP64 for either type (64 us at p = 50 with
+    // a column at a time and R in global memory, 51 us here)
+    const size_t sm = sizeof(double) * (size_t)(p + KB) * p;
+    cudaError_t e = launch_chol_cluster<1, KB, double>(p, S, lds, R, drop2, flags, sm, s);
+    if (e == cudaSuccess) ++g_launch_count;
+    return e;
+  }
   for (int cl : {16, 8}) {
-    if (p <= 64) break;
     if (cl == 16 && wide == 0) continue;
     const size_t sm = sizeof(T) * ((size_t)((p + cl - 1) / cl) + KB) * p;
     if (sm > 200 * 1024) break;
@@ -1473,9 +1637,11 @@ cudaError_t chol_upper_drop_f32(int p, const double* S, int lds, double* R, unsi
 cudaError_t trinv_upper(int p, const double* R, double* T, cudaStream_t s) {
   if (p > 512) return cudaErrorInvalidValue;
   // two columns per CTA: the FP64 work spreads over ~p / 2 SMs
-  const int warps = 2;
-  trinv_upper_kernel<<<(unsigned)ceil_div(p, warps), warps * 32, (size_t)warps * p * sizeof(double),
-                       s>>>(p, R, T);
+  const unsigned grid = (unsigned)ceil_div(p, 2);
+  if (p <= 64) trinv_upper_kernel<2><<<grid, 64, 0, s>>>(p, R, T);
+  else if (p <= 128) trinv_upper_kernel<4><<<grid, 64, 0, s>>>(p, R, T);
+  else if (p <= 256) trinv_upper_kernel<8><<<grid, 64, 0, s>>>(p, R, T);
+  else trinv_upper_kernel<16><<<grid, 64, 0, s>>>(p, R, T);
   ++g_launch_count;
   return cudaGetLastError();
 }
@@ -1556,9 +1722,13 @@ cudaError_t panel_to_colmajor64(const float* P, int ldp, int64_t rows, int cols,
   return cudaGetLastError();
 }
 
-cudaError_t panel_scale_cols(float* P, int ldp, int64_t n, int q, const double* d,
-                             cudaStream_t s) {
-  scale_cols_kernel<<<grid_for(n * q), 256, 0, s>>>(P, ldp, n, q, d);
+cudaError_t panel_scale_cols(const float* P, int ldp, int64_t n, int q, const double* d,
+                             float* out, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  if (ldp % 4 != 0) return cudaErrorInvalidValue;
+  const unsigned grid = (unsigned)std::min<int64_t>(8 * kNumSMs, ceil_div(n, 8));
+  scale_cols_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const float4*>(P), ldp / 4, n, q, d,
+                                         reinterpret_cast<float4*>(out));
   ++g_launch_count;
   return cudaGetLastError();
 }
@@ -1625,7 +1795,7 @@ cudaError_t oa_correction(int n, const double* A, const double* XtX, const doubl
 
 cudaError_t sort_eigen(int n, const double* lam, const double* X, double* evals, double* evecs,
                        unsigned* flags, cudaStream_t s) {
-  sort_eigen_kernel<<<1, 1024, sizeof(int) * n, s>>>(n, lam, X, evals, evecs, flags);
+  sort_eigen_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, s>>>(n, lam, X, evals, evecs, flags);
   ++g_launch_count;
   return cudaGetLastError();
 }

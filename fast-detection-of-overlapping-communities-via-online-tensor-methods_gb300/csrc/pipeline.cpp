@@ -461,8 +461,6 @@ void pipeline_whiten(mmsb_ctx* c, const double* const* sketches, bool finish) {
   double* Linv_b = c->tbuf<double>("Linv_b", (size_t)k);
   c->Ub = c->tbuf<float>("Ub", (size_t)c->nB * ldk);
   c->Uc = c->tbuf<float>("Uc", (size_t)c->nC * ldk);
-  float* Vc = c->tbuf<float>("Vc", (size_t)c->nB * ldk);
-  float* Vb = c->tbuf<float>("Vb", (size_t)c->nC * ldk);
 
   // pinv_Nystrom_sparse_component (Spectral.cpp:296-315) of
   //   Zc_den = inv Gx_c^T Gx_b (n_C x n_B), sketch R_c (n_B x 2k)
@@ -473,14 +471,14 @@ void pipeline_whiten(mmsb_ctx* c, const double* const* sketches, bool finish) {
     const DevCsr *Gin, *Gout_t, *Gout, *Gin_t;
     int64_t n_in, n_out;
     float* Rk;
-    float* V;
+    const float* V;  // the Nystrom step's U panel
     float* U;
     double* Linv;
     const char* tag;
     cudaStream_t st, aux;  // aux: the side's helper stream in its Nystrom step
   } sides[2] = {
-      {&XB, &XCt, &XC, &XBt, c->nB, c->nC, R[0], Vc, c->Uc, Linv_c, "zc", s, c->s3},
-      {&XC, &XBt, &XB, &XCt, c->nC, c->nB, R[1], Vb, c->Ub, Linv_b, "zb", c->s2, c->s4},
+      {&XB, &XCt, &XC, &XBt, c->nB, c->nC, R[0], nullptr, c->Uc, Linv_c, "zc", s, c->s3},
+      {&XC, &XBt, &XB, &XCt, c->nC, c->nB, R[1], nullptr, c->Ub, Linv_b, "zb", c->s2, c->s4},
   };
   ck(cudaEventRecord(c->fork_ev, s), "fork");
   ck(cudaStreamWaitEvent(c->s2, c->fork_ev, 0), "fork wait");
@@ -503,14 +501,14 @@ void pipeline_whiten(mmsb_ctx* c, const double* const* sketches, bool finish) {
     spmm(c, *sd.Gout, XR, ldp, 1.f, T1, st);                    // Gout XR     (n_X x p)
     spmm(c, *sd.Gin_t, T1, ldp, (float)inv, Gram, st);          // X^T X R     (n_in x p)
     Nys ny = svd_sym_nystrom(c, sd.tag, Gram, ldp, p, nullptr, sd.n_in, st, sd.aux);  // V, sigma
-    ck(cudaMemcpyAsync(sd.V, ny.U, sizeof(float) * sd.n_in * ldk, cudaMemcpyDeviceToDevice, st), "V");
+    sd.V = ny.U;
     // U = X V diag(sqrt(pinv(sigma)));  Linv = pinv(sqrt(sigma))  (Spectral.cpp:235-244, 307)
     ck(sqrt_pinv(k, ny.sig, tol, Linv_sqrt, sd.Linv, st), "Linv");
-    ck(cudaMemcpyAsync(VL, sd.V, sizeof(float) * sd.n_in * ldk, cudaMemcpyDeviceToDevice, st), "VL");
-    ck(panel_scale_cols(VL, ldk, sd.n_in, k, Linv_sqrt, st), "VL scale");
+    ck(panel_scale_cols(sd.V, ldk, sd.n_in, k, Linv_sqrt, VL, st), "VL scale");
     spmm(c, *sd.Gin, VL, ldk, 1.f, T3, st);
     spmm(c, *sd.Gout_t, T3, ldk, (float)inv, sd.U, st);
   }
+  const float *Vc = sides[0].V, *Vb = sides[1].V;
   if (!upload) {  // after side zc on this stream
     make_sketch(2, s);
     means();
@@ -541,8 +539,7 @@ void pipeline_whiten(mmsb_ctx* c, const double* const* sketches, bool finish) {
     ck(cudaEventRecord(c->fork_ev, s), "fork");
     ck(cudaStreamWaitEvent(s2, c->fork_ev, 0), "fork wait");
     // Z_B_part1 = Zb_num V_b diag(Linv_b), Zb_num = inv Gx_a^T Gx_c (Util.cpp:96-97)
-    ck(cudaMemcpyAsync(VLb, Vb, sizeof(float) * c->nC * ldk, cudaMemcpyDeviceToDevice, s2), "VL");
-    ck(panel_scale_cols(VLb, ldk, c->nC, k, Linv_b, s2), "Vb scale");
+    ck(panel_scale_cols(Vb, ldk, c->nC, k, Linv_b, VLb, s2), "Vb scale");
     spmm(c, XC, VLb, ldk, 1.f, T3b, s2);
     spmm(c, XAt, T3b, ldk, (float)inv, c->Zb1, s2);
     ck(gram_tsk(c->Zb1, ldk, k, R[2], ldp, p, c->nA, 1.0, Q1, part2, cap, s2), "Zb1^T R");
@@ -551,8 +548,7 @@ void pipeline_whiten(mmsb_ctx* c, const double* const* sketches, bool finish) {
     ck(cudaEventRecord(c->join_ev, s2), "join");
   }
   // Z_C_part1 = Zc_num V_c diag(Linv_c), Zc_num = inv Gx_a^T Gx_b (Util.cpp:83-84)
-  ck(cudaMemcpyAsync(VL, Vc, sizeof(float) * c->nB * ldk, cudaMemcpyDeviceToDevice, s), "VL");
-  ck(panel_scale_cols(VL, ldk, c->nB, k, Linv_c, s), "Vc scale");
+  ck(panel_scale_cols(Vc, ldk, c->nB, k, Linv_c, VL, s), "Vc scale");
   spmm(c, XB, VL, ldk, 1.f, T3);
   spmm(c, XAt, T3, ldk, (float)inv, c->Zc1);
   // core = U_c^T Zc_den U_b = inv (Gx_c U_c)^T (Gx_b U_b)  (Util.cpp:90-94)
@@ -571,8 +567,7 @@ void pipeline_whiten(mmsb_ctx* c, const double* const* sketches, bool finish) {
   // W = U_w diag(pinv(sqrt(sigma_w)))  (Util.cpp:116-123)
   Nys nw = svd_sym_nystrom(c, "w", Am, ldm2, m2, Bm, c->nA, s, c->s2);
   ck(sqrt_pinv(k, nw.sig, tol, nullptr, Linv_sqrt, s), "Lw");
-  ck(cudaMemcpyAsync(c->W, nw.U, sizeof(float) * c->nA * ldk, cudaMemcpyDeviceToDevice, s), "W");
-  ck(panel_scale_cols(c->W, ldk, c->nA, k, Linv_sqrt, s), "W scale");
+  ck(panel_scale_cols(nw.U, ldk, c->nA, k, Linv_sqrt, c->W, s), "W scale");
   c->have_white = true;
   pipeline_ydata(c);
   if (finish) pipeline_whiten_finish(c);
