@@ -81,10 +81,12 @@ size_t gram_tsk_partials(int64_t n, int pa, int pb);
 // columns q..ldy-1 of Y are zeroed.
 cudaError_t panel_times_small(const float* M, int ldm, int p, int64_t n, const double* F, int ldf,
                               int q, float* Y, int ldy, cudaStream_t s);
-// C (m x n) = alpha * op(A) op(B) + beta * C, FP64 column-major, small sizes.
+// C (m x n) = alpha * op(A) op(B) + beta * C0, FP64 column-major, small sizes
+// (C0 with C's leading dimension, not read when beta is 0; C0 == C allowed, C
+// apart from A and B).
 cudaError_t dgemm_small(bool ta, bool tb, int m, int n, int k, double alpha, const double* A,
-                        int lda, const double* B, int ldb, double beta, double* C, int ldc,
-                        cudaStream_t s);
+                        int lda, const double* B, int ldb, double beta, const double* C0, double* C,
+                        int ldc, cudaStream_t s);
 // Upper Cholesky S = R^T R with drop tolerance: a pivot <= drop2 zeroes row j of R.
 cudaError_t chol_upper_drop(int p, const double* S, int lds, double* R, double drop2,
                             unsigned* flags, cudaStream_t s);

@@ -27,8 +27,8 @@ constexpr int GCHUNK = 256; // rows accumulated in FP32 before the FP64 add
 __global__ void __launch_bounds__(256) gram_partial_kernel(
     const float* __restrict__ A, int lda, int pa, const float* __restrict__ B, int ldb, int pb,
     int64_t n, int64_t rows_per_split, double* __restrict__ partials) {
-  __shared__ float As[GR][GT + 1];
-  __shared__ float Bs[GR][GT + 1];
+  __shared__ __align__(16) float As[GR][GT + 4];
+  __shared__ __align__(16) float Bs[GR][GT + 4];
   const int ta = blockIdx.x, tb = blockIdx.y, split = blockIdx.z;
   const int tid = threadIdx.x;
   const int tx = tid % 16, ty = tid / 16;  // 4x4 patch at (ty*4, tx*4)
@@ -43,9 +43,12 @@ __global__ void __launch_bounds__(256) gram_partial_kernel(
       accd[i][j] = 0.0;
       acc[i][j] = 0.f;
     }
+  // A split has up to 8 stages and often an SM to itself: the next stage's rows
+  // are loaded while this one is summed, and patches past the columns are left
+  // out, since the shared memory's bandwidth sets the time of a stage (5,000 rows
+  // of 50 columns 23.4 -> 14.3 us, 1,000 rows of 10 columns 20 -> 11.9 us).
+  const bool live = ta * GT + ty * 4 < pa && tb * GT + tx * 4 < pb;
   int since = 0;
-  // the next stage's rows are loaded while this one is summed (23.4 us -> 20.7 us
-  // for 5,000 rows of 50 columns, where a split has 8 stages)
   constexpr int PER = GR * GT / 256;
   float va[PER], vb[PER];
   auto load = [&](int64_t rb) {
@@ -68,21 +71,21 @@ __global__ void __launch_bounds__(256) gram_partial_kernel(
     }
     __syncthreads();
     if (rb + GR < r1) load(rb + GR);
-#pragma unroll 4
-    for (int rr = 0; rr < GR; ++rr) {
-      float a[4], b[4];
+    if (live) {
+#pragma unroll 8
+      for (int rr = 0; rr < GR; ++rr) {
+        float a[4], b[4];
+        *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[rr][ty * 4]);
+        *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Bs[rr][tx * 4]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[rr][ty * 4 + i];
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[rr][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      }
     }
     __syncthreads();
     since += GR;
-    if (since >= GCHUNK) {
+    if (live && since >= GCHUNK) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -197,31 +200,38 @@ __global__ void __launch_bounds__(256) panel_small_kernel(
 
 // ---- small FP64 GEMM ------------------------------------------------------------
 
-template <int T>
-__global__ void __launch_bounds__(256) dgemm_small_kernel(bool ta, bool tb, int m, int n, int k,
-                                                          double alpha, const double* __restrict__ A,
-                                                          int lda, const double* __restrict__ B,
-                                                          int ldb, double beta,
-                                                          double* __restrict__ C, int ldc) {
-  constexpr int KC = 32, RG = 256 / T, RI = T / RG;  // thread: rows ty + RG*i, col tx
+// FP64 FMAs go at 2 per clock and SM (64 cycles per warp and SM quarter), so the
+// time is the largest number of warps on one quarter, times k: 8 x 8 tiles, an
+// entry per thread, spread the work in units of a warp.  (16 x 16 tiles of 8
+// warps, with k rounded up to 32: the 56 products of a whitening took 32 us on
+// average with 200 columns, 27 us here, 4.2 and 3.3 us with 10.)  A product of a matrix with its own transpose computes one
+// triangle of tiles: (i, j) and (j, i) are the same sums, bit for bit.
+constexpr int DG_T = 8, DG_K = 64;
+
+__global__ void __launch_bounds__(DG_T * DG_T) dgemm_small_kernel(
+    bool ta, bool tb, bool sym, int m, int n, int k, double alpha, const double* __restrict__ A,
+    int lda, const double* __restrict__ B, int ldb, double beta, const double* __restrict__ C0,
+    double* __restrict__ C, int ldc) {
+  constexpr int T = DG_T, KC = DG_K, NT = T * T;
+  if (sym && blockIdx.x > blockIdx.y) return;
   __shared__ double As[T][KC + 1];
   __shared__ double Bs[KC][T + 1];
   const int tid = threadIdx.x;
   const int tx = tid % T, ty = tid / T;
   const int i0 = blockIdx.x * T, j0 = blockIdx.y * T;
-  double acc[RI];
-#pragma unroll
-  for (int i = 0; i < RI; ++i) acc[i] = 0.0;
+  double acc = 0.0;
   for (int k0 = 0; k0 < k; k0 += KC) {
-    for (int e = tid; e < T * KC; e += 256) {
-      {  // As[ii][kk] = op(A)[i0+ii, k0+kk]; consecutive threads walk ii (column-major A)
+#pragma unroll
+    for (int u = 0; u < KC / T; ++u) {
+      const int e = tid + NT * u;
+      {  // As[ii][kk] = op(A)[i0+ii, k0+kk]; consecutive threads walk a column of A
         const int ii = ta ? e / KC : e % T, kk = ta ? e % KC : e / T;
         const int gi = i0 + ii, gk = k0 + kk;
         double v = 0.0;
         if (gi < m && gk < k) v = ta ? A[(int64_t)gi * lda + gk] : A[(int64_t)gk * lda + gi];
         As[ii][kk] = v;
       }
-      {  // Bs[kk][jj] = op(B)[k0+kk, j0+jj]; consecutive threads walk kk (column-major B)
+      {  // Bs[kk][jj] = op(B)[k0+kk, j0+jj]; consecutive threads walk a column of B
         const int kk = tb ? e / T : e % KC, jj = tb ? e % T : e / KC;
         const int gk = k0 + kk, gj = j0 + jj;
         double v = 0.0;
@@ -230,21 +240,17 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(bool ta, bool tb, int 
       }
     }
     __syncthreads();
+    const int kn = k - k0 < KC ? k - k0 : KC;
 #pragma unroll 4
-    for (int kk = 0; kk < KC; ++kk) {
-      const double b = Bs[kk][tx];
-#pragma unroll
-      for (int i = 0; i < RI; ++i) acc[i] = fma(As[ty + RG * i][kk], b, acc[i]);
-    }
+    for (int kk = 0; kk < kn; ++kk) acc = fma(As[ty][kk], Bs[kk][tx], acc);
     __syncthreads();
   }
-#pragma unroll
-  for (int i = 0; i < RI; ++i) {
-    const int gi = i0 + ty + RG * i, gj = j0 + tx;
-    if (gi < m && gj < n) {
-      double* c = C + (int64_t)gj * ldc + gi;
-      *c = alpha * acc[i] + (beta == 0.0 ? 0.0 : beta * *c);
-    }
+  const int gi = i0 + ty, gj = j0 + tx;
+  if (gi < m && gj < n) {
+    const int64_t at = (int64_t)gj * ldc + gi;
+    const double v = alpha * acc + (beta == 0.0 ? 0.0 : beta * C0[at]);
+    C[at] = v;
+    if (sym && blockIdx.x != blockIdx.y) C[(int64_t)gi * ldc + gj] = v;
   }
 }
 
@@ -1545,18 +1551,13 @@ cudaError_t panel_times_small(const float* M, int ldm, int p, int64_t n, const d
 }
 
 cudaError_t dgemm_small(bool ta, bool tb, int m, int n, int k, double alpha, const double* A,
-                        int lda, const double* B, int ldb, double beta, double* C, int ldc,
-                        cudaStream_t s) {
+                        int lda, const double* B, int ldb, double beta, const double* C0, double* C,
+                        int ldc, cudaStream_t s) {
   if (m == 0 || n == 0) return cudaSuccess;
-  // FP64 runs at 1/64 of the FP32 rate: spread the tiles over the SMs, with
-  // 16 x 16 tiles where 32 x 32 tiles would leave most SMs idle
-  if (ceil_div(m, 32) * ceil_div(n, 32) < (int64_t)(2 * kNumSMs) / 3) {
-    dim3 grid((unsigned)ceil_div(m, 16), (unsigned)ceil_div(n, 16));
-    dgemm_small_kernel<16><<<grid, 256, 0, s>>>(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-  } else {
-    dim3 grid((unsigned)ceil_div(m, 32), (unsigned)ceil_div(n, 32));
-    dgemm_small_kernel<32><<<grid, 256, 0, s>>>(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-  }
+  const bool sym = A == B && lda == ldb && ta != tb && m == n && beta == 0.0;
+  dim3 grid((unsigned)ceil_div(m, DG_T), (unsigned)ceil_div(n, DG_T));
+  dgemm_small_kernel<<<grid, DG_T * DG_T, 0, s>>>(ta, tb, sym, m, n, k, alpha, A, lda, B, ldb, beta,
+                                                  C0, C, ldc);
   ++g_launch_count;
   return cudaGetLastError();
 }

@@ -168,14 +168,13 @@ void sym_eig_refined(mmsb_ctx* c, const std::string& tag, int n, const double* A
       ck(cudaEventRecord(c->fork_ev, s), "fork");
       ck(cudaStreamWaitEvent(aux, c->fork_ev, 0), "fork wait");
     }
-    ck(dgemm_small(true, false, n, n, n, 1.0, X, n, X, n, 0.0, G, n, aux ? aux : s), "X^T X");
+    ck(dgemm_small(true, false, n, n, n, 1.0, X, n, X, n, 0.0, nullptr, G, n, aux ? aux : s), "X^T X");
     if (aux) ck(cudaEventRecord(c->join_ev, aux), "join");
-    ck(dgemm_small(false, false, n, n, n, 1.0, A, n, X, n, 0.0, AX, n, s), "A X");
-    ck(dgemm_small(true, false, n, n, n, 1.0, X, n, AX, n, 0.0, S, n, s), "X^T A X");
+    ck(dgemm_small(false, false, n, n, n, 1.0, A, n, X, n, 0.0, nullptr, AX, n, s), "A X");
+    ck(dgemm_small(true, false, n, n, n, 1.0, X, n, AX, n, 0.0, nullptr, S, n, s), "X^T A X");
     if (aux) ck(cudaStreamWaitEvent(s, c->join_ev, 0), "join wait");
     ck(oa_correction(n, A, G, S, E, lam, dstate, s), "oa");
-    ck(cudaMemcpyAsync(X2, X, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, s), "copy");
-    ck(dgemm_small(false, false, n, n, n, 1.0, X, n, E, n, 1.0, X2, n, s), "X + X E");
+    ck(dgemm_small(false, false, n, n, n, 1.0, X, n, E, n, 1.0, X, X2, n, s), "X + X E");
     std::swap(X, X2);
   }
   ck(sort_eigen(n, lam, X, evals, V, c->flags, s), "sort");
@@ -237,13 +236,13 @@ Nys svd_sym_nystrom(mmsb_ctx* c, const std::string& tag, const float* A, int lda
   ck(trinv_upper(m, R2, T2, st2), "R2^-1");
   if (nystrom) {
     ck(panel_to_colmajor64(Q1, ldq, p, m, Ap, p, st2), "Q1[0:p]");
-    ck(dgemm_small(false, false, p, m, m, 1.0, Ap, p, T2, m, 0.0, QAp, p, st2), "Q_A[0:p]");
+    ck(dgemm_small(false, false, p, m, m, 1.0, Ap, p, T2, m, 0.0, nullptr, QAp, p, st2), "Q_A[0:p]");
   }
   if (aux) ck(cudaEventRecord(c->join_ev, aux), "join");
-  ck(dgemm_small(false, false, m, m, m, 1.0, R2, m, R1, m, 0.0, RA, m, s), "R_A");
+  ck(dgemm_small(false, false, m, m, m, 1.0, R2, m, R1, m, 0.0, nullptr, RA, m, s), "R_A");
   // P = R_A B
   if (B)
-    ck(dgemm_small(false, false, m, p, m, 1.0, RA, m, B, m, 0.0, P, m, s), "P");
+    ck(dgemm_small(false, false, m, p, m, 1.0, RA, m, B, m, 0.0, nullptr, P, m, s), "P");
   else
     ck(cudaMemcpyAsync(P, RA, sizeof(double) * m * p, cudaMemcpyDeviceToDevice, s), "P");
   if (nystrom) {
@@ -254,13 +253,13 @@ Nys svd_sym_nystrom(mmsb_ctx* c, const std::string& tag, const float* A, int lda
     else  // MGS of the upper-triangular R_A is the identity (zero where R_jj == 0)
       ck(eye_mask(m, p, P, m, Qs, m, s), "mgs(R)");
     if (aux) ck(cudaStreamWaitEvent(s, c->join_ev, 0), "join wait");
-    ck(dgemm_small(false, false, p, p, m, 1.0, QAp, p, Qs, m, 0.0, QQ, p, s), "QQ");
-    ck(dgemm_small(false, false, m, p, p, 1.0, P, m, QQ, p, 0.0, Hm, m, s), "H");
+    ck(dgemm_small(false, false, p, p, m, 1.0, QAp, p, Qs, m, 0.0, nullptr, QQ, p, s), "QQ");
+    ck(dgemm_small(false, false, m, p, p, 1.0, P, m, QQ, p, 0.0, nullptr, Hm, m, s), "H");
   } else {
     ck(cudaMemcpyAsync(Hm, P, sizeof(double) * m * p, cudaMemcpyDeviceToDevice, s), "H");
     if (aux) ck(cudaStreamWaitEvent(s, c->join_ev, 0), "join wait");
   }
-  ck(dgemm_small(false, true, m, m, p, 1.0, Hm, m, Hm, m, 0.0, Zs, m, s), "H H^T");
+  ck(dgemm_small(false, true, m, m, p, 1.0, Hm, m, Hm, m, 0.0, nullptr, Zs, m, s), "H H^T");
   // Zs = H H^T.  The one-sided Jacobi runs on the Cholesky factor L of Zs
   // (L L^T = H H^T), not on H: L's columns are graded like the R factor of a
   // QR preconditioner, and the FP32 sweeps drop from ~13 to ~8 at p = 200,
@@ -268,7 +267,7 @@ Nys svd_sym_nystrom(mmsb_ctx* c, const std::string& tag, const float* A, int lda
   sym_eig_refined(c, tag, m, Zs, ev, Wv, nullptr, s, aux);
   // sigma = sqrt(ev_k); U = Q_A W_k diag(sigma > tol) = Q1 (R2^{-1} W_k) (masked)
   ck(sig_from_evals(k, ev, sig, s), "sig");
-  ck(dgemm_small(false, false, m, k, m, 1.0, T2, m, Wv, m, 0.0, F, m, s), "F");
+  ck(dgemm_small(false, false, m, k, m, 1.0, T2, m, Wv, m, 0.0, nullptr, F, m, s), "F");
   ck(mask_cols(m, k, F, m, sig, tol, s), "mask");
   ck(panel_times_small(Q1, ldq, m, n, F, m, k, U, ldk, s), "U");
   return Nys{U, sig};
@@ -560,7 +559,7 @@ void pipeline_whiten(mmsb_ctx* c, const double* const* sketches, bool finish) {
   // M2 sketch = (a0+1) Zc1 core (Zb1^T R_a) - a0 mu_a (mu_a^T R_a)  (Util.cpp:103-113),
   // kept factored as M2 = [Zc1 | mu_a] B with B = [(a0+1) core Zb1^T R_a ; -a0 mu_a^T R_a]
   // (rank <= k+1, so its Gram-Schmidt must see FP64 round-off, not FP32)
-  ck(dgemm_small(false, false, k, p, k, c->cfg.alpha0 + 1.0, core, k, Q1, k, 0.0, Bm, m2, s), "B");
+  ck(dgemm_small(false, false, k, p, k, c->cfg.alpha0 + 1.0, core, k, Q1, k, 0.0, nullptr, Bm, m2, s), "B");
   ck(set_row_scaled(m2, p, Bm, m2, k, -c->cfg.alpha0, ma, s), "B shift row");
   ck(panel_copy(c->Zc1, ldk, c->nA, k, Am, ldm2, s), "A_M");
   ck(panel_set_col(Am, ldm2, c->nA, k, c->mu, s), "A_M mu");
@@ -871,10 +870,10 @@ static double* final_qr_f64(mmsb_ctx* c) {
   double* T = c->tbuf<double>("fq.T", (size_t)k * k);
   ck(f32_to_f64(c->phi, Pa, (int64_t)k * k, s), "phi64");
   for (int pass = 0; pass < 2; ++pass) {
-    ck(dgemm_small(true, false, k, k, k, 1.0, Pa, k, Pa, k, 0.0, S, k, s), "Phi^T Phi");
+    ck(dgemm_small(true, false, k, k, k, 1.0, Pa, k, Pa, k, 0.0, nullptr, S, k, s), "Phi^T Phi");
     ck(chol_upper_drop(k, S, k, R, 1e-300, c->flags, s), "chol");
     ck(trinv_upper(k, R, T, s), "R^-1");
-    ck(dgemm_small(false, false, k, k, k, 1.0, Pa, k, T, k, 0.0, Pb, k, s), "Phi R^-1");
+    ck(dgemm_small(false, false, k, k, k, 1.0, Pa, k, T, k, 0.0, nullptr, Pb, k, s), "Phi R^-1");
     std::swap(Pa, Pb);
   }
   ck(f64_to_f32(Pa, c->phi, (int64_t)k * k, s), "phi32");
@@ -1079,7 +1078,7 @@ double pipeline_loss(mmsb_ctx* c, const double* phi, int64_t begin, int64_t coun
   float* G = c->tbuf<float>("G", (size_t)k * k);
   double* S = c->tbuf<double>("loss_S", (size_t)k * k);
   stpm_pass(c, kModeLoss, 0, 1, 2, begin, count, p0, p1, p2, 1.0, G, c->dscalar + 1);
-  ck(dgemm_small(true, false, k, k, k, 1.0, sw.phi64, k, sw.phi64, k, 0.0, S, k, c->s), "S");
+  ck(dgemm_small(true, false, k, k, k, 1.0, sw.phi64, k, sw.phi64, k, 0.0, nullptr, S, k, c->s), "S");
   ck(cube_sum(k * k, S, c->cfg.theta, c->dscalar + 2, c->s), "cube");
   double h[2] = {0, 0};
   ck(cudaMemcpyAsync(h, c->dscalar + 1, sizeof(double) * 2, cudaMemcpyDeviceToHost, c->s), "D2H");
@@ -1103,9 +1102,9 @@ void pipeline_loss_grad(mmsb_ctx* c, const double* phi, int64_t begin, int64_t c
   stpm_pass(c, kModeAdjoint, 0, 1, 2, begin, count, p0, p1, p2, 1.0 / (double)count, G, nullptr);
   ck(f32_to_f64(G, dT, (int64_t)k * k, c->s), "dT");
   // 6 theta Phi (S o S) - 2 dT
-  ck(dgemm_small(true, false, k, k, k, 1.0, sw.phi64, k, sw.phi64, k, 0.0, S, k, c->s), "S");
+  ck(dgemm_small(true, false, k, k, k, 1.0, sw.phi64, k, sw.phi64, k, 0.0, nullptr, S, k, c->s), "S");
   ck(hadamard_square((int64_t)k * k, S, S2, c->s), "S2");
-  ck(dgemm_small(false, false, k, k, k, 6.0 * c->cfg.theta, sw.phi64, k, S2, k, 0.0, out, k, c->s), "O");
+  ck(dgemm_small(false, false, k, k, k, 6.0 * c->cfg.theta, sw.phi64, k, S2, k, 0.0, nullptr, out, k, c->s), "O");
   ck(axpy_f64((int64_t)k * k, -2.0, dT, out, c->s), "grad");
   ck(cudaMemcpyAsync(dphi, out, sizeof(double) * k * k, cudaMemcpyDeviceToHost, c->s), "D2H");
   ck(cudaStreamSynchronize(c->s), "sync");
