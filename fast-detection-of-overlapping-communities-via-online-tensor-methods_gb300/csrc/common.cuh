@@ -108,6 +108,11 @@ cudaError_t mgs_cols(int m, int p, const double* P, int ldp, double* Q, int ldq,
 // doubles (the cluster threshold, then scratch for its three maxima).
 cudaError_t oa_correction(int n, const double* A, const double* XtX, const double* S, double* E,
                           double* lam, double* delta_state, cudaStream_t s);
+// All steps of that refinement and the sort in one kernel, where it fits (small
+// n); delta_state as above (the threshold only).
+bool oa_refine_fits(int n);
+cudaError_t oa_refine(int n, int steps, const double* A, const double* X, double* evals,
+                      double* evecs, double* delta_state, unsigned* flags, cudaStream_t s);
 cudaError_t sort_eigen(int n, const double* lam, const double* X, double* evals, double* evecs,
                        unsigned* flags, cudaStream_t s);
 cudaError_t panel_set_col(float* P, int ld, int64_t rows, int col, const double* v,

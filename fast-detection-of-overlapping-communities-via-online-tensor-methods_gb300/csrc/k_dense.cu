@@ -1372,6 +1372,173 @@ __global__ void __launch_bounds__(256) sort_eigen_kernel(int n, const double* __
   for (int r = lane; r < n; r += 32) evecs[(int64_t)rank * n + r] = X[(int64_t)i * n + r];
 }
 
+// All refinement steps and the sort in one kernel, for small n: as kernels of
+// their own (four products, the two above and a memset per step, each over n / 8
+// tiles) they are 3 to 6 us of latency each, about 90 us at n = 10 and 130 us at n = 50,
+// 20 and 45 us here.  The columns are split over a cluster (one CTA up to n =
+// 16, else 16: the FP64 units of more SMs); each CTA holds A and all of X and
+// sends its new columns, eigenvalues and column sums to the others.  An entry per
+// thread; every sum is the same chain as in the kernels above.
+constexpr int kOaMax = 64;
+
+template <int CL>
+__global__ void __launch_bounds__(256) oa_refine_kernel(int n, int steps, const double* __restrict__ A,
+                                                        const double* __restrict__ X0,
+                                                        double* __restrict__ evals,
+                                                        double* __restrict__ evecs,
+                                                        double* __restrict__ delta_state,
+                                                        unsigned* flags) {
+  namespace cg = cooperative_groups;
+  extern __shared__ double sm[];
+  const int ld = n | 1, nc = (n + CL - 1) / CL;  // odd stride: rows and columns free of conflicts
+  const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
+  const int j0 = rank * nc, own = max(0, min(nc, n - j0));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double *As = sm, *Xs = As + n * ld, *Xn = Xs + n * ld, *AX = Xn + n * ld, *G = AX + nc * ld,
+         *S = G + nc * ld, *lam = S + nc * ld, *mx = lam + n;  // mx: 3 column sums of n each
+  auto sync_all = [&]() {
+    if (CL > 1) cg::this_cluster().sync();
+    else __syncthreads();
+  };
+  auto put = [&](double* p, int q, double v) {  // p in CTA q's shared memory
+    if (CL > 1) *cg::this_cluster().map_shared_rank(p, q) = v;
+    else *p = v;
+  };
+  for (int e = tid; e < n * n; e += 256) {
+    const int i = e % n, j = e / n;
+    As[j * ld + i] = A[e];
+    Xs[j * ld + i] = X0[e];
+  }
+  sync_all();  // (and every CTA of the cluster has started)
+  const int i = tid % n, jc = tid / n, j = j0 + jc;
+  const bool live = jc < own;
+  const int o = jc * ld + i;
+  for (int step = 0; step < steps; ++step) {
+    if (live) {
+      double ax = 0.0, g = 0.0;
+#pragma unroll 2
+      for (int kk = 0; kk < n; ++kk) {
+        const double x = Xs[j * ld + kk];
+        ax = fma(As[kk * ld + i], x, ax);
+        g = fma(Xs[i * ld + kk], x, g);
+      }
+      AX[o] = ax;
+      G[o] = g;
+    }
+    __syncthreads();
+    if (live) {
+      double v = 0.0;
+#pragma unroll 2
+      for (int kk = 0; kk < n; ++kk) v = fma(Xs[i * ld + kk], AX[jc * ld + kk], v);
+      S[o] = v;
+    }
+    __syncthreads();
+    for (int c = warp; c < own; c += 8) {
+      const int jj = j0 + c;
+      const double xx = G[c * ld + jj];  // = 1 - R_jj
+      const double lj = xx > 0.0 ? S[c * ld + jj] / xx : 0.0;
+      double cs = 0.0, cr = 0.0;
+      for (int r = lane; r < n; r += 32) {
+        cs += fabs(S[c * ld + r] - (r == jj ? lj : 0.0));
+        cr += fabs((r == jj ? 1.0 : 0.0) - G[c * ld + r]);
+      }
+#pragma unroll
+      for (int off = 16; off; off >>= 1) {
+        cs += __shfl_xor_sync(0xffffffffu, cs, off);
+        cr += __shfl_xor_sync(0xffffffffu, cr, off);
+      }
+      if (lane < CL) {
+        put(lam + jj, lane, lj);
+        put(mx + jj, lane, cs);
+        put(mx + n + jj, lane, fabs(lj));
+        put(mx + 2 * n + jj, lane, cr);
+      }
+    }
+    sync_all();
+    unsigned long long m[3];  // (bit patterns order like the values, NaN above all)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      m[q] = 0ull;
+      for (int r = lane; r < n; r += 32)
+        m[q] = max(m[q], (unsigned long long)__double_as_longlong(mx[q * n + r]));
+#pragma unroll
+      for (int off = 16; off; off >>= 1) m[q] = max(m[q], __shfl_xor_sync(0xffffffffu, m[q], off));
+    }
+    const double dl = 2.0 * (__longlong_as_double((long long)m[0]) +
+                             __longlong_as_double((long long)m[1]) * __longlong_as_double((long long)m[2]));
+    if (rank == 0 && tid == 0) delta_state[0] = dl;  // reported for diagnostics
+    if (live) {
+      const double r = (i == j ? 1.0 : 0.0) - G[o];
+      double v = 0.5 * r;
+      if (i != j) {
+        const double gap = lam[j] - lam[i];
+        if (fabs(gap) > dl) v = (S[o] + lam[j] * r) / gap;
+      }
+      AX[o] = v;  // E
+    }
+    __syncthreads();
+    if (live) {
+      double v = 0.0;
+#pragma unroll 2
+      for (int kk = 0; kk < n; ++kk) v = fma(Xs[kk * ld + i], AX[jc * ld + kk], v);
+      v += Xs[j * ld + i];
+      for (int q = 0; q < CL; ++q) put(Xn + j * ld + i, q, v);
+    }
+    sync_all();
+    double* t = Xs;
+    Xs = Xn;
+    Xn = t;
+  }
+  for (int c = warp; c < own; c += 8) {  // as sort_eigen_kernel
+    const int jj = j0 + c;
+    const double lj = lam[jj];
+    const long long kj = order_key(lj);
+    int at = 0;
+    for (int r = lane; r < n; r += 32) {
+      const long long kr = order_key(lam[r]);
+      at += (kr > kj) || (kr == kj && r < jj);
+    }
+    at = __reduce_add_sync(0xffffffffu, at);
+    if (lane == 0) {
+      evals[at] = lj;
+      if (!isfinite(lj) && flags) atomicOr(flags, kFlagNonFinite);
+    }
+    for (int r = lane; r < n; r += 32) evecs[(int64_t)at * n + r] = Xs[jj * ld + r];
+  }
+}
+
+size_t oa_refine_smem(int n, int CL) {
+  const int ld = n | 1, nc = (n + CL - 1) / CL;
+  return sizeof(double) * ((size_t)3 * n * ld + 3 * nc * ld + 4 * n);
+}
+
+template <int CL>
+cudaError_t oa_refine_config(int n, cudaStream_t s, cudaLaunchConfig_t* lc,
+                             cudaLaunchAttribute* at) {
+  static bool set = false;
+  if (!set) {
+    MMSB_CUDA_TRY(cudaFuncSetAttribute(oa_refine_kernel<CL>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)oa_refine_smem(CL > 1 ? kOaMax : 16, CL)));
+    if (CL > 8)
+      MMSB_CUDA_TRY(cudaFuncSetAttribute(oa_refine_kernel<CL>,
+                                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    set = true;
+  }
+  *lc = cudaLaunchConfig_t{};
+  lc->gridDim = dim3(CL);
+  lc->blockDim = dim3(256);
+  lc->dynamicSmemBytes = oa_refine_smem(n, CL);
+  lc->stream = s;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CL;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  lc->attrs = at;
+  lc->numAttrs = CL > 1 ? 1 : 0;
+  return cudaSuccess;
+}
+
 // P (rows x q, row-major panel ld) gets column `col` = v (FP64 vector, length rows)
 __global__ void panel_set_col_kernel(float* __restrict__ P, int ld, int64_t rows, int col,
                                      const double* __restrict__ v) {
@@ -1791,6 +1958,39 @@ cudaError_t oa_correction(int n, const double* A, const double* XtX, const doubl
   oa_correction_kernel<<<dim3((unsigned)ceil_div(n, 256), (unsigned)n), 256, 0, s>>>(n, XtX, S, E,
                                                                                     lam, mx, delta_state);
   g_launch_count += 2;
+  return cudaGetLastError();
+}
+
+bool oa_refine_fits(int n) {
+  if (n <= 16) return true;
+  if (n > kOaMax) return false;
+  static const bool wide = []() {  // 16 CTAs are a non-portable cluster size
+    cudaLaunchConfig_t lc;
+    cudaLaunchAttribute at[1];
+    int clusters = 0;
+    const bool ok = oa_refine_config<16>(kOaMax, nullptr, &lc, at) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, oa_refine_kernel<16>, &lc) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok && clusters > 0;
+  }();
+  return wide;
+}
+
+cudaError_t oa_refine(int n, int steps, const double* A, const double* X, double* evals,
+                      double* evecs, double* delta_state, unsigned* flags, cudaStream_t s) {
+  if (n < 1 || n > kOaMax) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t lc;
+  cudaLaunchAttribute at[1];
+  if (n <= 16) {
+    MMSB_CUDA_TRY(oa_refine_config<1>(n, s, &lc, at));
+    MMSB_CUDA_TRY(cudaLaunchKernelEx(&lc, oa_refine_kernel<1>, n, steps, A, X, evals, evecs,
+                                     delta_state, flags));
+  } else {
+    MMSB_CUDA_TRY(oa_refine_config<16>(n, s, &lc, at));
+    MMSB_CUDA_TRY(cudaLaunchKernelEx(&lc, oa_refine_kernel<16>, n, steps, A, X, evals, evecs,
+                                     delta_state, flags));
+  }
+  ++g_launch_count;
   return cudaGetLastError();
 }
 

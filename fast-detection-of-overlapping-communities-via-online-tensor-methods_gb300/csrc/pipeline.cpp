@@ -162,6 +162,10 @@ void sym_eig_refined(mmsb_ctx* c, const std::string& tag, int n, const double* A
   }
   ck(eig_from_factor(n, Y, lam, X, work, c->flags, s), "jacobi");
   double* dstate = c->tbuf<double>(tag + ".edelta", 4);  // delta + three maxima
+  if (oa_refine_fits(n)) {
+    ck(oa_refine(n, 3, A, X, evals, V, dstate, c->flags, s), "eig refine");
+    return;
+  }
   ck(cudaMemsetAsync(dstate, 0, 4 * sizeof(double), s), "delta");
   for (int step = 0; step < 3; ++step) {
     if (aux) {
