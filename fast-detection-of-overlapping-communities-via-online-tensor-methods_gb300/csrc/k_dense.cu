@@ -565,11 +565,11 @@ __global__ void __launch_bounds__(64) trinv_upper_kernel(int p, const double* __
 
 // ---- one-sided Jacobi: eigenpairs of Y Y^T -------------------------------------
 
-// Eigenpairs from the converged columns of X (column-major, ld p): eigenvalue
+// Eigenpairs from the converged columns of X (column-major, ld): eigenvalue
 // = squared column norm, eigenvector = normalised column, sorted descending;
 // exactly zero columns are completed to an orthonormal basis.  Called by one
 // CTA (any block size that is a multiple of 32).
-__device__ void jacobi_finish(int p, const float* X, double* __restrict__ evals,
+__device__ void jacobi_finish(int p, const float* X, int ld, double* __restrict__ evals,
                               double* __restrict__ evecs, unsigned* flags) {
   __shared__ int order[512];
   __shared__ float nrm2[512];
@@ -578,7 +578,7 @@ __device__ void jacobi_finish(int p, const float* X, double* __restrict__ evals,
   // eigenvalue i = squared norm of column i
   for (int i = warp; i < p; i += nw) {
     float s = 0.f;
-    for (int t = lane; t < p; t += 32) s = fmaf(X[(int64_t)i * p + t], X[(int64_t)i * p + t], s);
+    for (int t = lane; t < p; t += 32) s = fmaf(X[(int64_t)i * ld + t], X[(int64_t)i * ld + t], s);
 #pragma unroll
     for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     if (lane == 0) nrm2[i] = s;
@@ -602,7 +602,8 @@ __device__ void jacobi_finish(int p, const float* X, double* __restrict__ evals,
     const float s = nrm2[i];
     const float inv = s > 0.f ? rsqrtf(s) : 0.f;
     if (lane == 0) evals[r] = (double)s;
-    for (int t = lane; t < p; t += 32) evecs[(int64_t)r * p + t] = (double)(X[(int64_t)i * p + t] * inv);
+    for (int t = lane; t < p; t += 32)
+      evecs[(int64_t)r * p + t] = (double)(X[(int64_t)i * ld + t] * inv);
   }
   // Exactly zero columns (null directions of a rank-deficient factor, ranked
   // last) carry no direction: complete the basis so that the refinement
@@ -659,14 +660,102 @@ __device__ void jacobi_finish(int p, const float* X, double* __restrict__ evals,
     __syncthreads();
   }}
 
-template <bool kSmem>
+// p < 96: the columns in shared memory, 8 lanes per pair of a round, 8 v + lane
+// (v < NV) being a lane's rows, held in registers between the sums and the
+// rotation; only as many threads as there are pairs to rotate, since a round
+// ends with a barrier.  What bounds it is the latency of a round: loads, three
+// sums, the rotation's divisions and square roots, stores, barrier.  (1,024
+// threads and loops over p read twice: 250 us at p = 50, 145 us here.)  Pairs, tests
+// and formulas as in jacobi_kernel below.
+__host__ __device__ constexpr int jacobi_small_ld(int NV) {  // == 8 mod 32: 4 neighbouring columns
+  return 8 * NV <= 8 ? 8 : 8 * NV <= 40 ? 40 : 8 * NV <= 72 ? 72 : 104;
+}
+
+template <int NV>
+__global__ void __launch_bounds__(384) jacobi_small_kernel(int p, const double* __restrict__ Y,
+                                                           double* __restrict__ evals,
+                                                           double* __restrict__ evecs,
+                                                           unsigned* flags, int max_sweeps,
+                                                           float tol) {
+  extern __shared__ float smem[];
+  constexpr int ld = jacobi_small_ld(NV);
+  float* X = smem;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  for (int e = tid; e < p * ld; e += nt) {
+    const int j = e / ld, i = e % ld;
+    X[e] = i < p ? (float)Y[j * p + i] : 0.f;
+  }
+  const int m = p + (p & 1), w = m - 1;
+  const int s = tid >> 3, l8 = tid & 7;
+  __syncthreads();
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    int a = s == 0 ? 0 : 1 + (s - 1) % w, b = 1 + (m - 2 - s + 2 * w) % w;
+    int rotated = 0;
+    for (int r = 0; r < m - 1; ++r) {
+      const int i = min(a, b), j = max(a, b);
+      if (s != 0) a = a == w ? 1 : a + 1;
+      b = b == w ? 1 : b + 1;
+      const bool live = s < m / 2 && j < p;
+      float* xi = X + (live ? i : 0) * ld + l8;
+      float* xj = X + (live ? j : 0) * ld + l8;
+      float x[NV], y[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) x[v] = xi[8 * v], y[v] = xj[8 * v];
+      float al = 0.f, be = 0.f, ga = 0.f;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        al = fmaf(x[v], x[v], al);
+        be = fmaf(y[v], y[v], be);
+        ga = fmaf(x[v], y[v], ga);
+      }
+#pragma unroll
+      for (int off = 4; off; off >>= 1) {
+        al += __shfl_xor_sync(0xffffffffu, al, off);
+        be += __shfl_xor_sync(0xffffffffu, be, off);
+        ga += __shfl_xor_sync(0xffffffffu, ga, off);
+      }
+      if (live && fabsf(ga) > tol * sqrtf(al * be) && ga != 0.f) {
+        const float zeta = (be - al) / (2.f * ga);
+        const float t = copysignf(1.f, zeta) / (fabsf(zeta) + sqrtf(1.f + zeta * zeta));
+        const float c = rsqrtf(1.f + t * t), sn = c * t;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          xi[8 * v] = c * x[v] - sn * y[v];
+          xj[8 * v] = sn * x[v] + c * y[v];
+        }
+        rotated = 1;
+      }
+      __syncthreads();
+    }
+    if (!__syncthreads_or(rotated)) break;
+  }
+  jacobi_finish(p, X, ld, evals, evecs, flags);
+}
+
+template <int NV>
+cudaError_t launch_jacobi_small(int p, const double* Y, double* evals, double* evecs,
+                                unsigned* flags, int max_sweeps, float tol, cudaStream_t s) {
+  const int threads = (int)std::max<int64_t>(64, round_up(8 * ((p + 1) / 2), 32));
+  static bool set = false;
+  if (!set) {  // (static and dynamic together pass 48 KB from p = 87)
+    MMSB_CUDA_TRY(cudaFuncSetAttribute(jacobi_small_kernel<NV>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(float) * 8 * NV * jacobi_small_ld(NV)));
+    set = true;
+  }
+  jacobi_small_kernel<NV><<<1, threads, sizeof(float) * p * jacobi_small_ld(NV), s>>>(
+      p, Y, evals, evecs, flags, max_sweeps, tol);
+  ++g_launch_count;
+  return cudaGetLastError();
+}
+
+// (the columns in global memory: where the cluster form below does not fit)
 __global__ void __launch_bounds__(1024) jacobi_kernel(int p, const double* __restrict__ Y,
                                                       double* __restrict__ evals,
                                                       double* __restrict__ evecs,
                                                       float* __restrict__ gwork,
                                                       unsigned* flags, int max_sweeps, float tol) {
-  extern __shared__ float smem[];
-  float* X = kSmem ? smem : gwork;  // column-major p x p
+  float* X = gwork;  // column-major p x p
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int64_t e = tid; e < (int64_t)p * p; e += nt) X[e] = (float)Y[e];
   const int m = p + (p & 1);  // players in the round-robin tournament
@@ -734,7 +823,7 @@ __global__ void __launch_bounds__(1024) jacobi_kernel(int p, const double* __res
     }
     if (!__syncthreads_or(rotated)) break;
   }
-  jacobi_finish(p, X, evals, evecs, flags);
+  jacobi_finish(p, X, p, evals, evecs, flags);
 }
 
 // ---- one-sided Jacobi on a cluster (block round-robin) --------------------------
@@ -977,7 +1066,7 @@ __global__ void __launch_bounds__(512) jacobi_cluster_kernel(int p, const double
   }
   __threadfence();
   cluster.sync();
-  if (t == 0) jacobi_finish(p, gwork, evals, evecs, flags);
+  if (t == 0) jacobi_finish(p, gwork, p, evals, evecs, flags);
 }
 
 // ---- Gram-Schmidt of the columns of a small m x p FP64 matrix (one CTA) -------------
@@ -1817,13 +1906,18 @@ cudaError_t trinv_upper(int p, const double* R, double* T, cudaStream_t s) {
 cudaError_t eig_from_factor(int p, const double* Y, double* evals, double* evecs, float* work,
                             unsigned* flags, cudaStream_t s) {
   if (p > 512) return cudaErrorInvalidValue;
-  const size_t sm = (size_t)p * p * sizeof(float);
   // the FP64 refinement converges quadratically only from a converged FP32
   // start (6 sweeps left 1e-3 off-diagonal mass at n = 200; 9-10 suffice)
   const int max_sweeps = 15;
   const float tol = 8.f * sqrtf((float)p) * 6e-8f;
-  // p >= 96: the 8-CTA cluster version while four blocks fit shared memory
-  if (p >= 96) {
+  if (p < 96)
+    return p <= 16   ? launch_jacobi_small<2>(p, Y, evals, evecs, flags, max_sweeps, tol, s)
+           : p <= 32 ? launch_jacobi_small<4>(p, Y, evals, evecs, flags, max_sweeps, tol, s)
+           : p <= 56 ? launch_jacobi_small<7>(p, Y, evals, evecs, flags, max_sweeps, tol, s)
+           : p <= 72 ? launch_jacobi_small<9>(p, Y, evals, evecs, flags, max_sweeps, tol, s)
+                     : launch_jacobi_small<12>(p, Y, evals, evecs, flags, max_sweeps, tol, s);
+  // the 8-CTA cluster version while four blocks fit shared memory
+  {
     const size_t smc = sizeof(float) * 4 * (size_t)jc_b(p) * jc_ld(p);
     if (smc <= 200 * 1024) {
       // 32 lanes per pair up to p = 256, else 16; NV: words of a column per lane
@@ -1853,17 +1947,7 @@ cudaError_t eig_from_factor(int p, const double* Y, double* evals, double* evecs
       return cudaLaunchKernelEx(&lc, kernel, p, Y, evals, evecs, work, flags, max_sweeps, tol);
     }
   }
-  if (sm <= 200 * 1024) {
-    static bool attr_set = false;
-    if (!attr_set) {
-      MMSB_CUDA_TRY(cudaFuncSetAttribute(jacobi_kernel<true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr_set = true;
-    }
-    jacobi_kernel<true><<<1, 1024, sm, s>>>(p, Y, evals, evecs, work, flags, max_sweeps, tol);
-  } else {
-    jacobi_kernel<false><<<1, 1024, 0, s>>>(p, Y, evals, evecs, work, flags, max_sweeps, tol);
-  }
+  jacobi_kernel<<<1, 1024, 0, s>>>(p, Y, evals, evecs, work, flags, max_sweeps, tol);
   ++g_launch_count;
   return cudaGetLastError();
 }
