@@ -75,7 +75,8 @@ inline bool gram_use_tc(int64_t n, int pa, int pb) { return pa >= 64 && pb >= 64
 int gram_tc_nsplit(int64_t n, int pa, int pb);
 cudaError_t gram_tc_partial(const float* A, int lda, int pa, const float* B, int ldb, int pb,
                             int64_t n, double* partials, int nsplit, unsigned* flags,
-                            cudaStream_t s, long long wait_limit = 0);
+                            cudaStream_t s, long long wait_limit,
+                            bool sym);
 size_t gram_tsk_partials(int64_t n, int pa, int pb);
 // Y[n x ldy] (row-major FP32) = M[n x ldm] (first p cols) * F (p x q, column-major FP64, ldf);
 // columns q..ldy-1 of Y are zeroed.

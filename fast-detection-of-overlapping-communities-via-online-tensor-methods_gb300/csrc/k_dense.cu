@@ -107,11 +107,17 @@ __global__ void __launch_bounds__(256) gram_partial_kernel(
     }
 }
 
-// (the splits in order, 8 loads in flight: the FP64 sums stay one chain)
+// (the splits in order, 8 loads in flight: the FP64 sums stay one chain; mirror >
+// 0: only tiles of that edge on and above the diagonal hold partials, p x p)
 __global__ void gram_reduce_kernel(const double* __restrict__ partials, int nsplit, int64_t m,
-                                   double alpha, double* __restrict__ S) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m;
-       e += (int64_t)gridDim.x * blockDim.x) {
+                                   double alpha, double* __restrict__ S, int mirror, int p) {
+  for (int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; at < m;
+       at += (int64_t)gridDim.x * blockDim.x) {
+    int64_t e = at;
+    if (mirror > 0) {
+      const int i = (int)(at % p), j = (int)(at / p);
+      if (i / mirror > j / mirror) e = (int64_t)i * p + j;
+    }
     double s = 0.0;
     int t = 0;
     for (; t + 8 <= nsplit; t += 8) {
@@ -122,7 +128,7 @@ __global__ void gram_reduce_kernel(const double* __restrict__ partials, int nspl
       for (int u = 0; u < 8; ++u) s += v[u];
     }
     for (; t < nsplit; ++t) s += __ldg(partials + (int64_t)t * m + e);
-    S[e] = alpha * s;
+    S[at] = alpha * s;
   }
 }
 
@@ -1777,11 +1783,12 @@ cudaError_t gram_tsk(const float* A, int lda, int pa, const float* B, int ldb, i
   if (gram_use_tc(n, pa, pb)) {
     // tcgen05 (kind::tf32, 3xTF32) partials over row splits, then the FP64 sum
     const int nsplit = gram_tc_nsplit(n, pa, pb);
+    const bool sym = A == B && lda == ldb && pa == pb;  // tiles of 128 x 128
     if ((int64_t)nsplit * pa * pb > partials_cap) return cudaErrorInvalidValue;
     MMSB_CUDA_TRY(gram_tc_partial(A, lda, pa, B, ldb, pb, n, partials, nsplit, flags, s,
-                                  wait_limit));
-    gram_reduce_kernel<<<grid_for((int64_t)pa * pb), 256, 0, s>>>(partials, nsplit,
-                                                                   (int64_t)pa * pb, alpha, S);
+                                  wait_limit, sym));
+    gram_reduce_kernel<<<grid_for((int64_t)pa * pb), 256, 0, s>>>(
+        partials, nsplit, (int64_t)pa * pb, alpha, S, sym ? 128 : 0, pa);
     ++g_launch_count;
     return cudaGetLastError();
   }
@@ -1791,8 +1798,8 @@ cudaError_t gram_tsk(const float* A, int lda, int pa, const float* B, int ldb, i
   dim3 grid((unsigned)ceil_div(pa, GT), (unsigned)ceil_div(pb, GT), (unsigned)nsplit);
   gram_partial_kernel<<<grid, 256, 0, s>>>(A, lda, pa, B, ldb, pb, n, rows_per_split, partials);
   ++g_launch_count;
-  gram_reduce_kernel<<<grid_for((int64_t)pa * pb), 256, 0, s>>>(partials, nsplit,
-                                                                 (int64_t)pa * pb, alpha, S);
+  gram_reduce_kernel<<<grid_for((int64_t)pa * pb), 256, 0, s>>>(
+      partials, nsplit, (int64_t)pa * pb, alpha, S, 0, pa);
   ++g_launch_count;
   return cudaGetLastError();
 }
