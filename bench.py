@@ -378,7 +378,7 @@ def run_ours(args, wl, ws, rank, local):
                 "algorithmic_flops_per_launch": flops / launches, "peak_source": pk["source"]}
 
     step_rf = tensor_entry("stpm_step_kernel (k x k update + Cholesky QR re-orthonormalisation, "
-                           "3xTF32 mma.sync on a KP/8-CTA cluster)", kern["step_ms"],
+                           "FP32 on a CTA cluster)", kern["step_ms"],
                            kern["step_flops"], kern["step_launches"])
     contract_rf = tensor_entry("stpm_contract_kernel (Z = Phi^T y, alpha0 terms, G += y^T C; "
                                "3xTF32 tcgen05 kind::tf32, accumulators in tensor memory)",
