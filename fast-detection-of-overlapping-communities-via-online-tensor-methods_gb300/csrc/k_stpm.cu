@@ -1220,12 +1220,13 @@ __global__ void __launch_bounds__(512, 1) stpm_step_batched(const StpmUpdateArgs
 //   G  += y3^T C                 A = y3   (M = j, K = x), B = C   (N = i, K = x)
 // Z1, Z2 and G live in tensor memory (columns [0, TM), [TM, 2 TM),
 // [2 TM, 2 TM + KP)); G accumulates over the CTA's tiles.  Every accumulation
-// truncates (about 0.3 of an ulp each), so past KP = 32 the products are spread:
+// truncates (about 0.3 of an ulp each), so the products are spread:
 // the small ones (hi lo, lo hi) of Z come first, its large ones go to two or
 // three accumulators, and the small products of G have one of their own.  The
 // first steps of a run, where the iterate is near singular, multiply that error
 // by 10 to 50: after 4 of them Phi was 3.6e-5 off at k = 100 (median of 8 runs)
-// with one chain of each and 1.5e-5 here, 0.9e-5 and 0.6e-5 at k = 33.  Operands are
+// with one chain of each and 1.5e-5 here, 0.9e-5 and 0.6e-5 at k = 33,
+// 0.41e-5 and 0.32e-5 at k = 24.  Operands are
 // staged hi / lo in shared memory, K-major without swizzle; y3 is staged
 // transposed (node index along K).  An M = 128 operand of KP < 128 rows
 // reads its rows past KP from the buffer after it: their products land in
@@ -1250,9 +1251,8 @@ struct ContractTc {
   static constexpr uint32_t REGION = ((REGION0 > STAGE ? REGION0 : STAGE) + 127) / 128 * 128;
   // alignment slack, m1 | m2, d-sums of the 4 node groups
   static constexpr size_t smem = 1024 + REGION + sizeof(float) * (2 * KP + 4 * KP);
-  static constexpr bool SPREAD = KP > 32;
   // further accumulators of Z1 | Z2: two, or one where two CTAs share an SM
-  static constexpr int NZX = !SPREAD ? 0 : KP <= 64 ? 1 : 2;
+  static constexpr int NZX = KP <= 64 ? 1 : 2;
   static constexpr uint32_t ZX = 2 * TM + 2 * KP;
   static constexpr uint32_t TMEM_COLS = KP <= 64 ? 256 : 512;
   static_assert(ZX + NZX * 2 * TM <= TMEM_COLS, "tensor memory columns");
@@ -1668,30 +1668,20 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       const uint64_t dpl = tc::smem_desc(sbase + C::PL, 128, C::SBOJ);
       const uint64_t dyh = tc::smem_desc(sbase + C::Y1H, 128, C::SBOJ);
       const uint64_t dyl = tc::smem_desc(sbase + C::Y1L, 128, C::SBOJ);
-      if constexpr (C::SPREAD) {
-        // the small products, then the first share of the large ones; the other
-        // shares in accumulators of their own (added in the epilogue)
+      // the small products, then the first share of the large ones; the other
+      // shares in accumulators of their own (added in the epilogue)
 #pragma unroll
-        for (int ks = 0; ks < KP / 8; ++ks) {
-          const uint64_t ko = 16u * ks;
-          tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, ks > 0 ? 1u : 0u);
-          tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
-        }
-        constexpr int SHARE = (KP / 8 + C::NZX) / (C::NZX + 1);
+      for (int ks = 0; ks < KP / 8; ++ks) {
+        const uint64_t ko = 16u * ks;
+        tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, ks > 0 ? 1u : 0u);
+        tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
+      }
+      constexpr int SHARE = (KP / 8 + C::NZX) / (C::NZX + 1);
 #pragma unroll
-        for (int ks = 0; ks < KP / 8; ++ks) {
-          const int part = ks / SHARE;
-          tc::mma_tf32(tmem + (part > 0 ? C::ZX + 2 * TM * (part - 1) : 0), dph + 16u * ks,
-                       dyh + 16u * ks, iz, part > 0 && ks % SHARE == 0 ? 0u : 1u);
-        }
-      } else {
-#pragma unroll
-        for (int ks = 0; ks < KP / 8; ++ks) {
-          const uint64_t ko = 16u * ks;
-          tc::mma_tf32(tmem, dph + ko, dyh + ko, iz, ks > 0 ? 1u : 0u);
-          tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, 1u);
-          tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
-        }
+      for (int ks = 0; ks < KP / 8; ++ks) {
+        const int part = ks / SHARE;
+        tc::mma_tf32(tmem + (part > 0 ? C::ZX + 2 * TM * (part - 1) : 0), dph + 16u * ks,
+                     dyh + 16u * ks, iz, part > 0 && ks % SHARE == 0 ? 0u : 1u);
       }
       tc::commit(&bars[0]);
     }
@@ -1773,9 +1763,9 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
 #pragma unroll
       for (int ks = 0; ks < TM / 8; ++ks) {
         const uint64_t ko = 16u * ks;
-        const uint32_t acc = (any || ks > 0) ? 1u : 0u, dl = C::SPREAD ? d + KP : d;
+        const uint32_t acc = (any || ks > 0) ? 1u : 0u, dl = d + KP;
         tc::mma_tf32(d, dah + ko, dbh + ko, ig, acc);
-        tc::mma_tf32(dl, dah + ko, dbl + ko, ig, C::SPREAD ? acc : 1u);
+        tc::mma_tf32(dl, dah + ko, dbl + ko, ig, acc);
         tc::mma_tf32(dl, dal + ko, dbh + ko, ig, 1u);
       }
       tc::commit(&bars[1]);
@@ -1798,12 +1788,10 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       if (ok && any) {
         const uint32_t at = tmem + ((uint32_t)(32 * sub) << 16) + (uint32_t)(2 * TM + ic);
         tc::tmem_ld4(at, v);
-        if constexpr (C::SPREAD) {
-          float lo[4];
-          tc::tmem_ld4(at + KP, lo);
+        float lo[4];
+        tc::tmem_ld4(at + KP, lo);
 #pragma unroll
-          for (int u = 0; u < 4; ++u) v[u] += lo[u];
-        }
+        for (int u = 0; u < 4; ++u) v[u] += lo[u];
       }
       if (j < KP)
 #pragma unroll
@@ -2959,8 +2947,8 @@ int stpm_partial_grid(int mode, int k, int64_t count, bool bf16) {
   // one wave: a second one repeats the per-CTA costs for a few CTAs (8,192
   // nodes, k = 100: 128 CTAs where 120 fit took 55 / 95 us in the loss and
   // adjoint forms, 39 / 69 us with 88).  As few CTAs as keep the largest share
-  // of tiles per CTA.  Not the tensor-core plain form with one chain per sum
-  // (KP = 32), where more tiles per CTA cost accuracy.
+  // of tiles per CTA.  Not the tensor-core plain form of KP = 32: its
+  // accumulators truncate, and its small grids have little to gain.
   const int KP = stpm_kp(k);
   const bool truncating = !bf16 && mode == kModePlain && KP <= 32;
   const int64_t resident = KP < 0 || truncating ? 0
