@@ -704,9 +704,13 @@ __global__ void __launch_bounds__(384) jacobi_small_kernel(int p, const double* 
       const bool live = s < m / 2 && j < p;
       float* xi = X + (live ? i : 0) * ld + l8;
       float* xj = X + (live ? j : 0) * ld + l8;
-      float x[NV], y[NV];
+      // (threads without a pair load nothing: their column 0 has an owner that
+      // may be storing it)
+      float x[NV] = {}, y[NV] = {};
+      if (live) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) x[v] = xi[8 * v], y[v] = xj[8 * v];
+        for (int v = 0; v < NV; ++v) x[v] = xi[8 * v], y[v] = xj[8 * v];
+      }
       float al = 0.f, be = 0.f, ga = 0.f;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
