@@ -334,7 +334,8 @@ __global__ void __launch_bounds__(256, 1) chol_upper_cluster_kernel(int p, const
   T* Rl = chs;                                   // Rl[lc p + i]
   T* BR = Rl + (size_t)ncl * p;                  // row block: BR[c p + i] = R[jb + c, i]
   __shared__ T DJ[KB * KB];                 // DJ[cc KB + c] = R[jb + c, jb + cc]
-  __shared__ T DI[KB];                      // 1 / R[jb + c, jb + c] (0 where dropped)
+  __shared__ T DR[KB];                      // R[jb + c, jb + c] (0 where dropped; FP64 form)
+  __shared__ T DI[KB];                      // and its reciprocal (0 where dropped)
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   for (int e = tid; e < ncl * p; e += nt) {
     const int lc = e / p, i = e % p, l = lc * CL + rank;
@@ -354,30 +355,29 @@ __global__ void __launch_bounds__(256, 1) chol_upper_cluster_kernel(int p, const
     }
     __syncthreads();
     if constexpr (std::is_same<T, double>::value) {
-      // FP64: 4 warps, 2 entries per thread, root-free: entry (i, l) -= a_ci (a_cl
-      // / a_cc), the reciprocal from an FP32 start and formed by every thread (a
-      // warp's FP64 instruction takes 64 cycles here whatever its lanes do, and
-      // a square root and a division per pivot took 1.3k); the rows are scaled by
-      // 1 / sqrt(a_cc) at the end.
+      // FP64: 4 warps, 2 entries per thread.  Every thread forms the pivot's root
+      // and reciprocal and scales the two entries of row c that it needs; row c
+      // itself is scaled at the end, so a pivot takes one barrier.  The products
+      // are those of the column-by-column form, bit for bit: the signs of the
+      // eigenvectors behind this factor hang on its last bits (root-free, with the
+      // rows scaled at the end, 28 of 70 graphs with k from 130 on came out in
+      // another frame).  p = 200: 290 us (182 us root-free).
       if (tid < 128) {
         static_assert(KB == 16, "two entries per thread");
         for (int c = 0; c < bs; ++c) {
           const double d = DJ[c * KB + c];
-          double inv = 0.0;
-          if (d > drop2) {
-            if (d > 1e-30 && d < 1e30) {
-              const double y = (double)__frcp_rn((float)d), e = fma(-d, y, 1.0);
-              inv = fma(y * e, 1.0 + e, y);  // e ~ 2^-24: the error is e^3
-            } else {
-              inv = 1.0 / d;
-            }
+          const double r = d > drop2 ? sqrt(d) : 0.0, ri = r > 0.0 ? 1.0 / r : 0.0;
+          if (tid == 0) {
+            if (!(d > drop2) && !(d == d)) atomicOr(flags, kFlagNonFinite);
+            DR[c] = r;
+            DI[c] = ri;
           }
           double v[2];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int e = tid + 128 * h, i = e % KB, l = e / KB;
             v[h] = DJ[e];
-            if (i > c && i <= l && l < bs) v[h] = fma(-DJ[i * KB + c], DJ[l * KB + c] * inv, v[h]);
+            if (i > c && i <= l && l < bs) v[h] = fma(-(DJ[i * KB + c] * ri), DJ[l * KB + c] * ri, v[h]);
           }
 #pragma unroll
           for (int h = 0; h < 2; ++h) {  // (row c, read by others, is not written)
@@ -386,17 +386,11 @@ __global__ void __launch_bounds__(256, 1) chol_upper_cluster_kernel(int p, const
           }
           asm volatile("bar.sync 1, 128;" ::: "memory");
         }
-        if (tid < bs) {
-          const double d = DJ[tid * KB + tid];
-          if (!(d == d)) atomicOr(flags, kFlagNonFinite);
-          DI[tid] = d > drop2 ? 1.0 / sqrt(d) : 0.0;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
         double v[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int e = tid + 128 * h, i = e % KB, l = e / KB;
-          v[h] = i <= l && l < bs ? DJ[e] * DI[i] : 0.0;
+          v[h] = i < l && l < bs ? DJ[e] * DI[i] : i == l && l < bs ? DR[i] : 0.0;
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) DJ[tid + 128 * h] = v[h];
@@ -1861,18 +1855,12 @@ static cudaError_t chol_upper_drop_t(int p, const double* S, int lds, double* R,
                                      unsigned* flags, cudaStream_t s) {
   if (p > 4096) return cudaErrorInvalidValue;
   // p > 64: a 16-CTA cluster (8 where 16 cannot be co-scheduled) while the
-  // columns and one row block fit shared memory, else one CTA
+  // columns and one row block fit shared memory, else one CTA a column at a time
+  // (p = 50: 78 us, the blocked form on one CTA 82 us)
   constexpr int KB = 16;
   static int wide = -1;
-  if (p <= 64) {
-    // the blocked form on one CTA, in FP64 for either type (64 us at p = 50 with
-    // a column at a time and R in global memory, 51 us here)
-    const size_t sm = sizeof(double) * (size_t)(p + KB) * p;
-    cudaError_t e = launch_chol_cluster<1, KB, double>(p, S, lds, R, drop2, flags, sm, s);
-    if (e == cudaSuccess) ++g_launch_count;
-    return e;
-  }
   for (int cl : {16, 8}) {
+    if (p <= 64) break;
     if (cl == 16 && wide == 0) continue;
     const size_t sm = sizeof(T) * ((size_t)((p + cl - 1) / cl) + KB) * p;
     if (sm > 200 * 1024) break;
