@@ -1161,31 +1161,15 @@ __global__ void __launch_bounds__(1024) cgs2_cols_kernel(int m, int p, const dou
   }
 }
 
-// The same CGS2 with the rows spread over a cluster of CL CTAs and the columns
-// taken in blocks of kCgsBlock, so that the cluster-wide sums -- two DSMEM
-// round trips and a cluster barrier each, which bound the column-by-column form
-// (1.25 ms at m = 101, p = 200) -- come three per block instead of three per
-// column.  CTA r keeps rows [r R, r R + R) of every finished column of Q in
-// shared memory.  Per block V:
-//   1. V -= Q (Q^T V), twice: partial dot products over the own rows, summed
-//      over the cluster in rank order (identical in every CTA), own rows updated;
-//   2. every CTA gathers the whole block and runs CGS2 with the drop rule inside
-//      it, redundantly, without a cluster barrier;
-//   3. V -= Q (Q^T V) once more: what step 2 cancelled may have left components
-//      along Q of a relative size that step 1's round-off had in V.
-// m = 101, p = 200: 0.68 ms; m = 151, p = 300: 2.65 ms (3.66 ms before).
-constexpr int kCgsBlock = 8;
-
-template <int CL>
-struct CgsSmem {  // doubles, of a CTA
-  static __host__ __device__ int rows(int m) { return (m + CL - 1) / CL; }
-  static __host__ __device__ size_t doubles(int m, int p) {
-    const size_t R = rows(m), n = (size_t)(p + 1) * kCgsBlock;
-    // Q rows, block rows (3), partial sums (2), sums, the whole block
-    return R * p + 3 * R * kCgsBlock + 3 * n + (size_t)m * kCgsBlock;
-  }
-};
-
+// The same CGS2 with the rows spread over a cluster of CL CTAs, so that the
+// FP64 work (about 4 m p^2 / 2 multiply-adds) runs on CL SMs instead of one.
+// CTA r keeps rows [r R, r R + R) of every finished column of Q in shared
+// memory; each projection pass forms partial dot products over its rows, the
+// cluster sums them (every CTA reads all partials through DSMEM, adding in
+// rank order, so all CTAs hold identical sums and take identical branches),
+// and each CTA updates its own rows.  Three cluster barriers per column
+// (pass 1 with |v|^2, pass 2, the final norm); the partial buffers alternate
+// so that a buffer is rewritten only after every CTA has read it.
 template <int CL>
 __global__ void __launch_bounds__(256) cgs2_cols_cluster_kernel(int m, int p,
                                                                 const double* __restrict__ P,
@@ -1194,146 +1178,78 @@ __global__ void __launch_bounds__(256) cgs2_cols_cluster_kernel(int m, int p,
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double csh[];
-  constexpr int KB = kCgsBlock;
-  const int R = CgsSmem<CL>::rows(m);              // rows per CTA
+  const int R = (m + CL - 1) / CL;                 // rows per CTA
   const int rank = (int)cluster.block_rank();
   const int r0 = rank * R, nr = max(0, min(R, m - r0));
-  const int np = (p + 1) * KB;
   double* Qs = csh;                                 // Qs[i R + rr] = Q[r0 + rr, i]
-  // block rows, V[c R + rr]: one buffer each for even and odd blocks (other CTAs
-  // gather it; it is rewritten two blocks later, after a cluster barrier that
-  // every CTA reaches behind that gather) and one for step 3
-  double* Vb = Qs + (size_t)R * p;
-  double* V = Vb;
-  double* part = Vb + 3 * (size_t)R * KB;           // 2 x np partial sums
-  double* d = part + 2 * (size_t)np;                // d[i KB + c]
-  double* W = d + np;                               // the whole block: W[c m + r]
-  __shared__ double red[KB];
+  double* v = Qs + (size_t)R * p;                   // R
+  double* part = v + R;                             // 2 x (p + 1) partial sums
+  double* d = part + 2 * (p + 1);                   // p + 1 reduced sums
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   int buf = 0, kept = 0;
-  // d[i KB + c] = Q_i . V_c for i < cnt, and |V_c|^2 at i = cnt, c < bs
-  auto reduce = [&](int cnt, int bs) {
-    double* pb = part + (size_t)buf * np;
-    for (int e = tid; e < (cnt + 1) * KB; e += nt) {
-      const int i = e / KB, c = e % KB;
-      if (c >= bs) continue;
-      const double* q = i < cnt ? Qs + (size_t)i * R : V + (size_t)c * R;
+  // partial sums of Q_i . v (i < cnt) and, with_norm, |v|^2 in slot cnt;
+  // then the cluster-wide sums into d[0 .. cnt]
+  auto reduce = [&](int cnt, bool with_norm) {
+    double* pb = part + buf * (p + 1);
+    for (int i = tid; i < cnt; i += nt) {
       double s = 0.0;
-      for (int rr = 0; rr < nr; ++rr) s = fma(q[rr], V[(size_t)c * R + rr], s);
-      pb[e] = s;
+      for (int rr = 0; rr < nr; ++rr) s = fma(Qs[(size_t)i * R + rr], v[rr], s);
+      pb[i] = s;
+    }
+    if (with_norm && warp == 0) {
+      double s = 0.0;
+      for (int rr = lane; rr < nr; rr += 32) s = fma(v[rr], v[rr], s);
+#pragma unroll
+      for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+      if (lane == 0) pb[cnt] = s;
     }
     cluster.sync();
-    for (int e = tid; e < (cnt + 1) * KB; e += nt) {
-      if (e % KB >= bs) continue;
-      double t[CL];
-#pragma unroll
-      for (int q = 0; q < CL; ++q) t[q] = cluster.map_shared_rank(pb, q)[e];
-      double s = t[0];
-#pragma unroll
-      for (int q = 1; q < CL; ++q) s += t[q];
-      d[e] = s;
+    const int tot = cnt + (with_norm ? 1 : 0);
+    for (int i = tid; i < tot; i += nt) {
+      double s = 0.0;
+      for (int q = 0; q < CL; ++q) s += cluster.map_shared_rank(pb, q)[i];
+      d[i] = s;
     }
     buf ^= 1;
     __syncthreads();
   };
-  // V_c -= sum_{i < cnt} d_ic Q_i over this CTA's rows (4 lanes per entry)
-  auto subtract = [&](int cnt, int bs) {
-    for (int e0 = 0; e0 < nr * bs; e0 += nt / 4) {
-      const int e = e0 + (tid >> 2), h = tid & 3;
-      const bool live = e < nr * bs;
-      const int c = live ? e / nr : 0, rr = live ? e % nr : 0;
+  // v -= sum_{i < cnt} d_i Q_i over this CTA's rows (a warp per row)
+  auto subtract = [&](int cnt) {
+    for (int rr = warp; rr < nr; rr += nw) {
       double s = 0.0;
-      if (live)
-        for (int i = h; i < cnt; i += 4) s = fma(d[i * KB + c], Qs[(size_t)i * R + rr], s);
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      if (live && h == 0) V[(size_t)c * R + rr] -= s;
+      for (int i = lane; i < cnt; i += 32) s = fma(d[i], Qs[(size_t)i * R + rr], s);
+#pragma unroll
+      for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+      if (lane == 0) v[rr] -= s;
     }
     __syncthreads();
   };
-  for (int j0 = 0; j0 < p; j0 += KB) {
-    const int bs = min(KB, p - j0);
-    V = Vb + (size_t)((j0 / KB) & 1) * R * KB;
-    for (int e = tid; e < nr * bs; e += nt)
-      V[(size_t)(e / nr) * R + e % nr] = P[(int64_t)(j0 + e / nr) * ldp + r0 + e % nr];
+  for (int j = 0; j < p; ++j) {
+    for (int rr = tid; rr < nr; rr += nt) v[rr] = P[(int64_t)j * ldp + r0 + rr];
     __syncthreads();
-    reduce(j0, bs);  // pass 1 dots and the norms
-    if (kept == m) {
-      // the kept columns span R^m: the residual of a column is round-off,
-      // about 1e-15 |v|, below tol whenever |v| < 1e10 tol, and it is dropped
-      bool skip = true;
-      for (int c = 0; c < bs; ++c) skip = skip && d[j0 * KB + c] < (1e10 * tol) * (1e10 * tol);
-      if (skip) {  // the same in every CTA and thread
-        for (int e = tid; e < nr * bs; e += nt) {
-          const int c = e / nr, rr = e % nr;
-          Qs[(size_t)(j0 + c) * R + rr] = 0.0;
-          Q[(int64_t)(j0 + c) * ldq + r0 + rr] = 0.0;
-        }
-        __syncthreads();
-        continue;
-      }
-    }
-    subtract(j0, bs);
-    if (j0 > 0) {
-      reduce(j0, bs);  // pass 2
-      subtract(j0, bs);
-    }
-    cluster.sync();  // every CTA's rows of the block are final
-    for (int e = tid; e < m * bs; e += nt) {
-      const int c = e / m, r = e % m;
-      W[e] = cluster.map_shared_rank(V, r / R)[(size_t)c * R + r % R];
-    }
-    __syncthreads();
-    // CGS2 inside the block, the same in every CTA
-    for (int c = 0; c < bs; ++c) {
-      double* v = W + (size_t)c * m;
-      for (int pass = 0; pass < 2 && c > 0; ++pass) {
-        for (int i = warp; i < c; i += nw) {
-          double s = 0.0;
-          for (int r = lane; r < m; r += 32) s = fma(W[(size_t)i * m + r], v[r], s);
-#pragma unroll
-          for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-          if (lane == 0) red[i] = s;
-        }
-        __syncthreads();
-        for (int r = tid; r < m; r += nt) {
-          double s = 0.0;
-          for (int i = 0; i < c; ++i) s = fma(red[i], W[(size_t)i * m + r], s);
-          v[r] -= s;
-        }
-        __syncthreads();
-      }
-      if (warp == 0) {
-        double s = 0.0;
-        for (int r = lane; r < m; r += 32) s = fma(v[r], v[r], s);
-#pragma unroll
-        for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        if (lane == 0) red[c] = s > tol * tol ? rsqrt(s) : 0.0;
+    reduce(j, true);  // pass 1 dots and |v|^2
+    // the kept columns span R^m: the residual of v is round-off, about
+    // 1e-15 |v|, below tol whenever |v| < 1e10 tol, and the column is dropped
+    if (kept == m && sqrt(d[j]) < 1e10 * tol) {
+      for (int rr = tid; rr < nr; rr += nt) {
+        Qs[(size_t)j * R + rr] = 0.0;
+        Q[(int64_t)j * ldq + r0 + rr] = 0.0;
       }
       __syncthreads();
-      const double sc = red[c];
-      if (sc > 0.0) ++kept;
-      for (int r = tid; r < m; r += nt) v[r] *= sc;
-      __syncthreads();
+      continue;
     }
-    // own rows back, and the last projection on the earlier columns (a dropped
-    // column stays zero)
-    V = Vb + 2 * (size_t)R * KB;
-    for (int e = tid; e < nr * bs; e += nt) {
-      const int c = e / nr, rr = e % nr;
-      V[(size_t)c * R + rr] = W[(size_t)c * m + r0 + rr];
+    subtract(j);
+    reduce(j, false);  // pass 2
+    subtract(j);
+    reduce(0, true);   // |v|^2 after both passes
+    const double nn = sqrt(d[0]);
+    const double sc = nn > tol ? 1.0 / nn : 0.0;
+    for (int rr = tid; rr < nr; rr += nt) {
+      const double qv = v[rr] * sc;
+      Qs[(size_t)j * R + rr] = qv;
+      Q[(int64_t)j * ldq + r0 + rr] = qv;
     }
-    __syncthreads();
-    if (j0 > 0) {
-      reduce(j0, bs);
-      subtract(j0, bs);
-    }
-    for (int e = tid; e < nr * bs; e += nt) {
-      const int c = e / nr, rr = e % nr;
-      const double q = V[(size_t)c * R + rr];
-      Qs[(size_t)(j0 + c) * R + rr] = q;
-      Q[(int64_t)(j0 + c) * ldq + r0 + rr] = q;
-    }
+    if (nn > tol) ++kept;
     __syncthreads();
   }
   cluster.sync();  // keep shared memory alive until every remote read is done
@@ -2009,8 +1925,8 @@ cudaError_t mgs_cols(int m, int p, const double* P, int ldp, double* Q, int ldq,
   static int wide = -1;
   for (int cl : {16, 8}) {
     if (cl == 16 && wide == 0) continue;
-    const size_t smc =
-        sizeof(double) * (cl == 16 ? CgsSmem<16>::doubles(m, p) : CgsSmem<8>::doubles(m, p));
+    const int rows = (m + cl - 1) / cl;
+    const size_t smc = sizeof(double) * ((size_t)rows * p + rows + 3 * ((size_t)p + 1));
     if (smc > 200 * 1024) break;
     cudaError_t e = cl == 16 ? launch_cgs2_cluster<16>(m, p, P, ldp, Q, ldq, tol, smc, s)
                              : launch_cgs2_cluster<8>(m, p, P, ldp, Q, ldq, tol, smc, s);

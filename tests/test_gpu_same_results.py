@@ -64,7 +64,9 @@ def frames(mm, k, seed):
 
 # frames that another rounding of the Cholesky factors turned
 TURNED = [(130, 2), (130, 19), (150, 3), (150, 6), (200, 1), (200, 4)]
-FRAMES = TURNED
+# last bits that another order of the Gram-Schmidt's sums changed
+BITS_GS = [(100, 0), (100, 8), (130, 1)]
+FRAMES = sorted(set(TURNED + BITS_GS))
 
 
 @pytest.mark.parametrize("k,seed", TURNED)
@@ -72,3 +74,10 @@ def test_whitening_keeps_its_frame(mm, k, seed):
     with np.load(GOLDEN / "frames.npz") as z:
         want = z[f"mu_{k}_{seed}"]
     assert rel(frames(mm, k, seed)[f"mu_{k}_{seed}"], want) < 2e-5
+
+
+@pytest.mark.parametrize("k,seed", BITS_GS)
+def test_whitening_keeps_its_bits(mm, k, seed):
+    with np.load(GOLDEN / "frames.npz") as z:
+        want = z[f"digest_{k}_{seed}"]
+    assert np.array_equal(frames(mm, k, seed)[f"digest_{k}_{seed}"], want)
