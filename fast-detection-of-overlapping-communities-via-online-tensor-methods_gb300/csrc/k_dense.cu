@@ -146,13 +146,28 @@ int gram_nsplit(int64_t n, int pa, int pb) {
 // every CTA (with that, and 16-byte loads of F, two concurrent products of n =
 // 50,000, p = q = 200 went from 271 to 258 us; the shared memory's bandwidth sets
 // the rest).  Results outside the normal FP32 range take the conversion.
-__device__ __forceinline__ float narrow(double x) {
+__device__ __forceinline__ bool narrows(double x) {  // to a normal FP32 number (or past the largest)
+  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 897u <= 253u;
+}
+
+__device__ __forceinline__ float narrow_normal(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const unsigned e = (hi >> 20) & 0x7ffu;
-  if (e - 897u > 253u) return x == 0.0 ? __uint_as_float(hi & 0x80000000u) : (float)x;
   const unsigned m = ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
   const unsigned rem = lo & 0x1fffffffu;
   return __uint_as_float((hi & 0x80000000u) | (m + (rem + (m & 1u) > 0x10000000u ? 1u : 0u)));
+}
+
+__device__ __forceinline__ float narrow(double x) {
+  if (!narrows(x)) return x == 0.0 ? __uint_as_float((unsigned)__double2hiint(x) & 0x80000000u) : (float)x;
+  return narrow_normal(x);
+}
+
+// (double)x of a normal number the same way
+__device__ __forceinline__ double widen_normal(float x) {
+  const unsigned u = __float_as_uint(x);
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))),
+                          (int)(u << 29));
 }
 
 constexpr int PT_R = 64, PT_C = 64, PT_K = 32;
@@ -1635,33 +1650,40 @@ __global__ void panel_to_colmajor_kernel(const float* __restrict__ P, int ldp, i
 }
 
 // out = P with column j < q scaled by d[j] (row-major, ld a multiple of 4, also
-// in place).  A warp per row, 16 bytes per lane; the factor as a pair of floats,
-// P dh + P dl in one fma, rounds as the FP64 product does but for its ties (an
-// FP64 multiplication and two conversions per entry made it 35 us for 50,000 x
-// 100; 15 us here, the copy before it included).
-__global__ void __launch_bounds__(256) scale_cols_kernel(const float4* __restrict__ P, int ld4,
-                                                         int64_t n, int q,
+// in place).  A warp per row, 16 bytes per lane.  Bound by the FP64 unit: one
+// FP64 product per entry, rounded to FP32 (the products stand in front of the
+// eigensolvers, whose vectors' signs hang on every rounding), with the
+// conversions on both sides in integer arithmetic where all four entries allow it
+// (a branch: as a select the conversions ran all the same).  50,000 x 100: 18.5 us
+// (31 us as a select; 35 us with conversions and the copy before it).
+__global__ void __launch_bounds__(256) scale_cols_kernel(const float4* P, int ld4, int64_t n, int q,
                                                          const double* __restrict__ d,
-                                                         float4* __restrict__ out) {
+                                                         float4* out) {
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int c0 = 0; c0 < ld4; c0 += 32) {
     const int c4 = c0 + lane;
-    float dh[4], dl[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int c = 4 * c4 + u;
-      const double v = c4 < ld4 && c < q ? d[c] : 1.0;
-      dh[u] = (float)v;
-      dl[u] = (float)(v - (double)dh[u]);
-    }
     if (c4 >= ld4) continue;
+    double f[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) f[u] = 4 * c4 + u < q ? d[4 * c4 + u] : 1.0;
     for (int64_t r = (int64_t)blockIdx.x * nw + (threadIdx.x >> 5); r < n; r += (int64_t)gridDim.x * nw) {
-      float4 x = P[r * ld4 + c4];
-      x.x = fmaf(x.x, dh[0], x.x * dl[0]);
-      x.y = fmaf(x.y, dh[1], x.y * dl[1]);
-      x.z = fmaf(x.z, dh[2], x.z * dl[2]);
-      x.w = fmaf(x.w, dh[3], x.w * dl[3]);
-      out[r * ld4 + c4] = x;
+      const float4 v = P[r * ld4 + c4];
+      const float x[4] = {v.x, v.y, v.z, v.w};
+      float y[4];
+      bool plain = true;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) plain = plain && ((__float_as_uint(x[u]) >> 23) & 0xffu) - 1u <= 253u;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double t = widen_normal(x[u]) * f[u];
+        plain = plain && narrows(t);
+        y[u] = narrow_normal(t);
+      }
+      if (!plain) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[u] = (float)((double)x[u] * f[u]);
+      }
+      out[r * ld4 + c4] = make_float4(y[0], y[1], y[2], y[3]);
     }
   }
 }
