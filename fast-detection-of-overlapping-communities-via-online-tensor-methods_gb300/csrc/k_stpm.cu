@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(256) stpm_reduce_kernel(StpmReduceArgs a) {
 // first-order product is on the own rows as well.  (Owning columns instead
 // took an exchange of X, of A and of Q1 per pass, the triangular inverse and
 // three k^3 products: a minibatch step, contraction included, took 54 us at
-// k = 100, 20.6 us at k = 10 and 330 us at k = 200; 45, 15.3 and 295 us here.)  At KP = 32 one CTA holds everything
-// and nothing is exchanged.
+// k = 100 and 330 us at k = 200; 45 and 295 us here.)  KP = 32 has a form of its
+// own (k_step32.cuh).
 //
 // All products are FP32 FMAs (a thread per column, 8 rows at a time, the row
 // operand broadcast from shared memory): mma.sync TF32 in 3xTF32 form gives
@@ -268,12 +268,11 @@ constexpr int kMaxShifts = 3;
 // columns fall into different banks
 __host__ __device__ constexpr int step_xld(int KP) { return KP + 4; }
 
-// CTAs of the step cluster: one at KP = 32 (the exchanges would cost more than
-// the products they split), KP / 8 to 128, KP / 16 above (at most 16).  A step of
+// CTAs of the step cluster: KP / 8 to 128, KP / 16 above (at most 16).  A step of
 // 4,000 nodes at k = 45, contraction included: 35.8 us with one CTA, 29.4 us
 // with KP / 16, 27.8 us with KP / 8; 5,000 nodes at k = 64: 43.6, 33.2, 31.3 us.
 __host__ __device__ constexpr int step_ctas(int KP) {
-  return KP <= 32 ? 1 : KP <= 128 ? KP / 8 : KP / 16;
+  return KP <= 128 ? KP / 8 : KP / 16;
 }
 
 template <int KP, int CL>
@@ -284,13 +283,13 @@ struct StepSmem {
   // cluster barriers
   static constexpr bool PULL = KP > 128;
   static constexpr int PW = (KP + RB + 63) / 64, BW = NT / 32 - PW - 1;  // panel, bulk warps
-  static constexpr size_t recv = CL > 1 && !PULL ? (size_t)KP * XLD : 0;
+  static constexpr size_t recv = !PULL ? (size_t)KP * XLD : 0;
   static constexpr size_t rows = (size_t)RB * XLD;
   // matrix, partials, X rows | Q1 rows | block to send, m1..3 and |phi_i|^2,
   // mu1..3, d-sums, original diagonal, diagonal block
   static constexpr size_t floats = (size_t)KP * XLD + recv + 3 * rows + 11 * KP + 128;
   static_assert(KP % CL == 0 && RB % 8 == 0 && BW >= 4, "row blocks of whole 8-row blocks");
-  static_assert(KP <= 256 && (CL > 1 || KP <= 32), "16-byte words per column");
+  static_assert(KP <= 256 && CL > 1, "16-byte words per column");
   static_assert(floats * sizeof(float) <= 227 * 1024 - 1024, "step kernel shared memory");
 };
 
@@ -621,7 +620,7 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
   constexpr int RB = S::RB, XLD = S::XLD, NT = S::NT;
   // one warp of the 512 threads issues the copy to each rank
   static_assert(CL <= 16, "cluster size");
-  const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
+  const int rank = (int)cg::this_cluster().block_rank();
   extern __shared__ __align__(16) float sm[];
   float* A = sm;                       // Phi, then Grams and factors, columns at A + c XLD
   float* Rv = A + KP * XLD;            // column block of the Gram partials of every rank
@@ -665,12 +664,10 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
       const float* mu = which == 0 ? a.mu1 : which == 1 ? a.mu2 : a.mu3;
       mus[e] = (mu && j < k) ? __ldg(mu + j) : 0.f;
     }
-  if (CL > 1) {
-    if (tid < CL) mbar_init(&s_part[tid], 1);
-    else if (tid < 2 * CL) mbar_init(&s_blk[tid - CL], 1);
-    else if (tid < 2 * CL + 2) mbar_init(&s_csync[tid - 2 * CL], CL);
-    if (tid < 2 * CL + 2) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
+  if (tid < CL) mbar_init(&s_part[tid], 1);
+  else if (tid < 2 * CL) mbar_init(&s_blk[tid - CL], 1);
+  else if (tid < 2 * CL + 2) mbar_init(&s_csync[tid - 2 * CL], CL);
+  if (tid < 2 * CL + 2) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
   if (online) {
     // mean terms phi_i . mu and |phi_i|^2 of all columns: Phi and mu only, so
@@ -698,7 +695,7 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
       }
     }
   }
-  if (CL > 1) cg::this_cluster().sync();  // barriers initialised everywhere before any copy
+  cg::this_cluster().sync();  // barriers initialised everywhere before any copy
   // launched with programmatic serialization after the contraction, the
   // prologue above overlapped its tail (Phi is final: the contraction lets
   // this kernel start only after its own wait on the previous step); from
@@ -798,18 +795,6 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
       return make_float4(w[0], w[1], w[2], w[3]);
     };
     const int cols = max(0, min(RB, kk - r0)), n4 = kk / 4;
-    if (CL == 1) {
-      __syncthreads();
-#pragma unroll 1
-      for (int e = tid; e < cols * 16; e += NT) {  // (n4 <= 16)
-        const int c = e >> 4, i4 = e & 15;
-        float4* p = reinterpret_cast<float4*>(A + c * XLD) + i4;
-        if (i4 < n4) *p = finish(*p, c, i4);
-      }
-      if (bad) atomicOr(a.flags, kFlagNonFinite);
-      __syncthreads();
-      return true;
-    }
     bool ok = true;
     if (!S::PULL) {
       // column block s of the partial to rank s, rank q's next neighbours
@@ -879,7 +864,6 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
   // whether any rank's block of E had an entry above kFirstOrderBelow (the
   // same in every CTA: the blocks carry it in their padding)
   auto more_orders = [&]() -> bool {
-    if (CL == 1) return __syncthreads_or(emax > kFirstOrderBelow) != 0;
     bool more = false;
     for (int q = 0; q < CL; ++q) more = more || A[q * RB * XLD + KP] != 0.f;
     return more;
@@ -1036,7 +1020,7 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
       ++orders;
       // no copy to this CTA is outstanding after the last pass; its own may
       // still be read by others, so it stays until every rank has arrived here
-      if (CL > 1 && !more) csync_arrive();
+      if (!more) csync_arrive();
       // own rows of M - M F: RT rows of one column per item, F's column in
       // 16-byte words down to the diagonal
       constexpr int RT = RB >= 32 ? 4 : 2;
@@ -1173,29 +1157,13 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
   }
   if (timed_out && tid == 0) atomicOr(a.flags, kFlagTimeout);
   if (rank == 0 && tid == 0 && a.orth_passes) atomicAdd(a.orth_passes, passes);
-  if (CL > 1) {
-    // keep shared memory alive until remote readers and writers are done
-    // (bounded: after a timeout the ranks may stand at different barriers)
-    if (timed_out) csync_arrive();
-    if (!csync_wait()) {
-      if (tid == 0) atomicOr(a.flags, kFlagTimeout);
-      __nanosleep(100000);  // let copies a stalled exchange left in flight land
-    }
+  // keep shared memory alive until remote readers and writers are done
+  // (bounded: after a timeout the ranks may stand at different barriers)
+  if (timed_out) csync_arrive();
+  if (!csync_wait()) {
+    if (tid == 0) atomicOr(a.flags, kFlagTimeout);
+    __nanosleep(100000);  // let copies a stalled exchange left in flight land
   }
-}
-
-template <int KP, int CL>
-__global__ void __launch_bounds__(512, 1) stpm_step_kernel(StpmUpdateArgs a) {
-  step_body<KP, CL>(a);
-}
-
-// one cluster per graph: blockIdx.y selects the graph's arguments; graphs
-// with no update in this round (active == 0) leave at once
-template <int KP, int CL>
-__global__ void __launch_bounds__(512, 1) stpm_step_batched(const StpmUpdateArgs* __restrict__ args) {
-  const StpmUpdateArgs a = args[blockIdx.y];
-  if (!a.active) return;
-  step_body<KP, CL>(a);
 }
 
 // ---- partial contractions on the tensor cores -----------------------------------
@@ -1225,8 +1193,8 @@ __global__ void __launch_bounds__(512, 1) stpm_step_batched(const StpmUpdateArgs
 // three accumulators, and the small products of G have one of their own.  The
 // first steps of a run, where the iterate is near singular, multiply that error
 // by 10 to 50: after 4 of them Phi was 3.6e-5 off at k = 100 (median of 8 runs)
-// with one chain of each and 1.5e-5 here, 0.9e-5 and 0.6e-5 at k = 33,
-// 0.41e-5 and 0.32e-5 at k = 24.  Operands are
+// with one chain of each and 1.5e-5 here, 0.9e-5 and 0.6e-5 at k = 33.  (KP = 32
+// keeps one chain of each, see CHAIN.)  Operands are
 // staged hi / lo in shared memory, K-major without swizzle; y3 is staged
 // transposed (node index along K).  An M = 128 operand of KP < 128 rows
 // reads its rows past KP from the buffer after it: their products land in
@@ -1251,8 +1219,12 @@ struct ContractTc {
   static constexpr uint32_t REGION = ((REGION0 > STAGE ? REGION0 : STAGE) + 127) / 128 * 128;
   // alignment slack, m1 | m2, d-sums of the 4 node groups
   static constexpr size_t smem = 1024 + REGION + sizeof(float) * (2 * KP + 4 * KP);
+  // KP = 32: one accumulator for Z1 | Z2 and one for G, each a single chain, and
+  // Phi^T mu from the step kernel, behind the image: results up to k = 32 keep
+  // their roundings (k_step32.cuh)
+  static constexpr bool CHAIN = KP == 32;
   // further accumulators of Z1 | Z2: two, or one where two CTAs share an SM
-  static constexpr int NZX = KP <= 64 ? 1 : 2;
+  static constexpr int NZX = CHAIN ? 0 : KP <= 64 ? 1 : 2;
   static constexpr uint32_t ZX = 2 * TM + 2 * KP;
   static constexpr uint32_t TMEM_COLS = KP <= 64 ? 256 : 512;
   static_assert(ZX + NZX * 2 * TM <= TMEM_COLS, "tensor memory columns");
@@ -1260,6 +1232,24 @@ struct ContractTc {
   static_assert(KP % 16 == 0 && KP >= 32 && KP <= 112, "tensor-core contraction: KP in [32, 112]");
   static_assert(smem <= 227 * 1024, "tensor-core contraction shared memory");
 };
+
+#include "k_step32.cuh"
+
+template <int KP, int CL>
+__global__ void __launch_bounds__(512, 1) stpm_step_kernel(StpmUpdateArgs a) {
+  if constexpr (KP == 32) step32::body(a);
+  else step_body<KP, CL>(a);
+}
+
+// one cluster per graph: blockIdx.y selects the graph's arguments; graphs
+// with no update in this round (active == 0) leave at once
+template <int KP, int CL>
+__global__ void __launch_bounds__(512, 1) stpm_step_batched(const StpmUpdateArgs* __restrict__ args) {
+  const StpmUpdateArgs a = args[blockIdx.y];
+  if (!a.active) return;
+  if constexpr (KP == 32) step32::body(a);
+  else step_body<KP, CL>(a);
+}
 
 // BF16 tensor-core form of the adjoint contraction (tcgen05.mma kind::f16,
 // BF16 operands, FP32 accumulation), for KP in [32, 112]: per tile of TM = 64
@@ -1580,7 +1570,7 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
     if (tid < 2 * KP) mv[tid] = m;
     __syncthreads();
   };
-  bool need_means = a.phi_img != nullptr;
+  bool need_means = !C::CHAIN && a.phi_img != nullptr;
   if (a.phi_img) {
     // the previous step kernel wrote Phi's operand image: bulk copies of the
     // hi | lo image (in 4 pieces); Phi^T mu_q is formed behind the first
@@ -1594,6 +1584,14 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       for (int q = 0; q < 4; ++q)
         bulk_copy_g2s(base + C::PH + q * piece, static_cast<const unsigned char*>(a.phi_img) + q * piece,
                       piece, &bars[2]);
+    }
+    if constexpr (C::CHAIN) {
+      const float* mimg =
+          reinterpret_cast<const float*>(static_cast<const unsigned char*>(a.phi_img) + 2 * C::PSZ);
+      float m = 0.f;
+      if (tid < 2 * KP) m = mimg[tid];
+      __syncthreads();  // every read of mus done (mv and mus share storage)
+      if (tid < 2 * KP) mv[tid] = m;
     }
     if (!tc::mbar_wait(&bars[2], 0u, tc::wait_limit_or_default(a.wait_limit))) img_timed_out = true;
   } else {
@@ -1673,12 +1671,13 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
 #pragma unroll
       for (int ks = 0; ks < KP / 8; ++ks) {
         const uint64_t ko = 16u * ks;
-        tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, ks > 0 ? 1u : 0u);
+        if (C::CHAIN) tc::mma_tf32(tmem, dph + ko, dyh + ko, iz, ks > 0 ? 1u : 0u);
+        tc::mma_tf32(tmem, dph + ko, dyl + ko, iz, C::CHAIN || ks > 0 ? 1u : 0u);
         tc::mma_tf32(tmem, dpl + ko, dyh + ko, iz, 1u);
       }
       constexpr int SHARE = (KP / 8 + C::NZX) / (C::NZX + 1);
 #pragma unroll
-      for (int ks = 0; ks < KP / 8; ++ks) {
+      for (int ks = 0; ks < (C::CHAIN ? 0 : KP / 8); ++ks) {
         const int part = ks / SHARE;
         tc::mma_tf32(tmem + (part > 0 ? C::ZX + 2 * TM * (part - 1) : 0), dph + 16u * ks,
                      dyh + 16u * ks, iz, part > 0 && ks % SHARE == 0 ? 0u : 1u);
@@ -1763,9 +1762,9 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
 #pragma unroll
       for (int ks = 0; ks < TM / 8; ++ks) {
         const uint64_t ko = 16u * ks;
-        const uint32_t acc = (any || ks > 0) ? 1u : 0u, dl = d + KP;
+        const uint32_t acc = (any || ks > 0) ? 1u : 0u, dl = C::CHAIN ? d : d + KP;
         tc::mma_tf32(d, dah + ko, dbh + ko, ig, acc);
-        tc::mma_tf32(dl, dah + ko, dbl + ko, ig, acc);
+        tc::mma_tf32(dl, dah + ko, dbl + ko, ig, C::CHAIN ? 1u : acc);
         tc::mma_tf32(dl, dal + ko, dbh + ko, ig, 1u);
       }
       tc::commit(&bars[1]);
@@ -1788,10 +1787,12 @@ __device__ __forceinline__ void contract_tc(const StpmPartialArgs& a, int nblock
       if (ok && any) {
         const uint32_t at = tmem + ((uint32_t)(32 * sub) << 16) + (uint32_t)(2 * TM + ic);
         tc::tmem_ld4(at, v);
-        float lo[4];
-        tc::tmem_ld4(at + KP, lo);
+        if (!C::CHAIN) {
+          float lo[4];
+          tc::tmem_ld4(at + KP, lo);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] += lo[u];
+          for (int u = 0; u < 4; ++u) v[u] += lo[u];
+        }
       }
       if (j < KP)
 #pragma unroll
@@ -2810,8 +2811,16 @@ cudaError_t launch_partial_batched_m(int KP, const StpmPartialArgs* args, int gr
 }
 
 template <int KP, int CL>
+constexpr size_t step_smem() {
+  if constexpr (KP == 32)
+    return step32::kSmem;
+  else
+    return sizeof(float) * StepSmem<KP, CL>::floats;
+}
+
+template <int KP, int CL>
 cudaError_t launch_step_t(const StpmUpdateArgs& a, cudaStream_t s) {
-  const size_t smem = sizeof(float) * StepSmem<KP, CL>::floats;
+  const size_t smem = step_smem<KP, CL>();
   static bool set = false;
   if (!set) {
     MMSB_CUDA_TRY(cudaFuncSetAttribute(stpm_step_kernel<KP, CL>,
@@ -2864,7 +2873,7 @@ cudaError_t launch_step_k(const StpmUpdateArgs& a, cudaStream_t s) {
 
 template <int KP, int CL>
 cudaError_t launch_step_batched_t(const StpmUpdateArgs* args, int graphs, cudaStream_t s) {
-  const size_t smem = sizeof(float) * StepSmem<KP, CL>::floats;
+  const size_t smem = step_smem<KP, CL>();
   static bool set = false;
   if (!set) {
     MMSB_CUDA_TRY(cudaFuncSetAttribute(stpm_step_batched<KP, CL>,
@@ -3011,7 +3020,8 @@ int stpm_step_kp(int k) { return stpm_kp(k); }
 size_t stpm_phi_image_bytes(int k) {
   const int kp = stpm_kp(k);
   if (kp < 32 || kp > 112) return 0;
-  return (size_t)8 * kp * kp;  // hi | lo (ContractTc<KP>::PSZ each)
+  // hi | lo (ContractTc<KP>::PSZ each); at KP = 32 then m1 | m2
+  return (size_t)8 * kp * kp + (kp == 32 ? (size_t)8 * kp : 0);
 }
 
 cudaError_t stpm_partial_batched(int mode, int KP, const StpmPartialArgs* args, int graphs,

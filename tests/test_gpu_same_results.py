@@ -83,3 +83,31 @@ def test_whitening_keeps_its_bits(mm, k, seed):
     with np.load(GOLDEN / "frames.npz") as z:
         want = z[f"digest_{k}_{seed}"]
     assert np.array_equal(frames(mm, k, seed)[f"digest_{k}_{seed}"], want)
+
+
+def solve(mm, method, precision, k, seed):
+    g = graph(mm, 77 + 1000 * k + seed, 2100 + 5 * (seed % 40), k, 0.3, 0.01)
+    cfg = dict(stpm_method=getattr(mm, "STPM_" + method), precision=getattr(mm, "PREC_" + precision),
+               sweeps=5, minibatch=-(-g.parts[0] // 8), seed=seed, tau=0.2)
+    with mm.Pipeline(k=k, alpha0=1.0, **cfg) as p:
+        p.upload(g).run()
+        lam, pi, phi = p.lam(), p.pi(), p.phi()
+    name = f"{method}_{precision}_{k}_{seed}"
+    return {"lam_" + name: np.asarray(lam), "digest_" + name: digest(pi, phi)}
+
+
+# graphs of 2,100 to 2,300 nodes whose lambda another rounding of the k x k step
+# or of the contraction moved by 2.6e-5 to 0.6
+MOVED = [("ONLINE", "FP32", 5, 1), ("ONLINE", "FP32", 5, 91), ("ONLINE", "FP32", 6, 22),
+         ("ONLINE", "FP32", 8, 27), ("ONLINE", "FP32", 12, 19), ("ONLINE", "BF16", 6, 6),
+         ("ONLINE", "BF16", 12, 8)]
+SOLVES = MOVED
+
+
+@pytest.mark.parametrize("method,precision,k,seed", MOVED)
+def test_solve_keeps_its_results(mm, method, precision, k, seed):
+    name = f"{method}_{precision}_{k}_{seed}"
+    got = solve(mm, method, precision, k, seed)
+    with np.load(GOLDEN / "solves.npz") as z:
+        assert rel(got["lam_" + name], z["lam_" + name]) < 2e-5
+        assert np.array_equal(got["digest_" + name], z["digest_" + name])
