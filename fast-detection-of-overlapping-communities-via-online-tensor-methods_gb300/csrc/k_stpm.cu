@@ -1299,6 +1299,10 @@ template <int KP, int MODE, bool BF>
 struct Contract {
   static constexpr bool TC = MODE == kModePlain && !BF && KP <= 112;
   static constexpr bool TCBF = MODE == kModeAdjoint && BF && KP <= 112;
+  // FP32 on mma.sync in 3xTF32 form: the adjoint steps of KP = 32, whose results
+  // keep their roundings (k_step32.cuh); the other FP32 forms off tcgen05 are FFMA
+  static constexpr bool MMA32 = MODE == kModeAdjoint && !BF && KP == 32;
+  static constexpr bool FFMA = !BF && !TC && !MMA32;
   using T = typename std::conditional<BF, __nv_bfloat16, float>::type;
   // two CTAs per SM up to KP = 64 (64 registers a thread: without the bound the
   // compiler takes 82 at KP = 48, and an iteration of the power method at k = 33,
@@ -1340,11 +1344,11 @@ struct Contract {
   static constexpr size_t DPART = ((size_t)KP * IB + 3 * IB + 4 + 3) / 4 * 4;
   static constexpr size_t stage_bytes =
       sizeof(float) *
-      (DPART + (BF ? 0 : (size_t)(TM / 2) * 3 * IB + (size_t)(GPARTS - 1) * KP * IB));
+      (DPART + (FFMA ? (size_t)(TM / 2) * 3 * IB + (size_t)(GPARTS - 1) * KP * IB : 0));
   static constexpr size_t region = ((tile_bytes > stage_bytes ? tile_bytes : stage_bytes) + 15) / 16 * 16;
-  // m1..3, loss partials, and the warps' d-sums (BF16) or mu1..3 (FP32)
+  // m1..3, loss partials, and the warps' d-sums (MMA) or mu1..3 (FFMA)
   static constexpr size_t smem_mma =
-      region + sizeof(float) * (3 * IB + NW + (BF ? NW * 3 * IB : 3 * KP));
+      region + sizeof(float) * (3 * IB + NW + (FFMA ? 3 * KP : NW * 3 * IB));
   static_assert(TC || TCBF || smem_mma <= 227 * 1024 - 1024, "contraction shared memory");
   static constexpr size_t smem = contract_smem<KP, TC, TCBF>(smem_mma);
   static_assert(NBC <= 4, "one loss slot per column block");
@@ -1374,6 +1378,14 @@ __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(smem_addr(p)));
+}
+
+// v = hi + lo with hi rounded to TF32; lo is passed as full FP32 bits: a TF32
+// MMA reads only the top 19 bits of an operand, so lo enters truncated to
+// TF32 (|error| <= 2^-10 |lo| <= 2^-21 |v|) without a second conversion
+__device__ __forceinline__ void split_tf32(float v, uint32_t& hi, uint32_t& lo) {
+  hi = step32::tf32_round(v);
+  lo = __float_as_uint(v - __uint_as_float(hi));
 }
 
 // The cluster's CTAs staged their partials (column block cb: G block, 3
@@ -2374,11 +2386,11 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
     contract_tc_bf<KP>(a, nblocks, smraw, stage);
     partial_cluster_sum<KP, IB, Cfg::NBC, MODE>(a, stage, 0, 0);
     return;
-  } else if constexpr (!BF) {
+  } else if constexpr (Cfg::FFMA) {
     contract_ffma<KP, MODE>(a, nblocks, smraw);
     return;
   }
-  if constexpr (BF) {
+  if constexpr (BF || Cfg::MMA32) {
   // programmatic serialization: wait for the previous kernel (the step that
   // wrote Phi), then let the next one be scheduled early
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -2470,9 +2482,11 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
           const int q = e / (TM * NCH), rem = e % (TM * NCH), xx = rem / NCH, c = rem % NCH;
           v[u] = make_uint4(0u, 0u, 0u, 0u);
           if (e < N) {
-            const T* Y = static_cast<const T*>(q == 0 ? a.yh1 : q == 1 ? a.yh2 : a.yh3);
-            if (xx < nvalid && c * CH < a.ldyh)
-              v[u] = __ldg(reinterpret_cast<const uint4*>(Y + (x0 + xx) * a.ldyh + c * CH));
+            const T* Y = BF ? static_cast<const T*>(q == 0 ? a.yh1 : q == 1 ? a.yh2 : a.yh3)
+                            : reinterpret_cast<const T*>(q == 0 ? a.y1 : q == 1 ? a.y2 : a.y3);
+            const int64_t ld = BF ? a.ldyh : a.ldy;
+            if (xx < nvalid && c * CH < ld)
+              v[u] = __ldg(reinterpret_cast<const uint4*>(Y + (x0 + xx) * ld + c * CH));
           }
         }
 #pragma unroll
@@ -2494,7 +2508,7 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
       for (int q = 0; q < NZ; ++q)
 #pragma unroll
         for (int r = 0; r < 4; ++r) z[q][r] = 0.f;
-      {
+      if constexpr (BF) {
 #pragma unroll 2
         for (int k0 = 0; k0 < KP; k0 += 16) {
           const T* pa = Phis + m0 * PLD + k0 + 2 * t4;
@@ -2511,6 +2525,35 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
             mma_bf16(z[q], afl, bf);
           }
         }
+      } else {
+        float zc[NZ][4];
+#pragma unroll
+        for (int q = 0; q < NZ; ++q)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) zc[q][r] = 0.f;
+#pragma unroll 2
+        for (int k0 = 0; k0 < KP; k0 += 8) {
+          const float* pa = Phis + m0 * PLD + k0 + t4;
+          uint32_t ah[4], al[4];
+          split_tf32(pa[g * PLD], ah[0], al[0]);
+          split_tf32(pa[(g + 8) * PLD], ah[1], al[1]);
+          split_tf32(pa[g * PLD + 4], ah[2], al[2]);
+          split_tf32(pa[(g + 8) * PLD + 4], ah[3], al[3]);
+#pragma unroll
+          for (int q = 0; q < NZ; ++q) {
+            const float* pb = Ys + q * TM * LDY + (n0 + g) * LDY + k0 + t4;
+            uint32_t bh[2], bl[2];
+            split_tf32(pb[0], bh[0], bl[0]);
+            split_tf32(pb[4], bh[1], bl[1]);
+            step32::mma_tf32(z[q], ah, bh);
+            step32::mma_tf32(zc[q], ah, bl);
+            step32::mma_tf32(zc[q], al, bh);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < NZ; ++q)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) z[q][r] += zc[q][r];
       }
       // epilogue: fragment r holds (i = m0 + g + 8 (r >> 1), x = n0 + 2 t4 + (r & 1))
       float dl[3][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
@@ -2545,7 +2588,10 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           T* dst = CT + c * IB * LDC + (m0 + g + 8 * h) * LDC + n0 + 2 * t4;
-          *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(cv[c][2 * h], cv[c][2 * h + 1]);
+          if constexpr (BF)
+            *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(cv[c][2 * h], cv[c][2 * h + 1]);
+          else
+            *reinterpret_cast<float2*>(dst) = make_float2(cv[c][2 * h], cv[c][2 * h + 1]);
         }
 #pragma unroll
       for (int qd = 0; qd < 3; ++qd) {
@@ -2574,13 +2620,27 @@ __device__ __forceinline__ void contract_body(const StpmPartialArgs& a, int nblo
           for (int c = 0; c < NC; ++c) {
             const T* Yo = Ys + (MODE == kModePlain ? 2 : c) * TM * LDY;
             const T* Cc = CT + c * IB * LDC;
-            {
+            if constexpr (BF) {
               uint32_t af[4];
               const int q = lane >> 3, rr = lane & 7;
               ldsm_x4_trans(af, Yo + (k0 + (q >> 1) * 8 + rr) * LDY + m0 + (q & 1) * 8);
               const T* pb = Cc + (n0 + g) * LDC + k0 + 2 * t4;
               const uint32_t bf[2] = {ld_b32(pb), ld_b32(pb + 8)};
               mma_bf16(gacc[u], af, bf);
+            } else {
+              const float* pa = Yo + (k0 + t4) * LDY + m0 + g;
+              uint32_t ah[4], al[4];
+              split_tf32(pa[0], ah[0], al[0]);
+              split_tf32(pa[8], ah[1], al[1]);
+              split_tf32(pa[4 * LDY], ah[2], al[2]);
+              split_tf32(pa[4 * LDY + 8], ah[3], al[3]);
+              const float* pb = Cc + (n0 + g) * LDC + k0 + t4;
+              uint32_t bh[2], bl[2];
+              split_tf32(pb[0], bh[0], bl[0]);
+              split_tf32(pb[4], bh[1], bl[1]);
+              step32::mma_tf32(gacc[u], ah, bh);
+              step32::mma_tf32(gacc[u], ah, bl);
+              step32::mma_tf32(gacc[u], al, bh);
             }
           }
         }
@@ -2956,11 +3016,11 @@ int stpm_partial_grid(int mode, int k, int64_t count, bool bf16) {
   // one wave: a second one repeats the per-CTA costs for a few CTAs (8,192
   // nodes, k = 100: 128 CTAs where 120 fit took 55 / 95 us in the loss and
   // adjoint forms, 39 / 69 us with 88).  As few CTAs as keep the largest share
-  // of tiles per CTA.  Not the tensor-core plain form of KP = 32: its
-  // accumulators truncate, and its small grids have little to gain.
+  // of tiles per CTA.  Not the iterations of KP = 32, whose results keep their
+  // roundings (k_step32.cuh): the split is the order of their sums.
   const int KP = stpm_kp(k);
-  const bool truncating = !bf16 && mode == kModePlain && KP <= 32;
-  const int64_t resident = KP < 0 || truncating ? 0
+  const bool keep = mode != kModeLoss && KP <= 32;
+  const int64_t resident = KP < 0 || keep ? 0
                            : bf16               ? partial_resident_p<true>(mode, KP)
                                                 : partial_resident_p<false>(mode, KP);
   if (resident > 0 && g > resident) {

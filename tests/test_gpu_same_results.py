@@ -101,6 +101,8 @@ def solve(mm, method, precision, k, seed):
 MOVED = [("ONLINE", "FP32", 5, 1), ("ONLINE", "FP32", 5, 91), ("ONLINE", "FP32", 6, 22),
          ("ONLINE", "FP32", 8, 27), ("ONLINE", "FP32", 12, 19), ("ONLINE", "BF16", 6, 6),
          ("ONLINE", "BF16", 12, 8)]
+MOVED += [("ADJOINT", "FP32", 5, 3), ("ADJOINT", "FP32", 8, 29), ("ADJOINT", "FP32", 12, 39),
+          ("ADJOINT", "BF16", 6, 1), ("ADJOINT", "BF16", 12, 19)]
 SOLVES = MOVED
 
 
