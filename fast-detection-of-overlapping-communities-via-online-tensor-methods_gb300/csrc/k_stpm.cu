@@ -258,7 +258,8 @@ constexpr float kPivotFloor = 1e-7f;
 constexpr float kShiftBelow = 1e-5f;
 // a first-order pass leaves about k |E|^2: it is repeated while an entry of E
 // is above this (the pivot ratios do not bound cond(X): with a few hundred
-// nodes per minibatch at k = 160 an exact pass left 0.1), at most 4 times
+// nodes per minibatch at k = 160 an exact pass left 0.1), at most 4 times; from
+// |E| = 1 / k on it need not contract, and exact passes run instead
 constexpr float kFirstOrderBelow = 1e-4f;
 constexpr float kShiftScale = 1e-5f;
 constexpr int kMaxShifts = 3;
@@ -839,9 +840,11 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
       csync_arrive();  // every rank has read the partials: blocks may land on them
       if (!csync_wait()) return false;
     }
-    // (a flag in the padding of the block's first column: see more_orders)
+    // (a flag in the padding of the block's first column: see left_over)
     const bool large = __syncthreads_or(first_order && emax > kFirstOrderBelow) != 0;
-    if (tid == 0) St[KP] = large ? 1.f : 0.f;
+    const bool wide = large && __syncthreads_or(emax * (float)k > 1.f) != 0;
+    const float flag = wide ? 2.f : large ? 1.f : 0.f;
+    if (tid == 0) St[KP] = flag;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (lane == 0 && warp < CL - 1)
@@ -852,7 +855,7 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
       if ((e & 63) < n4)
         reinterpret_cast<float4*>(A + (r0 + (e >> 6)) * XLD)[e & 63] =
             reinterpret_cast<const float4*>(St + (e >> 6) * XLD)[e & 63];
-    if (tid == 0) A[r0 * XLD + KP] = large ? 1.f : 0.f;
+    if (tid == 0) A[r0 * XLD + KP] = flag;
     if (tid < CL && tid != rank) {
       mbar_arrive_expect_tx(&s_blk[tid], kBlockBytes);
       ok = mbar_wait_bounded(&s_blk[tid], par_blk, wl);
@@ -861,12 +864,13 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
     return !__syncthreads_or(!ok);
   };
 
-  // whether any rank's block of E had an entry above kFirstOrderBelow (the
-  // same in every CTA: the blocks carry it in their padding)
-  auto more_orders = [&]() -> bool {
-    bool more = false;
-    for (int q = 0; q < CL; ++q) more = more || A[q * RB * XLD + KP] != 0.f;
-    return more;
+  // 1 where any rank's block of E had an entry above kFirstOrderBelow, 2 where
+  // one was above 1 / k (the same in every CTA: the blocks carry it in their
+  // padding)
+  auto left_over = [&]() -> float {
+    float f = 0.f;
+    for (int q = 0; q < CL; ++q) f = fmaxf(f, A[q * RB * XLD + KP]);
+    return f;
   };
 
   float* M = Xr;  // own rows of the matrix to orthonormalise
@@ -1008,7 +1012,7 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
   int passes = 0, shifts = 0, plain_left = a.max_passes;
   float shift = 0.f;
   bool first_order = false;  // the second pass: E = M^T M - I, Phi = M (I - F)
-  int orders = 0;
+  int orders = 0, wide_left = a.max_passes;
   float emax_all = 0.f;
   while (true) {
     if (!gram(M, first_order)) {
@@ -1016,7 +1020,16 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
       break;
     }
     if (first_order) {
-      const bool more = more_orders() && orders < 4;
+      const float left = left_over();
+      if (left > 1.f && wide_left > 0) {
+        --wide_left;
+        emax_all = fmaxf(emax_all, emax);
+        emax = 0.f;
+        first_order = false;
+        continue;
+      }
+      const bool more = left > 0.f && orders < 4;
+      if (left > 0.f && !more && rank == 0 && tid == 0) atomicOr(a.flags, kFlagNoConvergence);
       ++orders;
       // no copy to this CTA is outstanding after the last pass; its own may
       // still be read by others, so it stays until every rank has arrived here

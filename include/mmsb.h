@@ -132,8 +132,10 @@ typedef struct mmsb_stats {
   double step_flops;
   int64_t step_launches;
   /* largest max_ij |Q1^T Q1 - I| over the steps, Q1 the result of the exact
-   * Cholesky QR passes of a step before its first-order pass (the returned
-   * Phi is orthonormal to about the square of this, or FP32 round-off) */
+   * Cholesky QR passes of a step before a first-order pass.  For k > 32 those
+   * repeat, or give way to further exact passes, while an entry is above 1e-4;
+   * for k <= 32 one runs, and Phi is orthonormal to about the square of this,
+   * or FP32 round-off */
   double orth_err_max;
 } mmsb_stats;
 
