@@ -7,7 +7,7 @@
 #include <functional>
 #include <cstring>
 #include <memory>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -54,48 +54,81 @@ void d2h(mmsb_ctx* c, void* dst, const void* src, size_t bytes) {
   ck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->s), "D2H");
 }
 
-// A large result into the caller's buffer.  Into pageable memory it goes
-// through page-locked slots of the context, a thread per slot: what bounds it
-// is the host's first touch of the caller's pages, which the driver's own
-// staging does on one thread (the three 20 MB panels of n = 200,000, k = 100:
-// 5.5 ms through a host copy, 1.6 ms here).
-void d2h_large(mmsb_ctx* c, void* dst, const void* src, size_t bytes) {
+// The context's page-locked slots and their events; false where the host has no
+// such memory to give.
+bool host_slots(mmsb_ctx* c) {
+  if (c->host_slots) return true;
+  void* p = nullptr;
+  if (cudaMallocHost(&p, mmsb_ctx::kHostSlotBytes * mmsb_ctx::kHostSlots) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  for (auto& e : c->host_ev)
+    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFreeHost(p);
+      return false;
+    }
+  c->host_slots = p;
+  return true;
+}
+
+// The first k of ld columns of an n-row panel into the caller's buffer, rows
+// packed.  Into pageable memory a large panel goes through page-locked slots of
+// the context, a thread per slot: what bounds it is the host's first touch of the
+// caller's pages, which the driver's own staging does on one thread (the three
+// 20 MB panels of n = 200,000, k = 100: 5.5 ms through a host copy, 1.6 ms here).
+// The threads drop the padding columns too, so that no device memory is needed
+// for it: a context that just fitted can still be read.
+void d2h_rows(mmsb_ctx* c, float* dst, const float* src, int64_t n, int k, int ld) {
   constexpr size_t kSlot = mmsb_ctx::kHostSlotBytes;
   constexpr int kSlots = mmsb_ctx::kHostSlots;
+  const size_t row = sizeof(float) * (size_t)ld, bytes = row * (size_t)n;
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) cudaGetLastError();
-  if (at.type == cudaMemoryTypeHost || bytes < ((size_t)64 << 10)) {
+  // memory that CUDA knows, of whatever kind, takes the copy itself
+  if (ld == k && (at.type != cudaMemoryTypeUnregistered || bytes < ((size_t)64 << 10))) {
     d2h(c, dst, src, bytes);
     return;
   }
-  if (bytes < 4 * kSlot) {
-    std::vector<char> h(bytes);  // (touched here, not by the driver's copy)
-    d2h(c, h.data(), src, bytes);
-    ck(cudaStreamSynchronize(c->s), "sync");
-    std::memcpy(dst, h.data(), bytes);
+  auto unpack = [&](int64_t r0, int64_t rows, const char* from) {
+    if (ld == k) {
+      std::memcpy(dst + r0 * k, from, (size_t)rows * row);
+      return;
+    }
+    for (int64_t r = 0; r < rows; ++r)
+      std::memcpy(dst + (r0 + r) * k, from + (size_t)r * row, sizeof(float) * (size_t)k);
+  };
+  if (bytes < 4 * kSlot || row > kSlot || !host_slots(c)) {
+    const int64_t per = std::min<int64_t>(n, std::max<int64_t>(1, (int64_t)(4 * kSlot / row)));
+    std::vector<char> h((size_t)per * row);  // (touched here, not by the driver's copy)
+    for (int64_t r0 = 0; r0 < n; r0 += per) {
+      const int64_t rows = std::min(per, n - r0);
+      d2h(c, h.data(), src + r0 * ld, (size_t)rows * row);
+      ck(cudaStreamSynchronize(c->s), "sync");
+      unpack(r0, rows, h.data());
+    }
     return;
   }
-  if (!c->host_slots) {
-    ck(cudaMallocHost(&c->host_slots, kSlot * kSlots), "staging");
-    for (auto& e : c->host_ev) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-  }
+  const int64_t per = (int64_t)(kSlot / row);  // whole rows per slot
   std::atomic<int> bad{(int)cudaSuccess};
   auto work = [&](int t) {
     cudaError_t e = cudaSetDevice(c->cfg.device);
     char* slot = static_cast<char*>(c->host_slots) + kSlot * t;
-    for (size_t off = kSlot * t; off < bytes && e == cudaSuccess; off += kSlot * kSlots) {
-      const size_t len = std::min(kSlot, bytes - off);
-      e = cudaMemcpyAsync(slot, static_cast<const char*>(src) + off, len, cudaMemcpyDeviceToHost, c->s);
+    for (int64_t r0 = per * t; r0 < n && e == cudaSuccess; r0 += per * kSlots) {
+      const int64_t rows = std::min(per, n - r0);
+      e = cudaMemcpyAsync(slot, src + r0 * ld, (size_t)rows * row, cudaMemcpyDeviceToHost, c->s);
       if (e == cudaSuccess) e = cudaEventRecord(c->host_ev[t], c->s);
       if (e == cudaSuccess) e = cudaEventSynchronize(c->host_ev[t]);
-      if (e == cudaSuccess) std::memcpy(static_cast<char*>(dst) + off, slot, len);
+      if (e == cudaSuccess) unpack(r0, rows, slot);
     }
     if (e != cudaSuccess) bad.store((int)e);
   };
   std::vector<std::thread> pool;
   try {
+    pool.reserve(kSlots);
     for (int t = 1; t < kSlots; ++t) pool.emplace_back(work, t);
-  } catch (const std::system_error&) {
+  } catch (const std::exception&) {  // no thread, or no memory for one
   }
   work(0);
   // slots that got no thread
@@ -293,7 +326,7 @@ mmsb_status mmsb_get_pi(mmsb_ctx* c, float* pi) {
   if (!c || !pi) return MMSB_ERR_INVALID_ARG;
   if (!c->have_post) return MMSB_ERR_STATE;
   return guard(c, [&]() {
-    d2h_large(c, pi, c->pi, sizeof(float) * (size_t)mmsb_num_nodes(c) * c->k);
+    d2h_rows(c, pi, c->pi, mmsb_num_nodes(c), c->k, c->k);
     ck(cudaStreamSynchronize(c->s), "sync");
   });
 }
@@ -492,19 +525,8 @@ mmsb_status mmsb_get_whitened(mmsb_ctx* c, float* ya, float* yb, float* yc, doub
   if (!c->have_y) return MMSB_ERR_STATE;
   return guard(c, [&]() {
     float* outs[3] = {ya, yb, yc};
-    // straight into the caller's buffers: the rows are packed on the device
-    // where the panel has padding columns (a staging copy and a row loop on
-    // the host took 5.5 ms for the three 20 MB panels of n = 200,000, k = 100)
-    for (int q = 0; q < 3; ++q) {
-      if (!outs[q]) continue;
-      const float* src = c->y[q];
-      if (c->ldk != c->k) {
-        float* pack = c->tbuf<float>("y_pack", (size_t)c->nX * c->k);
-        ck(panel_copy(src, c->ldk, c->nX, c->k, pack, c->k, c->s), "pack y");
-        src = pack;
-      }
-      d2h_large(c, outs[q], src, sizeof(float) * (size_t)c->nX * c->k);
-    }
+    for (int q = 0; q < 3; ++q)
+      if (outs[q]) d2h_rows(c, outs[q], c->y[q], c->nX, c->k, c->ldk);
     std::vector<double> m64(3 * (size_t)c->k);
     d2h(c, m64.data(), c->ymu64, m64.size() * sizeof(double));
     ck(cudaStreamSynchronize(c->s), "sync");
