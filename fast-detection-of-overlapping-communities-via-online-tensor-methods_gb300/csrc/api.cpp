@@ -727,12 +727,15 @@ mmsb_status mmsb_op_gram(const float* A, int64_t n, int32_t pa, const float* B, 
   std::unique_ptr<mmsb_ctx> own(c);
   return guard(c, [&]() {
     float* dA = c->tbuf<float>("A", (size_t)n * pa);
-    float* dB = c->tbuf<float>("B", (size_t)n * pb);
+    // one panel given twice is one panel on the device: the Cholesky QR's form
+    const bool same = A == B && pa == pb;
+    float* dB = same ? dA : c->tbuf<float>("B", (size_t)n * pb);
     double* dS = c->tbuf<double>("S", (size_t)pa * pb);
     const int64_t cap = (int64_t)gram_tsk_partials(n, pa, pb);
     double* part = c->tbuf<double>("part", (size_t)cap);
     ck(cudaMemcpyAsync(dA, A, sizeof(float) * n * pa, cudaMemcpyHostToDevice, c->s), "H2D");
-    ck(cudaMemcpyAsync(dB, B, sizeof(float) * n * pb, cudaMemcpyHostToDevice, c->s), "H2D");
+    if (!same)
+      ck(cudaMemcpyAsync(dB, B, sizeof(float) * n * pb, cudaMemcpyHostToDevice, c->s), "H2D");
     ck(gram_tsk(dA, pa, pa, dB, pb, pb, n, alpha, dS, part, cap, c->s, c->flags), "gram");
     d2h(c, S, dS, sizeof(double) * pa * pb);
     ck(cudaStreamSynchronize(c->s), "sync");
