@@ -915,12 +915,13 @@ void stpm_online_stats(mmsb_ctx* c, int64_t steps) {
   ck(cudaStreamSynchronize(c->s), "sync");
   c->stats.orth_passes = passes;
   c->stats.orth_err_max = oerr;
-  // per online update 4 k^3 (the Gram Phi^T Phi and the product with its
-  // square) and 3 k^3 for the first-order pass (Gram, triangular product);
-  // per exact Cholesky QR pass 2 k^3 (Gram) + k^3 (triangular product) +
-  // k^3 / 3 (Cholesky) + k^3 / 3 (triangular inverse)
+  // per online update 3 k^3 for a first-order pass (Gram, triangular product;
+  // a repeated one is not counted); per exact Cholesky QR pass 2 k^3 (Gram) +
+  // k^3 / 3 (Cholesky) + k^3 (the rows of X through the factor); 4 k^3 in the
+  // first update of a run (the Gram Phi^T Phi and the product with its square:
+  // later ones have Phi^T Phi = I)
   const double kkk = (double)k * k * k;
-  c->stats.step_flops = kkk * (7.0 * (double)steps + 11.0 / 3.0 * (double)passes);
+  c->stats.step_flops = kkk * (3.0 * (double)steps + 10.0 / 3.0 * (double)passes + 4.0);
   check_flags(c, "stpm");
   collect_kernel_times(c);
   c->have_phi = true;

@@ -122,9 +122,9 @@ typedef struct mmsb_stats {
   int64_t orth_passes;     /* exact Cholesky QR passes summed over the STPM steps */
   /* STPM kernels of the last mmsb_stpm, timed with CUDA events around each
    * launch; flops are algorithmic (k, not the padded tile size):
-   * contraction 2 k^2 per node per Z and per G product, step 7 k^3 per
-   * online update (its Grams and products, the first-order QR pass) plus
-   * 11/3 k^3 per exact Cholesky QR pass */
+   * contraction 2 k^2 per node per Z and per G product, step 3 k^3 per
+   * online update (a first-order QR pass) plus 10/3 k^3 per exact Cholesky QR
+   * pass plus 4 k^3 per run (the first update's Phi (Phi^T Phi)^.2) */
   double contract_ms;
   double contract_flops;
   int64_t contract_launches;

@@ -31,3 +31,19 @@ def test_hidden_condition(mm, oracle, k, cond):
     assert np.abs(phi.T @ phi - np.eye(k)).max() < 1e-5
     # (the tensor value's sign may have turned columns)
     assert np.abs(np.tril(phi.T @ x, -1)).max() < 6e-7 * k * np.linalg.norm(x, 2)
+
+
+def test_step_flops(mm):
+    """What is counted is what runs: 3 k^3 per step, 10/3 k^3 per exact pass and
+    4 k^3 once for the first step's Phi (Phi^T Phi)^.2."""
+    k, nx = 40, 400
+    rng = np.random.default_rng(1)
+    y = {n: rng.standard_normal((k, nx)) for n in ("Da", "Db", "Dc")}
+    y.update({n + "_mu": y[n].mean(axis=1) for n in ("Da", "Db", "Dc")})
+    e = mm.CsrBlock(nx, 1, np.zeros(nx + 1, np.int64), np.zeros(0, np.int32))
+    o = mm.CsrBlock(1, 1, np.zeros(2, np.int64), np.zeros(0, np.int32))
+    with mm.Pipeline(k=k, alpha0=1.0, stpm_method=mm.STPM_ONLINE, sweeps=2, minibatch=100) as p:
+        p.upload(mm.Graph([e, e, e, o, o], (nx, 1, 1, 1))).set_whitened(y).stpm()
+        s = p.stats()
+    assert s["stpm_steps"] == 8
+    assert s["step_flops"] == pytest.approx(k ** 3 * (3 * 8 + 10 / 3 * s["orth_passes"] + 4))
