@@ -16,11 +16,14 @@
 // the cubic form (three Z's, three coefficient matrices, one stacked
 // contraction) and the loss.
 //
-// The contraction runs on the tensor cores (stpm_contract_kernel); partials
-// of 8-CTA clusters are summed through distributed shared memory and reduced
+// The contraction (stpm_contract_kernel) runs on tcgen05 in the plain FP32 form
+// and the BF16 adjoint form up to KP = 112, on mma.sync in the other BF16 forms
+// and the FP32 adjoint steps of KP = 32, else as FFMA; partials of 8-CTA
+// clusters are summed through distributed shared memory and reduced
 // deterministically by stpm_reduce or by the step kernel.  The k x k update
 // (orthogonality term, step, Cholesky QR) runs on one cluster that splits the
-// rows of the iterate and exchanges Gram blocks by bulk copies.
+// rows of the iterate and exchanges Gram blocks by bulk copies (at KP = 32 its
+// columns, k_step32.cuh).
 #include "common.cuh"
 
 #include <cstdlib>
@@ -226,8 +229,8 @@ __global__ void __launch_bounds__(256) stpm_reduce_kernel(StpmReduceArgs a) {
 // first-order product is on the own rows as well.  (Owning columns instead
 // took an exchange of X, of A and of Q1 per pass, the triangular inverse and
 // three k^3 products: a minibatch step, contraction included, took 54 us at
-// k = 100 and 330 us at k = 200; 45 and 295 us here.)  KP = 32 has a form of its
-// own (k_step32.cuh).
+// k = 100 and 330 us at k = 200; 45 and 295 us here, 250 us with the contraction
+// in FFMA.)  KP = 32 has a form of its own (k_step32.cuh).
 //
 // All products are FP32 FMAs (a thread per column, 8 rows at a time, the row
 // operand broadcast from shared memory): mma.sync TF32 in 3xTF32 form gives
@@ -1179,20 +1182,21 @@ __device__ __forceinline__ void step_body(const StpmUpdateArgs& a) {
   }
 }
 
-// ---- partial contractions on the tensor cores -----------------------------------
+// ---- partial contractions --------------------------------------------------------
 //
 // Per tile of TM nodes, with Phi resident in shared memory:
-//   Z_q^T = Phi^T Y_q^T           (k x TM, m16n8k8 3xTF32 or m16n8k16 BF16 MMAs;
-//                                  both operands contiguous along j)
-//   C = c0 Z1.Z2 + c2 (Z1 m2 + m1 Z2)   (on the Z fragments; stored i-major)
-//   G += Yout^T C                 (k x k, accumulated in registers over the
-//                                  CTA's tiles; the Yout operand is read
-//                                  transposed: strided loads in FP32,
-//                                  ldmatrix.trans in BF16)
+//   Z_q^T = Phi^T Y_q^T           (k x TM)
+//   C = c0 Z1.Z2 + c2 (Z1 m2 + m1 Z2)
+//   G += Yout^T C                 (k x k, accumulated over the CTA's tiles)
 //   d_i += sum_x Z1 Z2            (per column i)
-// The FP32 form keeps FP32 accuracy through the 3xTF32 split; the BF16 form
-// reads y rounded to BF16, Phi as a BF16 pair (hi + lo: Z = hi^T y + lo^T y,
-// two MMAs), the coefficients C rounded to BF16, and accumulates in FP32.
+// in one of four forms: contract_tc (tcgen05, 3xTF32: the plain FP32 form up to
+// KP = 112), contract_tc_bf (tcgen05, BF16: the adjoint form up to KP = 112),
+// contract_ffma (the other FP32 forms) and the mma.sync body of contract_body
+// (the other BF16 forms, m16n8k16; m16n8k8 in 3xTF32 form for the FP32 adjoint
+// steps of KP = 32).  The BF16 forms read y rounded to BF16, Phi as a BF16 pair
+// (hi + lo: Z = hi^T y + lo^T y, two MMAs) and the coefficients C rounded to
+// BF16, and accumulate in FP32.
+//
 // Tensor-core form of the plain FP32 contraction (tcgen05.mma kind::tf32,
 // 3xTF32: D += Ahi Bhi + Ahi Blo + Alo Bhi), for KP in [32, 112].  Per tile
 // of TM = 32 nodes:
