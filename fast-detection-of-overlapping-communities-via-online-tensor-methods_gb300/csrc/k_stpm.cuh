@@ -39,7 +39,8 @@ struct StpmPartialArgs {
   long long wait_limit;  // clock64 cycles a bounded wait may take (0: about one second)
   // tensor-core plain FP32 form (KP <= 112): Phi already split into its TF32
   // hi / lo operand image, as the previous step kernel wrote it
-  // (stpm_phi_image_bytes); null: the contraction stages Phi itself
+  // (stpm_phi_image_bytes), at KP = 32 followed by Phi^T mu1 | Phi^T mu2 (2 KP
+  // floats); null: the contraction stages Phi itself
   const void* phi_img;
 };
 
@@ -103,7 +104,7 @@ struct StpmUpdateArgs {
   // the contraction's operand image of the new Phi (stpm_phi_image_bytes), or
   // null
   void* phi_img;
-  // convergence trace (may be null): CTA q writes sum over its rows of
+  // convergence trace (may be null): CTA q writes sum over its rows (KP = 32: columns) of
   // (Phi_new - trace_snap)^2 to trace_out[q] and sets trace_snap = Phi_new there
   float* trace_snap;
   double* trace_out;
