@@ -174,6 +174,26 @@ __global__ void __launch_bounds__(1024) scan_kernel(unsigned long long* __restri
   }
 }
 
+// A thread per row, where rows are short and many: the atomics of a warp's rows
+// overlap, and a warp per row would leave most lanes without an entry.
+__global__ void scatter_short_kernel(const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                     const float* __restrict__ val, int64_t n_rows, int64_t n_cols,
+                                     int64_t nnz, unsigned long long* __restrict__ cursor,
+                                     int32_t* __restrict__ ciT, float* __restrict__ valT) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = rp[r] > 0 ? rp[r] : 0, e = rp[r + 1] < nnz ? rp[r + 1] : nnz;
+    for (int64_t j = b; j < e; ++j) {
+      const int32_t c = ci[j];
+      if (c < 0 || (int64_t)c >= n_cols) continue;
+      const unsigned long long pos = atomicAdd(&cursor[c], 1ull);
+      if (pos >= (unsigned long long)nnz) continue;
+      ciT[pos] = (int32_t)r;
+      if (valT) valT[pos] = val[j];
+    }
+  }
+}
+
 // A warp per row: a thread per row walked its entries one atomic's latency at a
 // time (1,000 rows of 110 entries 41 us, 6.3 us here).  Lanes with the same column
 // (duplicate entries) take consecutive places in their order, so that duplicates
@@ -441,12 +461,22 @@ cudaError_t csr_transpose(const int64_t* rp, const int32_t* ci, const float* val
   u64_to_i64_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(1024, ceil_div(n_cols + 1, T))), T, 0, s>>>(cnt, n_cols + 1, rpT);
   ++g_launch_count;
   if (nnz > 0) {
+    // a thread per row from 65,536 rows of fewer than 8 entries on (upload of five
+    // blocks: 500,000 rows of 2 2.20 ms, 2.40 ms with a warp per row; of 8 3.02 and
+    // 3.07 ms; 100,000 rows of 4 0.75 and 0.78 ms; but 20,000 rows of 4 0.38 and 0.36
+    // ms, 100,000 rows of 24 1.30 and 1.24 ms)
+    const bool short_rows = n_rows >= 65536 && nnz < 8 * n_rows;
     const unsigned GR =
-        (unsigned)std::max<int64_t>(1, std::min<int64_t>(16384, ceil_div(n_rows * 32, T)));
+        short_rows
+            ? (unsigned)std::min<int64_t>(4096, ceil_div(n_rows, T))
+            : (unsigned)std::max<int64_t>(1, std::min<int64_t>(16384, ceil_div(n_rows * 32, T)));
     // row 0 in every slot first: a malformed block (row ranges that overlap
     // or skip entries) then leaves valid row indices, never stale words
     MMSB_CUDA_TRY(cudaMemsetAsync(tmp_c, 0, sizeof(int32_t) * nnz, s));
-    scatter_kernel<<<GR, T, 0, s>>>(rp, ci, val, n_rows, n_cols, nnz, cnt, tmp_c, tmp_v);
+    if (short_rows)
+      scatter_short_kernel<<<GR, T, 0, s>>>(rp, ci, val, n_rows, n_cols, nnz, cnt, tmp_c, tmp_v);
+    else
+      scatter_kernel<<<GR, T, 0, s>>>(rp, ci, val, n_rows, n_cols, nnz, cnt, tmp_c, tmp_v);
     ++g_launch_count;
     segment_sort_kernel<<<(unsigned)ceil_div(n_cols * 32, T), T, 0, s>>>(rpT, n_cols, tmp_c, tmp_v,
                                                                           ciT, valT);
