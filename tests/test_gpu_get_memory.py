@@ -40,3 +40,22 @@ def test_whitened_rows(mm, k, nx):
         got = p.whitened()
     for n in y:
         assert np.array_equal(got[n], y[n])
+
+
+@pytest.mark.parametrize("k,nx", [(4, 5000), (8, 100000), (100, 60000)])
+def test_whitened_rows_into_old_and_new_pages(mm, k, nx):
+    """The same rows whether the buffer's pages were touched (numpy.ones, another
+    array's memory used again) or not (a fresh mapping)."""
+    import ctypes
+    import mmap
+    p, y = context(mm, k, nx)
+    with p:
+        for make in (lambda: np.ones(k * nx, np.float32),
+                     lambda: np.frombuffer(mmap.mmap(-1, 4 * k * nx), np.float32)):
+            outs = [make() for _ in range(3)]
+            for _ in range(2):
+                ptr = [o.ctypes.data_as(ctypes.POINTER(ctypes.c_float)) for o in outs]
+                p._ck(mm.lib().mmsb_get_whitened(p._h, *ptr, None, None, None))
+                for o, n in zip(outs, ("Da", "Db", "Dc")):
+                    assert np.array_equal(o.reshape((k, nx), order="F"), y[n])
+                    o[:] = 0.0
