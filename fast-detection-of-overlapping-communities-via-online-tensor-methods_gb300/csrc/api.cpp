@@ -736,7 +736,7 @@ mmsb_status mmsb_op_spmm(const mmsb_csr* g, int transpose, const float* P, int64
     float* dP = c->tbuf<float>("P", hp.size());
     float* dY = c->tbuf<float>("Y", hy.size());
     ck(cudaMemcpyAsync(dP, hp.data(), hp.size() * sizeof(float), cudaMemcpyHostToDevice, c->s), "H2D");
-    ck(spmm_f32(use.rp, use.ci, use.val, use.n_rows, dP, ld, alpha, dY, c->s), "spmm");
+    ck(spmm_f32(use.rp, use.ci, use.val, use.n_rows, use.nnz, dP, ld, alpha, dY, c->s), "spmm");
     d2h(c, hy.data(), dY, hy.size() * sizeof(float));
     ck(cudaStreamSynchronize(c->s), "sync");
     for (int64_t r = 0; r < n_out; ++r) std::memcpy(Y + r * p, &hy[(size_t)r * ld], sizeof(float) * p);

@@ -38,7 +38,7 @@ extern thread_local int64_t g_launch_count;
 // p_rows (rows of P, i.e. columns of G), when given, lets panels far larger
 // than L2 run as column slices that stay L2-resident.
 cudaError_t spmm_f32(const int64_t* rp, const int32_t* ci, const float* val, int64_t n_rows,
-                     const float* P, int ld, float alpha, float* Y, cudaStream_t s,
+                     int64_t nnz, const float* P, int ld, float alpha, float* Y, cudaStream_t s,
                      int64_t p_rows = 0);
 // Checks an uploaded block: ORs 1 into *bad for a decreasing row offset, 2
 // for a column index outside [0, n_cols).
@@ -57,7 +57,7 @@ cudaError_t row_sums_f64(const int64_t* rp, const float* val, int64_t n_rows, do
 // written to pi[(row_offset + r) * k + i] and set bits.  raw_scale > 0:
 // raw_scale * raw written instead (no normalisation, bits untouched).
 cudaError_t unwhiten_normprob(const int64_t* rp, const int32_t* ci, const float* val,
-                              int64_t n_rows, const float* P, int ldp, int k, float tau,
+                              int64_t n_rows, int64_t nnz, const float* P, int ldp, int k, float tau,
                               int64_t row_offset, float* pi, uint32_t* bits, cudaStream_t s,
                               float raw_scale = 0.f);
 

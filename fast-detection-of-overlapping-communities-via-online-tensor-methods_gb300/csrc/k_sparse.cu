@@ -91,21 +91,28 @@ __global__ void __launch_bounds__(256) spmm_rows_kernel(
 // latency of its chains of loads sets the time: then 16 gathers in flight per
 // lane (a row of 250 nonzeros in 16 round trips instead of 63; SpMM of a
 // 1,000 x 1,000 block with 10 columns 34 us -> 11.5 us), else 4 (more cost
-// registers and occupancy: 3,117 -> 2,956 GB/s on 400-column panels).
+// registers and occupancy: 3,117 -> 2,956 GB/s on 400-column panels).  Rows of
+// fewer than 16 nonzeros on average have no use for the deep form and pay for its
+// registers (60,000 rows of 8, 10 columns: 10.3 us, 13.1 us deep; 30,000 rows of 4,
+// 30 columns 7.8 and 10.2 us; at 16 the two are even, at 40 the deep one gains 7%).
 constexpr int64_t kFewThreads = (int64_t)kNumSMs * 1024;
+
+bool deep_gather(int64_t n_rows, int64_t nnz, int lanes) {
+  return n_rows * lanes < kFewThreads && nnz >= 16 * n_rows;
+}
 
 template <int G>
 cudaError_t launch_spmm(const int64_t* rp, const int32_t* ci, const float* val, int64_t n_rows,
-                        const float* P, int c4, float alpha, float* Y, cudaStream_t s,
+                        int64_t nnz, const float* P, int c4, float alpha, float* Y, cudaStream_t s,
                         int cb = 0, int ce = -1) {
-  // small grids in small CTAs, so that they spread over the SMs
-  const bool few = n_rows * G < kFewThreads;
-  const int threads = few ? 64 : 256;
+  // (the deep form in small CTAs, so that a small grid spreads over the SMs)
+  const bool deep = deep_gather(n_rows, nnz, G);
+  const int threads = deep ? 64 : 256;
   const int64_t blocks = ceil_div(n_rows * G, threads);
   const float4* p4 = reinterpret_cast<const float4*>(P);
   float4* y4 = reinterpret_cast<float4*>(Y);
   if (ce < 0) ce = c4;
-  if (few)
+  if (deep)
     spmm_rows_kernel<G, 16><<<(unsigned)blocks, threads, 0, s>>>(rp, ci, val, n_rows, p4, c4, alpha, y4, cb, ce);
   else
     spmm_rows_kernel<G, 4><<<(unsigned)blocks, threads, 0, s>>>(rp, ci, val, n_rows, p4, c4, alpha, y4, cb, ce);
@@ -380,7 +387,7 @@ __global__ void __launch_bounds__(256) unwhiten_normprob_kernel(
 }  // namespace
 
 cudaError_t spmm_f32(const int64_t* rp, const int32_t* ci, const float* val, int64_t n_rows,
-                     const float* P, int ld, float alpha, float* Y, cudaStream_t s,
+                     int64_t nnz, const float* P, int ld, float alpha, float* Y, cudaStream_t s,
                      int64_t p_rows) {
   if (ld % 4 != 0) return cudaErrorInvalidValue;
   if (n_rows == 0) return cudaSuccess;
@@ -398,20 +405,20 @@ cudaError_t spmm_f32(const int64_t* rp, const int32_t* ci, const float* val, int
     w4 = std::max(8, w4 / 8 * 8);
     for (int cb = 0; cb < c4; cb += w4) {
       const int ce = std::min(c4, cb + w4);
-      cudaError_t e = w4 >= 64   ? launch_spmm<32>(rp, ci, val, n_rows, P, c4, alpha, Y, s, cb, ce)
-                      : w4 >= 32 ? launch_spmm<16>(rp, ci, val, n_rows, P, c4, alpha, Y, s, cb, ce)
-                      : w4 >= 16 ? launch_spmm<8>(rp, ci, val, n_rows, P, c4, alpha, Y, s, cb, ce)
-                                 : launch_spmm<4>(rp, ci, val, n_rows, P, c4, alpha, Y, s, cb, ce);
+      cudaError_t e = w4 >= 64   ? launch_spmm<32>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s, cb, ce)
+                      : w4 >= 32 ? launch_spmm<16>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s, cb, ce)
+                      : w4 >= 16 ? launch_spmm<8>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s, cb, ce)
+                                 : launch_spmm<4>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s, cb, ce);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
   }
-  if (c4 <= 2) return launch_spmm<1>(rp, ci, val, n_rows, P, c4, alpha, Y, s);
-  if (c4 <= 4) return launch_spmm<2>(rp, ci, val, n_rows, P, c4, alpha, Y, s);
-  if (c4 <= 8) return launch_spmm<4>(rp, ci, val, n_rows, P, c4, alpha, Y, s);
-  if (c4 <= 16) return launch_spmm<8>(rp, ci, val, n_rows, P, c4, alpha, Y, s);
-  if (c4 <= 32) return launch_spmm<16>(rp, ci, val, n_rows, P, c4, alpha, Y, s);
-  return launch_spmm<32>(rp, ci, val, n_rows, P, c4, alpha, Y, s);
+  if (c4 <= 2) return launch_spmm<1>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s);
+  if (c4 <= 4) return launch_spmm<2>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s);
+  if (c4 <= 8) return launch_spmm<4>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s);
+  if (c4 <= 16) return launch_spmm<8>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s);
+  if (c4 <= 32) return launch_spmm<16>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s);
+  return launch_spmm<32>(rp, ci, val, n_rows, nnz, P, c4, alpha, Y, s);
 }
 
 // Input checks of an uploaded block (the transposes and SpMMs index with
@@ -496,16 +503,16 @@ cudaError_t row_sums_f64(const int64_t* rp, const float* val, int64_t n_rows, do
 }
 
 cudaError_t unwhiten_normprob(const int64_t* rp, const int32_t* ci, const float* val,
-                              int64_t n_rows, const float* P, int ldp, int k, float tau,
+                              int64_t n_rows, int64_t nnz, const float* P, int ldp, int k, float tau,
                               int64_t row_offset, float* pi, uint32_t* bits, cudaStream_t s,
                               float raw_scale) {
   if (ldp % 4 != 0 || k > 256 || k > ldp) return cudaErrorInvalidValue;
   if (n_rows == 0) return cudaSuccess;
-  const bool few = n_rows * 32 < kFewThreads;
-  const int T = few ? 64 : 256;
+  const bool deep = deep_gather(n_rows, nnz, 32);
+  const int T = deep ? 64 : 256;
   const unsigned grid = (unsigned)ceil_div(n_rows * 32, T);
   const float4* p4 = reinterpret_cast<const float4*>(P);
-  if (few)
+  if (deep)
     unwhiten_normprob_kernel<16><<<grid, T, 0, s>>>(rp, ci, val, n_rows, p4, ldp / 4, k, tau,
                                                     row_offset, pi, bits, raw_scale);
   else

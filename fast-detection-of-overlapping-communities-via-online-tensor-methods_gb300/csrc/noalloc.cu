@@ -113,6 +113,6 @@ extern "C" mmsb_status mmsb_op_spmm_t_noalloc(const int64_t* d_row_ptr, const in
   e = mmsb::csr_transpose(d_row_ptr, d_col_idx, d_val, n_rows, n_cols, nnz, rp_t, ci_t, val_t,
                           work, st);
   if (e == cudaSuccess)
-    e = mmsb::spmm_f32(rp_t, ci_t, val_t, n_cols, d_P, (int)p, alpha, d_Y, st);
+    e = mmsb::spmm_f32(rp_t, ci_t, val_t, n_cols, nnz, d_P, (int)p, alpha, d_Y, st);
   return e == cudaSuccess ? MMSB_OK : MMSB_ERR_CUDA;
 }

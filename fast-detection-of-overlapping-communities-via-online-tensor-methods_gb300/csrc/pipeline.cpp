@@ -116,11 +116,11 @@ void spmm(mmsb_ctx* c, const DevCsr& g, const float* P, int ld, float alpha, flo
   const size_t slot = c->spmm_events.size();
   if (slot < c->spmm_pool.size()) {
     ck(cudaEventRecord(c->spmm_pool[slot].first, st), "event");
-    ck(spmm_f32(g.rp, g.ci, g.val, g.n_rows, P, ld, alpha, Y, st, g.n_cols), "spmm");
+    ck(spmm_f32(g.rp, g.ci, g.val, g.n_rows, g.nnz, P, ld, alpha, Y, st, g.n_cols), "spmm");
     ck(cudaEventRecord(c->spmm_pool[slot].second, st), "event");
     c->spmm_events.push_back(slot);
   } else {
-    ck(spmm_f32(g.rp, g.ci, g.val, g.n_rows, P, ld, alpha, Y, st, g.n_cols), "spmm");
+    ck(spmm_f32(g.rp, g.ci, g.val, g.n_rows, g.nnz, P, ld, alpha, Y, st, g.n_cols), "spmm");
   }
   c->stats.spmm_launches += 1;
   c->stats.spmm_bytes += 8.0 * (g.n_rows + 1) + 4.0 * g.nnz * (g.val ? 2 : 1) +
@@ -1018,10 +1018,10 @@ void pipeline_post(mmsb_ctx* c) {
   ck(panel_times_small(c->Ub, ldk, k, c->nB, ZP, k, k, PA2, ldk, s), "PA2");
   const float tau = c->cfg.tau;
   const DevCsr &XA = c->g[0], &BA = c->g[3], &CA = c->g[4], &BAt = c->gt[3];
-  ck(unwhiten_normprob(XA.rp, XA.ci, XA.val, XA.n_rows, PA, ldk, k, tau, 0, c->pi, c->bits, s), "pi_x");
-  ck(unwhiten_normprob(BAt.rp, BAt.ci, BAt.val, BAt.n_rows, PA2, ldk, k, tau, c->nX, c->pi, c->bits, s), "pi_a");
-  ck(unwhiten_normprob(BA.rp, BA.ci, BA.val, BA.n_rows, PA, ldk, k, tau, c->nX + c->nA, c->pi, c->bits, s), "pi_b");
-  ck(unwhiten_normprob(CA.rp, CA.ci, CA.val, CA.n_rows, PA, ldk, k, tau, c->nX + c->nA + c->nB, c->pi, c->bits, s), "pi_c");
+  ck(unwhiten_normprob(XA.rp, XA.ci, XA.val, XA.n_rows, XA.nnz, PA, ldk, k, tau, 0, c->pi, c->bits, s), "pi_x");
+  ck(unwhiten_normprob(BAt.rp, BAt.ci, BAt.val, BAt.n_rows, BAt.nnz, PA2, ldk, k, tau, c->nX, c->pi, c->bits, s), "pi_a");
+  ck(unwhiten_normprob(BA.rp, BA.ci, BA.val, BA.n_rows, BA.nnz, PA, ldk, k, tau, c->nX + c->nA, c->pi, c->bits, s), "pi_b");
+  ck(unwhiten_normprob(CA.rp, CA.ci, CA.val, CA.n_rows, CA.nnz, PA, ldk, k, tau, c->nX + c->nA + c->nB, c->pi, c->bits, s), "pi_c");
   c->have_post = true;
 }
 
@@ -1037,10 +1037,10 @@ void pipeline_post_raw(mmsb_ctx* c, double lambda_norm, float* out) {
   float* PA2 = c->tbuf<float>("PA2", (size_t)c->nB * ldk);
   const float sc = (float)lambda_norm;
   const DevCsr &XA = c->g[0], &BA = c->g[3], &CA = c->g[4], &BAt = c->gt[3];
-  ck(unwhiten_normprob(XA.rp, XA.ci, XA.val, XA.n_rows, PA, ldk, k, 0.f, 0, out, nullptr, s, sc), "raw pi_x");
-  ck(unwhiten_normprob(BAt.rp, BAt.ci, BAt.val, BAt.n_rows, PA2, ldk, k, 0.f, c->nX, out, nullptr, s, sc), "raw pi_a");
-  ck(unwhiten_normprob(BA.rp, BA.ci, BA.val, BA.n_rows, PA, ldk, k, 0.f, c->nX + c->nA, out, nullptr, s, sc), "raw pi_b");
-  ck(unwhiten_normprob(CA.rp, CA.ci, CA.val, CA.n_rows, PA, ldk, k, 0.f, c->nX + c->nA + c->nB, out, nullptr, s, sc), "raw pi_c");
+  ck(unwhiten_normprob(XA.rp, XA.ci, XA.val, XA.n_rows, XA.nnz, PA, ldk, k, 0.f, 0, out, nullptr, s, sc), "raw pi_x");
+  ck(unwhiten_normprob(BAt.rp, BAt.ci, BAt.val, BAt.n_rows, BAt.nnz, PA2, ldk, k, 0.f, c->nX, out, nullptr, s, sc), "raw pi_a");
+  ck(unwhiten_normprob(BA.rp, BA.ci, BA.val, BA.n_rows, BA.nnz, PA, ldk, k, 0.f, c->nX + c->nA, out, nullptr, s, sc), "raw pi_b");
+  ck(unwhiten_normprob(CA.rp, CA.ci, CA.val, CA.n_rows, CA.nnz, PA, ldk, k, 0.f, c->nX + c->nA + c->nB, out, nullptr, s, sc), "raw pi_c");
 }
 
 // ---------------------------------------------------------------------------
