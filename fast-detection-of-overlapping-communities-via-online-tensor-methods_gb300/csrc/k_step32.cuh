@@ -312,7 +312,7 @@ inline __device__ float chol_blocked(float* A, int k, float* tinv, float* rd, fl
   return *s_ratio;
 }
 
-// Columns c0 .. c0+NB of W = R^-1 (NB = 8 or 16: whole 8-column blocks) into
+// Columns c0 .. c0+NB of W = R^-1 (whole 8-column blocks) into
 // Wb (column jb at Wb + jb * XLD, rows past the diagonal block zero), by
 // block back substitution per 8-column block K: W_KK = T_KK, then upwards in
 // levels of 16 rows aligned to 16 (one 8-row level first when K is odd):
@@ -328,7 +328,7 @@ inline __device__ float chol_blocked(float* A, int k, float* tinv, float* rd, fl
 // get unit columns.  tmp: 128 floats.  Whole CTA of at least 5 warps; ends
 // with a barrier.
 inline __device__ void inverse_columns(const float* R, const float* tinv, float* x16, int c0, int k,
-                                float* Wb, float* tmp) {
+                                       float* Wb, float* tmp) {
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int e = tid; e < NB * XLD; e += nt) Wb[e] = 0.f;
   // X(a, b) = -sum_i T_2m(a, i) sum_j R(16m + i, 16m + 8 + j) T_2m+1(j, b)
